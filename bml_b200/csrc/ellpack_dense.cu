@@ -28,6 +28,7 @@
 #include "device_util.cuh"
 
 #include <cstring>
+#include <type_traits>
 
 using namespace b200;
 
@@ -42,7 +43,7 @@ struct DenseFlags
     int overflow;
     int max_width;
     int bad_input;
-    int pad;
+    int asym; // X^2: the image differs from its transpose
 };
 
 // image[i * ld + col] += value for every stored entry (duplicates add up, as
@@ -125,8 +126,12 @@ template <> __device__ __forceinline__ float fma_t<float>(float a, float b, floa
 // A^T (16 x 128) and B (16 x 128).
 template <typename T>
 __global__ void __launch_bounds__(DTHREADS, 1) dense_gemm_kernel(const T *__restrict__ A, const T *__restrict__ B,
-                                                                 T *__restrict__ Cm, size_t ld, int Kp)
+                                                                 T *__restrict__ Cm, size_t ld, int Kp,
+                                                                 const int *asym)
 {
+    const bool sym = asym && *asym == 0;
+    if (sym && blockIdx.x < blockIdx.y)
+        return;
     extern __shared__ __align__(16) unsigned char dsm[];
     T(*As)[DK][DT] = reinterpret_cast<T(*)[DK][DT]>(dsm);
     T(*Bs)[DK][DT] = reinterpret_cast<T(*)[DK][DT]>(dsm + 2 * sizeof(T) * DK * DT);
@@ -199,7 +204,135 @@ __global__ void __launch_bounds__(DTHREADS, 1) dense_gemm_kernel(const T *__rest
     for (int m = 0; m < 8; ++m)
 #pragma unroll
         for (int n = 0; n < 8; ++n)
+        {
             Cm[(i0 + ty + 16 * m) * ld + j0 + tx + 16 * n] = acc[m][n];
+            if (sym && blockIdx.x > blockIdx.y)
+                Cm[(j0 + tx + 16 * n) * ld + i0 + ty + 16 * m] = acc[m][n];
+        }
+}
+
+// -------------------------------------------------------------------------
+// FP64 GEMM on the tensor instructions (mma.sync m8n8k4, 37 TFLOP/s; the FMA
+// pipe reaches 34).  128 x 128 of C per CTA of 8 warps, each 64 x 32 (8 x 4
+// accumulator tiles, 64 doubles per lane); k in steps of 16 through a ring of
+// GS stages filled by 16-byte cp.async, so three steps are in flight while one
+// is multiplied.  Rows of A's stage are 20 doubles apart and rows of B's 132:
+// the 16 lanes of a half warp, (row, k) = (lane / 4, lane % 4) of A and (k,
+// column) = (lane % 4, lane / 4) of B, then read 16 distinct bank pairs.
+// 12 8-byte loads feed 32 MMAs, an eighth of the shared-memory rate.
+// Symmetric C (A == B with equal mirrored entries, *asym == 0): only the
+// tiles on and above the diagonal are formed and each is stored twice.
+// -------------------------------------------------------------------------
+constexpr int GS = 4;                  // stages
+constexpr int GA = 20, GB = DT + 4;    // row strides of the stages, in doubles
+constexpr int GSTAGE = DT * GA + DK * GB;
+
+__device__ __forceinline__ void cp16(double *dst, const double *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned) __cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+
+__global__ void __launch_bounds__(DTHREADS, 1) dense_gemm_f64_kernel(const double *__restrict__ A,
+                                                                     const double *__restrict__ B,
+                                                                     double *__restrict__ Cm, size_t ld, int Kp,
+                                                                     const int *asym)
+{
+    extern __shared__ __align__(16) unsigned char dsm[];
+    double *st = reinterpret_cast<double *>(dsm);
+    const bool sym = asym && *asym == 0;
+    if (sym && blockIdx.x < blockIdx.y)
+        return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int wm = (warp >> 2) * 64, wn = (warp & 3) * 32;
+    const size_t i0 = (size_t) blockIdx.y * DT, j0 = (size_t) blockIdx.x * DT;
+    // thread t copies 8 chunks: A row t >> 3 (+ 32 u), k 2 (t & 7); B row t >> 6 (+ 4 u), columns 2 (t & 63)
+    const double *pa = A + (i0 + (tid >> 3)) * ld + 2 * (tid & 7);
+    const double *pb = B + (size_t) (tid >> 6) * ld + j0 + 2 * (tid & 63);
+    const int sa = (tid >> 3) * GA + 2 * (tid & 7), sb = DT * GA + (tid >> 6) * GB + 2 * (tid & 63);
+    auto fetch = [&](int step) {
+        double *s = st + (step % GS) * GSTAGE;
+        const double *a = pa + (size_t) step * DK, *b = pb + (size_t) step * DK * ld;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+        {
+            cp16(s + sa + 32 * u * GA, a + 32 * u * ld);
+            cp16(s + sb + 4 * u * GB, b + 4 * u * ld);
+        }
+    };
+    double acc[8][4][2];
+#pragma unroll
+    for (int m = 0; m < 8; ++m)
+#pragma unroll
+        for (int n = 0; n < 4; ++n)
+            acc[m][n][0] = acc[m][n][1] = 0.0;
+    const int steps = Kp / DK; // a multiple of 8
+    for (int s = 0; s < GS - 1; ++s)
+    {
+        fetch(s);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    const int fa = (wm + (lane >> 2)) * GA + (lane & 3), fb = DT * GA + (lane & 3) * GB + wn + (lane >> 2);
+    for (int step = 0; step < steps; ++step)
+    {
+        asm volatile("cp.async.wait_group %0;" ::"n"(GS - 2) : "memory");
+        __syncthreads();
+        if (step + GS - 1 < steps)
+            fetch(step + GS - 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const double *s = st + (step % GS) * GSTAGE;
+#pragma unroll
+        for (int k = 0; k < DK; k += 4)
+        {
+            double a[8], b[4];
+#pragma unroll
+            for (int m = 0; m < 8; ++m)
+                a[m] = s[fa + 8 * m * GA + k];
+#pragma unroll
+            for (int n = 0; n < 4; ++n)
+                b[n] = s[fb + k * GB + 8 * n];
+#pragma unroll
+            for (int m = 0; m < 8; ++m)
+#pragma unroll
+                for (int n = 0; n < 4; ++n)
+                    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                                 : "+d"(acc[m][n][0]), "+d"(acc[m][n][1])
+                                 : "d"(a[m]), "d"(b[n]));
+        }
+    }
+    const int r = lane >> 2, q = 2 * (lane & 3);
+#pragma unroll
+    for (int m = 0; m < 8; ++m)
+#pragma unroll
+        for (int n = 0; n < 4; ++n)
+        {
+            const size_t row = i0 + wm + 8 * m + r, col = j0 + wn + 8 * n + q;
+            *reinterpret_cast<double2 *>(Cm + row * ld + col) = make_double2(acc[m][n][0], acc[m][n][1]);
+            if (sym && blockIdx.x > blockIdx.y)
+            {
+                Cm[col * ld + row] = acc[m][n][0];
+                Cm[(col + 1) * ld + row] = acc[m][n][1];
+            }
+        }
+}
+
+// *asym = 1 when some entry of the image differs from its mirror (a NaN
+// differs from itself).  One CTA per pair of 32 x 32 blocks.
+template <typename T> __global__ void __launch_bounds__(256) dense_sym_kernel(const T *A, size_t ld, int *asym)
+{
+    __shared__ T t[32][33];
+    if (blockIdx.x < blockIdx.y || *(volatile int *) asym)
+        return;
+    const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+    const size_t i0 = (size_t) blockIdx.y * 32, j0 = (size_t) blockIdx.x * 32;
+    for (int r = y; r < 32; r += 8)
+        t[r][x] = A[(j0 + r) * ld + i0 + x];
+    __syncthreads();
+    int bad = 0;
+    for (int r = y; r < 32; r += 8)
+        bad |= A[(i0 + r) * ld + j0 + x] != t[x][r];
+    if (__any_sync(FULL, bad) && x == 0)
+        atomicExch(asym, 1);
 }
 
 template <typename T> __device__ __forceinline__ bool above_d(T x, double thr);
@@ -306,11 +439,30 @@ bool dense_typed(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bml_matrix_el
                                                        A->ld, NA, B->N, pat, ld, touched, trace ? dA : nullptr);
     if (!LAUNCH_OK("dense_diag_kernel"))
         return false;
+    if (same)
+    {
+        dense_sym_kernel<T><<<dim3((unsigned) (ld / 32), (unsigned) (ld / 32)), 256, 0, c->stream>>>(DA, ld, &flags->asym);
+        if (!LAUNCH_OK("dense_sym_kernel"))
+            return false;
+    }
     const dim3 grid((unsigned) (ld / DT), (unsigned) (ld / DT));
-    const size_t smemG = 4 * sizeof(T) * DK * DT;
-    if (!CUDA_OK(cudaFuncSetAttribute(dense_gemm_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smemG)))
-        return false;
-    dense_gemm_kernel<T><<<grid, DTHREADS, smemG, c->stream>>>(DA, DB, DC, ld, (int) ld);
+    const int *asym = same ? &flags->asym : nullptr;
+    if constexpr (std::is_same<T, double>::value)
+    {
+        const size_t smemG = GS * GSTAGE * sizeof(double);
+        if (!CUDA_OK(cudaFuncSetAttribute(dense_gemm_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int) smemG)))
+            return false;
+        dense_gemm_f64_kernel<<<grid, DTHREADS, smemG, c->stream>>>(DA, DB, DC, ld, (int) ld, asym);
+    }
+    else
+    {
+        const size_t smemG = 4 * sizeof(T) * DK * DT;
+        if (!CUDA_OK(cudaFuncSetAttribute(dense_gemm_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int) smemG)))
+            return false;
+        dense_gemm_kernel<T><<<grid, DTHREADS, smemG, c->stream>>>(DA, DB, DC, ld, (int) ld, asym);
+    }
     if (!LAUNCH_OK("dense_gemm_kernel"))
         return false;
     dense_compact_kernel<T><<<wgrid, 256, 0, c->stream>>>(DC, ld, NA, ncols, touched, thr, static_cast<T *>(C->d_value),
