@@ -111,7 +111,7 @@ bml_matrix_ellblock_t *eb_alloc_blocks(bml_matrix_precision_t prec, int NB, int 
         A->indexb[q] = -1;
     A->nnzb = static_cast<int *>(calloc(NB, sizeof(int)));
     A->ptr_value = static_cast<void **>(calloc((size_t) NB * MB, sizeof(void *)));
-    A->h_pool = calloc(eb_pool_elems(A), sz);
+    A->h_pool = b200_mirror_alloc(eb_pool_elems(A) * sz);
     A->domain = b200_default_domain(N, M, mode);
     A->domain2 = b200_default_domain(N, M, mode);
     bool ok = A->bsize && A->indexb && A->nnzb && A->ptr_value && A->h_pool;
@@ -164,7 +164,7 @@ void eb_free(bml_matrix_ellblock_t *A)
             if (p)
                 cudaFreeAsync(p, c->stream);
     }
-    free(A->h_pool);
+    b200_mirror_free(A->h_pool, eb_pool_elems(A) * prec_size(A->matrix_precision));
     free(A->ptr_value);
     free(A->indexb);
     free(A->nnzb);

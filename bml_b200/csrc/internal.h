@@ -125,6 +125,9 @@ bool ell_to_host(bml_matrix_ellpack_t *A);     // download if device is newer
 inline void ell_mark_device(bml_matrix_ellpack_t *A) { A->mirror = MIRROR_DEVICE_NEWER; }
 inline void ell_mark_host(bml_matrix_ellpack_t *A) { A->mirror = MIRROR_HOST_NEWER; }
 
+// Zeroed host memory of a matrix mirror, and its release (with its size).
+void *b200_mirror_alloc(size_t bytes);
+void b200_mirror_free(void *p, size_t bytes);
 bml_domain_t *b200_default_domain(int N, int M, bml_distribution_mode_t mode);
 void b200_free_domain(bml_domain_t *D);
 

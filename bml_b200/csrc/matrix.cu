@@ -5,6 +5,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <cmath>
+#include <sys/mman.h>
 
 size_t prec_size(bml_matrix_precision_t p)
 {
@@ -63,6 +64,31 @@ void b200_free_domain(bml_domain_t *d)
     free(d);
 }
 
+// Zeroed host mirror arrays.  Large ones are mapped directly: their pages
+// exist from the first touch on, so the mirror of a matrix that stays on the
+// device costs nothing.  (calloc maps only blocks above a threshold that
+// grows to 32 MB as such blocks are freed, and clears the others: 1.6 ms for
+// a temporary of N = 4096, M = 1536, which made up most of an adjoint step.)
+static const size_t MIRROR_MAPPED = 256 << 10;
+
+void *b200_mirror_alloc(size_t bytes)
+{
+    if (bytes < MIRROR_MAPPED)
+        return calloc(bytes, 1);
+    void *p = mmap(nullptr, bytes, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | MAP_NORESERVE, -1, 0);
+    return p == MAP_FAILED ? nullptr : p;
+}
+
+void b200_mirror_free(void *p, size_t bytes)
+{
+    if (!p)
+        return;
+    if (bytes < MIRROR_MAPPED)
+        free(p);
+    else
+        munmap(p, bytes);
+}
+
 bml_matrix_ellpack_t *ell_alloc(bml_matrix_precision_t prec, int N, int M,
                                 bml_distribution_mode_t mode, bool zero)
 {
@@ -92,10 +118,8 @@ bml_matrix_ellpack_t *ell_alloc(bml_matrix_precision_t prec, int N, int M,
     A->N = N;
     A->M = M;
     A->ld = b200_round_up(M, 32);
-    // Host mirror: calloc pages are mapped on first touch, so an unused
-    // mirror of a large matrix costs no host memory traffic.
-    A->value = calloc((size_t) N * M, sz);
-    A->index = static_cast<int *>(calloc((size_t) N * M, sizeof(int)));
+    A->value = b200_mirror_alloc((size_t) N * M * sz);
+    A->index = static_cast<int *>(b200_mirror_alloc((size_t) N * M * sizeof(int)));
     A->nnz = static_cast<int *>(calloc((size_t) N, sizeof(int)));
     A->domain = b200_default_domain(N, M, mode);
     A->domain2 = b200_default_domain(N, M, mode);
@@ -151,8 +175,8 @@ void ell_free(bml_matrix_ellpack_t *A)
                 cudaFreeAsync(A->d_nnz, c->stream);
         }
     }
-    free(A->value);
-    free(A->index);
+    b200_mirror_free(A->value, (size_t) A->N * A->M * prec_size(A->matrix_precision));
+    b200_mirror_free(A->index, (size_t) A->N * A->M * sizeof(int));
     free(A->nnz);
     b200_free_domain(A->domain);
     b200_free_domain(A->domain2);
