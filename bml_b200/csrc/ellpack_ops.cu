@@ -3,7 +3,9 @@
 // Each kernel reproduces the reference loop's arithmetic and output order.
 #include "device_util.cuh"
 
+#include <algorithm>
 #include <cfloat>
+#include <climits>
 #include <cstring>
 
 using namespace b200;
@@ -98,7 +100,7 @@ template <typename T, int W>
 __global__ void __launch_bounds__(W * 32) add_kernel(T *Av, int *Ai, int *An, int lda, int Ma,
                                                    const T *Bv, const int *Bi, const int *Bn,
                                                    int ldb, int N, double alpha, double beta,
-                                                   double thr, int logts, int *overflow)
+                                                   double thr, int logts, const unsigned char *todo, int *overflow)
 {
     constexpr int NT = W * 32;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -118,6 +120,8 @@ __global__ void __launch_bounds__(W * 32) add_kernel(T *Av, int *Ai, int *An, in
 
     for (int i = blockIdx.x; i < N; i += gridDim.x)
     {
+        if (todo && !todo[i])
+            continue;
         for (int s = tid; s < TS; s += NT)
             keys[s] = B200_EMPTY_KEY;
         __syncthreads();
@@ -269,6 +273,199 @@ __global__ void __launch_bounds__(W * 32) add_kernel(T *Av, int *Ai, int *An, in
                 atomicExch(overflow, 1);
         }
         __syncthreads(); // before the next row reuses the shared arrays
+    }
+}
+
+// The same sum through a direct table, for rows whose columns of B span less
+// than MAP_COLS: map[col % MAP_COLS] is the place of the column in B's row
+// (plus one), so finding B's entry of a column of A is one 2-byte read instead
+// of a hash probe, and neither row is staged in shared memory: entries wait in
+// registers (MAP_U a thread) for the block's prefix.  64 KB a CTA whatever M
+// is (the hash form takes 20 M + 16 times the power of two above M bytes: at
+// M = 2048 two CTAs per SM and 1.33 ms for the update of the 40^3 iterate).
+// Rows it cannot hold are left untouched and marked in `todo` for the hash
+// form, *left set.  A's part is rewritten in place: a round's entries are
+// read before they are written, at or before their own places.
+constexpr int MAP_COLS = 32768;
+constexpr int MAP_U = 4; // entries per thread of a round
+
+template <typename T, int W>
+__global__ void __launch_bounds__(W * 32, 3) add_map_kernel(T *Av, int *Ai, int *An, int lda, int Ma, const T *Bv,
+                                                       const int *Bi, const int *Bn, int ldb, int N, double alpha,
+                                                       double beta, double thr, unsigned char *todo, int *left,
+                                                       int *overflow)
+{
+    constexpr int NT = W * 32;
+    constexpr unsigned short USED = 0x8000u;
+    extern __shared__ __align__(16) unsigned char smem[];
+    unsigned short *map = reinterpret_cast<unsigned short *>(smem);
+    __shared__ int cnt[2][W];
+    __shared__ int lo, hi;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
+    const T thr_t = (T) thr;
+    const bool use_a = alpha > 0.0 || alpha < 0.0;
+    const bool use_b = beta > 0.0 || beta < 0.0;
+    for (int s = tid; s < MAP_COLS / 8; s += NT)
+        reinterpret_cast<uint4 *>(smem)[s] = make_uint4(0u, 0u, 0u, 0u);
+    for (int i = blockIdx.x; i < N; i += gridDim.x)
+    {
+        const int na = use_a ? An[i] : 0;
+        const int nb = use_b ? Bn[i] : 0;
+        if (tid == 0)
+        {
+            lo = INT_MAX;
+            hi = -1;
+        }
+        // the first round of both rows, loaded before anything waits for it
+        const size_t ra = (size_t) i * lda, rb = (size_t) i * ldb;
+        int kb[MAP_U], kk[MAP_U];
+        T xb[MAP_U], xx[MAP_U];
+        unsigned keep[MAP_U];
+#pragma unroll
+        for (int u = 0; u < MAP_U; ++u)
+        {
+            const int p = (warp * MAP_U + u) * 32 + lane;
+            kb[u] = p < nb ? __ldg(Bi + rb + p) : -1;
+            kk[u] = p < na ? Ai[ra + p] : -1;
+            xx[u] = p < na ? Av[ra + p] : T(0);
+            xb[u] = p < nb ? __ldg(Bv + rb + p) : T(0);
+        }
+        __syncthreads(); // also: the map is clear, and cnt free
+        int mn = INT_MAX, mx = -1;
+#pragma unroll
+        for (int u = 0; u < MAP_U; ++u)
+        {
+            const int p = (warp * MAP_U + u) * 32 + lane;
+            if (p < nb)
+            {
+                mn = min(mn, kb[u]);
+                mx = max(mx, kb[u]);
+                map[kb[u] & (MAP_COLS - 1)] = (unsigned short) (p + 1);
+            }
+        }
+        for (int q = NT * MAP_U + tid; q < nb; q += NT)
+        {
+            const int k = __ldg(Bi + rb + q);
+            mn = min(mn, k);
+            mx = max(mx, k);
+            map[k & (MAP_COLS - 1)] = (unsigned short) (q + 1);
+        }
+        for (int o = 16; o; o >>= 1)
+        {
+            mn = min(mn, __shfl_xor_sync(FULL, mn, o));
+            mx = max(mx, __shfl_xor_sync(FULL, mx, o));
+        }
+        if (lane == 0 && mx >= 0)
+        {
+            atomicMin(&lo, mn);
+            atomicMax(&hi, mx);
+        }
+        __syncthreads();
+        const int blo = lo, bhi = hi;
+        if (bhi - blo >= MAP_COLS || nb >= USED)
+        {
+            for (int q = tid; q < nb; q += NT)
+                map[__ldg(Bi + rb + q) & (MAP_COLS - 1)] = 0;
+            if (tid == 0)
+            {
+                todo[i] = 1;
+                *reinterpret_cast<volatile int *>(left) = 1;
+            }
+            __syncthreads();
+            continue;
+        }
+        int ll = 0; // kept so far (uniform)
+        int flip = 0;
+        // A's entries, then B's new ones, in rounds of NT * MAP_U; thread t of warp w holds entries
+        // w * 32 * MAP_U + u * 32 + lane of the round
+        auto emit = [&](const int(&ek)[MAP_U], const T(&ex)[MAP_U]) {
+            int c = 0;
+#pragma unroll
+            for (int u = 0; u < MAP_U; ++u)
+                c += __popc(keep[u]);
+            if (lane == 0)
+                cnt[flip][warp] = c;
+            __syncthreads();
+            int at = ll, all = 0;
+#pragma unroll
+            for (int w = 0; w < W; ++w)
+            {
+                const int cw = cnt[flip][w];
+                at += w < warp ? cw : 0;
+                all += cw;
+            }
+#pragma unroll
+            for (int u = 0; u < MAP_U; ++u)
+            {
+                const int p = at + __popc(keep[u] & lanemask_lt());
+                if ((keep[u] >> lane & 1u) && p < Ma)
+                {
+                    Av[ra + p] = ex[u];
+                    Ai[ra + p] = ek[u];
+                }
+                at += __popc(keep[u]);
+            }
+            ll += all;
+            flip ^= 1;
+        };
+        for (int p0 = 0; p0 < na; p0 += NT * MAP_U)
+        {
+            if (p0 > 0)
+#pragma unroll
+                for (int u = 0; u < MAP_U; ++u)
+                {
+                    const int p = p0 + (warp * MAP_U + u) * 32 + lane;
+                    kk[u] = p < na ? Ai[ra + p] : -1;
+                    xx[u] = p < na ? Av[ra + p] : T(0);
+                }
+#pragma unroll
+            for (int u = 0; u < MAP_U; ++u)
+            {
+                xx[u] = axpy_d(T(0), alpha, xx[u]);
+                if (kk[u] >= blo && kk[u] <= bhi)
+                {
+                    const unsigned short m = map[kk[u] & (MAP_COLS - 1)];
+                    if (m)
+                    {
+                        map[kk[u] & (MAP_COLS - 1)] = m | USED;
+                        xx[u] = axpy_d(xx[u], beta, __ldg(Bv + rb + (m & (USED - 1)) - 1));
+                    }
+                }
+                keep[u] = __ballot_sync(FULL, p0 + (warp * MAP_U + u) * 32 + lane < na && fabs(xx[u]) > thr_t);
+            }
+            emit(kk, xx);
+        }
+        __syncthreads(); // A's marks in the map
+        for (int p0 = 0; p0 < nb; p0 += NT * MAP_U)
+        {
+            if (p0 > 0)
+#pragma unroll
+                for (int u = 0; u < MAP_U; ++u)
+                {
+                    const int p = p0 + (warp * MAP_U + u) * 32 + lane;
+                    kb[u] = p < nb ? __ldg(Bi + rb + p) : -1;
+                    xb[u] = p < nb ? __ldg(Bv + rb + p) : T(0);
+                }
+#pragma unroll
+            for (int u = 0; u < MAP_U; ++u)
+            {
+                bool fresh = false;
+                if (p0 + (warp * MAP_U + u) * 32 + lane < nb)
+                {
+                    fresh = !(map[kb[u] & (MAP_COLS - 1)] & USED);
+                    map[kb[u] & (MAP_COLS - 1)] = 0;
+                    xb[u] = axpy_d(T(0), beta, xb[u]);
+                }
+                keep[u] = __ballot_sync(FULL, fresh && fabs(xb[u]) > thr_t);
+            }
+            emit(kb, xb);
+        }
+        if (tid == 0)
+        {
+            An[i] = min(ll, Ma);
+            if (ll > Ma)
+                atomicExch(overflow, 1);
+        }
     }
 }
 
@@ -757,6 +954,66 @@ bool check_pair(const bml_matrix_ellpack_t *A, const bml_matrix_ellpack_t *B, co
     return true;
 }
 
+constexpr int ADD_W = 8; // warps of an add CTA
+
+// xa[lda] newx[ldb] (matrix precision) | ka[lda] keys[TS] pos[TS] newk[ldb] cnt[8]
+template <typename T> size_t add_hash_smem(const bml_matrix_ellpack_t *A, const bml_matrix_ellpack_t *B, int logts)
+{
+    return (size_t) (A->ld + B->ld) * (sizeof(T) + 4) + ((size_t) 2 << logts) * 4 + ADD_W * 4 + 64;
+}
+
+template <typename T>
+bool add_typed(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, double alpha, double beta, double threshold)
+{
+    B200Context *c = b200_ctx();
+    // flags: rows left to the hash form, overflow
+    int *flags = reinterpret_cast<int *>(static_cast<unsigned char *>(c->d_small) + 2048);
+    int *pin = reinterpret_cast<int *>(static_cast<unsigned char *>(c->pinned) + 2048);
+    T *av = static_cast<T *>(A->d_value);
+    const T *bv = static_cast<const T *>(B->d_value);
+    unsigned char *todo = static_cast<unsigned char *>(b200_scratch(A->N));
+    if (!todo || !CUDA_OK(cudaMemsetAsync(todo, 0, A->N, c->stream)) ||
+        !CUDA_OK(cudaMemsetAsync(flags, 0, 2 * sizeof(int), c->stream)))
+        return false;
+    const size_t smemM = MAP_COLS * sizeof(unsigned short);
+    auto km = add_map_kernel<T, ADD_W>;
+    if (!CUDA_OK(cudaFuncSetAttribute(km, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smemM)))
+        return false;
+    km<<<min(A->N, c->sm_count * 3), 32 * ADD_W, smemM, c->stream>>>(av, A->d_index, A->d_nnz, A->ld, A->M, bv,
+                                                                     B->d_index, B->d_nnz, B->ld, A->N, alpha, beta,
+                                                                     threshold, todo, flags, flags + 1);
+    if (!LAUNCH_OK("add_map_kernel"))
+        return false;
+    ell_mark_device(A);
+    if (!CUDA_OK(cudaMemcpyAsync(pin, flags, 2 * sizeof(int), cudaMemcpyDeviceToHost, c->stream)) || !b200_sync())
+        return false;
+    if (pin[0])
+    {
+        // the hash holds A's row at most half full
+        int logts = 5;
+        while ((1 << logts) < 2 * A->M)
+            ++logts;
+        const size_t smem = add_hash_smem<T>(A, B, logts);
+        auto k = add_kernel<T, ADD_W>;
+        if (!CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)))
+            return false;
+        int occ = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 32 * ADD_W, smem);
+        k<<<min(A->N, c->sm_count * (occ > 0 ? occ : 1)), 32 * ADD_W, smem, c->stream>>>(
+            av, A->d_index, A->d_nnz, A->ld, A->M, bv, B->d_index, B->d_nnz, B->ld, A->N, alpha, beta, threshold,
+            logts, todo, flags + 1);
+        if (!LAUNCH_OK("add_kernel") ||
+            !CUDA_OK(cudaMemcpyAsync(pin, flags, 2 * sizeof(int), cudaMemcpyDeviceToHost, c->stream)) || !b200_sync())
+            return false;
+    }
+    if (pin[1])
+    {
+        b200_set_error(BML_B200_ERR_ROW_OVERFLOW, "add: a row of the sum has more than M=%d entries", A->M);
+        return false;
+    }
+    return true;
+}
+
 } // namespace
 
 bool ell_add(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, double alpha, double beta,
@@ -777,17 +1034,11 @@ bool ell_add(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, double alpha, dou
         ell_free(T0);
         return ok;
     }
-    int *ovf = zeroed_flag(c);
-    if (!ovf)
-        return false;
-    // the hash holds A's row at most half full
-    const int need = 2 * A->M;
     int logts = 5;
-    while ((1 << logts) < need)
+    while ((1 << logts) < 2 * A->M)
         ++logts;
-    const size_t sz = prec_size(A->matrix_precision);
-    // xa[lda] newx[ldb] (matrix precision) | ka[lda] keys[TS] pos[TS] newk[ldb] cnt[8]
-    const size_t smem = (size_t) (A->ld + B->ld) * (sz + 4) + ((size_t) 2 << logts) * 4 + 8 * 4 + 64;
+    const size_t smem =
+        A->matrix_precision == double_real ? add_hash_smem<double>(A, B, logts) : add_hash_smem<float>(A, B, logts);
     if (smem > c->smem_optin)
     {
         // rows too wide for the hash: through a dense image of the row sums
@@ -803,44 +1054,8 @@ bool ell_add(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, double alpha, dou
         return false;
     }
     if (A->matrix_precision == double_real)
-    {
-        auto k = add_kernel<double, 8>;
-        if (!CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)))
-            return false;
-        int occ = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 256, smem);
-        const int grid = min(A->N, c->sm_count * (occ > 0 ? occ : 1));
-        k<<<grid, 256, smem, c->stream>>>(static_cast<double *>(A->d_value), A->d_index, A->d_nnz,
-                                          A->ld, A->M, static_cast<const double *>(B->d_value),
-                                          B->d_index, B->d_nnz, B->ld, A->N, alpha, beta,
-                                          threshold, logts, ovf);
-    }
-    else
-    {
-        auto k = add_kernel<float, 8>;
-        if (!CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)))
-            return false;
-        int occ = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 256, smem);
-        const int grid = min(A->N, c->sm_count * (occ > 0 ? occ : 1));
-        k<<<grid, 256, smem, c->stream>>>(static_cast<float *>(A->d_value), A->d_index, A->d_nnz,
-                                          A->ld, A->M, static_cast<const float *>(B->d_value),
-                                          B->d_index, B->d_nnz, B->ld, A->N, alpha, beta,
-                                          threshold, logts, ovf);
-    }
-    if (!LAUNCH_OK("add_kernel"))
-        return false;
-    ell_mark_device(A);
-    int hov = 0;
-    if (!read_flag(c, ovf, &hov))
-        return false;
-    if (hov)
-    {
-        b200_set_error(BML_B200_ERR_ROW_OVERFLOW, "add: a row of the sum has more than M=%d entries",
-                       A->M);
-        return false;
-    }
-    return true;
+        return add_typed<double>(A, B, alpha, beta, threshold);
+    return add_typed<float>(A, B, alpha, beta, threshold);
 }
 
 bool ell_add_identity(bml_matrix_ellpack_t *A, double beta, double threshold)
@@ -1016,11 +1231,31 @@ bool ell_trace_mult(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, double *tr
     B200Context *c = b200_ctx();
     if (!c || !ell_to_device(A) || !ell_to_device(B))
         return false;
+    // The hash takes the rows of the narrower matrix (the sum is symmetric in
+    // A and B), sized by its widest row where finding that out (a pass over
+    // the row lengths and a round trip, about 15 us each) is small against the
+    // operation: sized by M = 2048, tr(D H) of the 40^3 density matrix took
+    // 3.2 ms with 4 warps per SM.
+    int wb = B->M;
+    if ((long long) A->N * (A->M + B->M) >= 1 << 22)
+    {
+        int wa = A->M;
+        long long t;
+        if (!ell_nnz_total(A, &t, &wa) || (B != A && !ell_nnz_total(B, &t, &wb)))
+            return false;
+        if (B == A)
+            wb = wa;
+        if (wa < wb)
+        {
+            std::swap(A, B);
+            wb = wa;
+        }
+    }
     double *part = static_cast<double *>(b200_scratch((size_t) A->N * sizeof(double)));
     if (!part)
         return false;
     int logts = 5;
-    while ((1 << logts) < 2 * B->M)
+    while ((1 << logts) < 2 * wb)
         ++logts;
     int warps_per_block = 4;
     size_t smem = (size_t) warps_per_block * 2 * (1 << logts) * sizeof(int);
