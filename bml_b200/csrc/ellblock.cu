@@ -1769,6 +1769,15 @@ bool eb_multiply_typed(bml_matrix_ellblock_t *A, bml_matrix_ellblock_t *B, bml_m
     bool bs32 = A->maxbs == 32 && B->maxbs == 32 && C->maxbs == 32;
     for (int ib = 0; bs32 && ib < A->NB; ib++)
         bs32 = A->bsize[ib] == 32 && B->bsize[ib] == 32;
+    if (sizeof(T) == 8 && bs32 && !ell_x2_exact())
+    {
+        bool taken = false;
+        const bool ok = eb_multiply_f64(A, B, C, thr, trace, (size_t) g_eb_slab_budget, &taken);
+        if (taken)
+            eb_mark_device(C);
+        if (taken || !ok)
+            return ok;
+    }
     const int grid0 = bs32 ? eb_grid<T>(c, A->NB, 4) : eb_grid<T>(c, A->NB, 2);
     const size_t slot_bytes = (size_t) A->slot_elems * sizeof(T);
     // Accumulator slots per CTA: room for all NB block columns (the

@@ -37,6 +37,10 @@ bool eb_write_mm(bml_matrix_ellblock_t *A, FILE *f);
 bool eb_read_mm(bml_matrix_ellblock_t *A, FILE *f, long long ne, bool symmetric);
 // X2 = X*X on the tensor cores: FP16 hi/lo split, FP32 accumulation; blocks of 32.
 bool eb_multiply_x2_tc(bml_matrix_ellblock_t *X, bml_matrix_ellblock_t *X2, double threshold, double *trace);
+// C = A*B in FP64 for 32 x 32 blocks, unordered form (ellblock_f64.cu); *taken
+// false, with no status set, when NB or the spill exceeds what it holds.
+bool eb_multiply_f64(bml_matrix_ellblock_t *A, bml_matrix_ellblock_t *B, bml_matrix_ellblock_t *C, double threshold,
+                     double *trace, size_t budget, bool *taken);
 bool eb_multiply_x2(bml_matrix_ellblock_t *X, bml_matrix_ellblock_t *X2, double threshold,
                     double *trace);
 bool eb_multiply_AB(bml_matrix_ellblock_t *A, bml_matrix_ellblock_t *B, bml_matrix_ellblock_t *C,
