@@ -583,6 +583,10 @@ struct TcTab
     uint4 *list;          // [pcap] the pairs sorted by wave, in (j, kp) order within a wave
     int *wstart;          // [wcap + 1] first pair of each wave in list
     int jcap, kcap, pcap, wcap;
+    // a group's waves are shared among `slices` CTAs, each a run of consecutive waves; the blocks that row r
+    // keeps in slice s then lie at runs[r * slices + s] = {first position, blocks}
+    int slices;
+    int2 *runs;
 };
 
 // Rank of the set bits of bits[0..nwords): pre[w] = set bits before word w,
@@ -804,9 +808,9 @@ __global__ void __launch_bounds__(TC_THREADS, Cfg::CTAS)
         if (tid == 0)
             S.grp = atomicAdd(&flags[4], 1);
         __syncthreads();
-        const int grp = S.grp;
-        if (grp >= ngroups || dead)
+        if (S.grp >= ngroups * G.slices || dead)
             break;
+        const int grp = S.grp / G.slices, slice = S.grp % G.slices;
         const int ib0 = grp * TC_GROUP;
         // ---- the group's block columns J: a bitmap over NB, index = rank ----
         const int nwords = (X.NB + 31) >> 5;
@@ -954,7 +958,9 @@ __global__ void __launch_bounds__(TC_THREADS, Cfg::CTAS)
             }
         }
         __syncthreads();
-        // ---- the pairs sorted by wave (a stable counting sort) ----
+        // the waves of this slice, and the pairs in them
+        const int wlo = (int) ((long long) nW * slice / G.slices), whi = (int) ((long long) nW * (slice + 1) / G.slices);
+        // ---- their pairs sorted by wave (a stable counting sort) ----
         // The J entries are cut into nq ranges of consecutive entries, one
         // per warp (nq = 4 when four rows of wave counters fit, else 1); warp
         // q places its range's pairs, in (j, kp) order, after those of the
@@ -968,13 +974,21 @@ __global__ void __launch_bounds__(TC_THREADS, Cfg::CTAS)
         if (nq == 1)
         {
             for (int p = tid; p < npairs; p += TC_THREADS)
-                atomicAdd(&cnt[G.ptile[p] / TC_TILES], 1);
+            {
+                const int w = G.ptile[p] / TC_TILES;
+                if (w >= wlo && w < whi)
+                    atomicAdd(&cnt[w], 1);
+            }
         }
         else
         {
             const int pl = G.jstart[jlo], ph = G.jstart[jhi];
             for (int p = pl + lane; p < ph; p += 32)
-                atomicAdd(&cnt[warp * nW + G.ptile[p] / TC_TILES], 1);
+            {
+                const int w = G.ptile[p] / TC_TILES;
+                if (w >= wlo && w < whi)
+                    atomicAdd(&cnt[warp * nW + w], 1);
+            }
         }
         __syncthreads();
         if (warp == 0)
@@ -1035,8 +1049,13 @@ __global__ void __launch_bounds__(TC_THREADS, Cfg::CTAS)
                     for (int k0 = 0; k0 < n; k0 += 32)
                     {
                         const int kp = k0 + lane;
-                        const int t = kp < n ? G.ptile[ps + kp] : -1;
-                        const int w = t >= 0 ? t / TC_TILES : -1 - lane;
+                        int t = kp < n ? G.ptile[ps + kp] : -1;
+                        int w = t >= 0 ? t / TC_TILES : -1 - lane;
+                        if (w < wlo || w >= whi)
+                        {
+                            t = -1;
+                            w = -1 - lane;
+                        }
                         const unsigned peers = __match_any_sync(FULL, w);
                         const int leader = __ffs(peers) - 1;
                         int base = 0;
@@ -1057,29 +1076,30 @@ __global__ void __launch_bounds__(TC_THREADS, Cfg::CTAS)
             }
         }
         __syncthreads();
+        const int nsorted = G.wstart[nW];
         // a step starts (a new left operand) where j changes within a wave,
         // and at every wave's first pair
-        for (int p = tid; p < npairs; p += TC_THREADS)
+        for (int p = tid; p < nsorted; p += TC_THREADS)
         {
             const unsigned x = G.list[p].x;
             if (p == 0 || ((x ^ G.list[p - 1].x) & 0x000FFFF0u))
                 G.list[p].x = x | 0x80000000u;
         }
         __syncthreads();
-        for (int w = tid; w < nW; w += TC_THREADS)
-            if (G.wstart[w] < npairs) // every wave has a pair: each tile is some pair's
+        for (int w = wlo + tid; w < whi; w += TC_THREADS)
+            if (G.wstart[w] < nsorted) // every wave has a pair: each tile is some pair's
                 G.list[G.wstart[w]].x |= 0x80000000u;
         __syncthreads();
         // every step's tiles, into its first record (ptile is free again: the
         // sort above was its last reader); the pairs of a step have distinct
         // tiles unless a row of X repeats a block column
         int badstep = 0;
-        for (int p = tid; p < npairs; p += TC_THREADS)
+        for (int p = tid; p < nsorted; p += TC_THREADS)
             if (G.list[p].x >> 31)
             {
                 unsigned m = 1u << (G.list[p].x & 15u);
                 int n = 1;
-                for (int q = p + 1; q < npairs && !(G.list[q].x >> 31); ++q, ++n)
+                for (int q = p + 1; q < nsorted && !(G.list[q].x >> 31); ++q, ++n)
                     m |= 1u << (G.list[q].x & 15u);
                 badstep |= __popc(m) != n;
                 G.ptile[p] = (int) m;
@@ -1090,14 +1110,20 @@ __global__ void __launch_bounds__(TC_THREADS, Cfg::CTAS)
                 atomicExch(&flags[2], 1);
             continue;
         }
-        for (int p = tid; p < npairs; p += TC_THREADS)
+        for (int p = tid; p < nsorted; p += TC_THREADS)
             if (G.list[p].x >> 31)
                 G.list[p].x = (G.list[p].x & 0x8000000Fu) | (unsigned) G.ptile[p] << 4;
-        int kept = 0;
+        // the row's blocks of earlier slices come first: as many places as it has products in
+        int before = 0;
+        for (int t = lane; t < min(wlo * TC_TILES, nK); t += 32)
+            before += (G.ttouch[t] >> warp) & 1;
+        for (int o = 16; o; o >>= 1)
+            before += __shfl_xor_sync(FULL, before, o);
+        int kept = before;
         double trc = 0.0;
 
         // ---- tr X of the group's rows (FP64, row order) ----
-        if (myrow < X.NB)
+        if (myrow < X.NB && slice == 0)
         {
             double s = 0.0;
             for (int j0 = 0; j0 < X.nnzb[myrow]; j0 += 32)
@@ -1124,7 +1150,7 @@ __global__ void __launch_bounds__(TC_THREADS, Cfg::CTAS)
         __syncthreads();
 
         // ---- waves of TC_TILES output tiles ----
-        for (int w = 0; w < nW && !dead; ++w)
+        for (int w = wlo; w < whi && !dead; ++w)
         {
             const int t0 = w * TC_TILES;
             const int nt = min(TC_TILES, nK - t0);
@@ -1487,7 +1513,13 @@ __global__ void __launch_bounds__(TC_THREADS, Cfg::CTAS)
             tc_fence_before();
             __syncthreads();
         }
-        if (myrow < X.NB && lane == 0)
+        if (myrow < X.NB && lane == 0 && G.slices > 1)
+        {
+            G.runs[(size_t) myrow * G.slices + slice] = make_int2(before, kept - before);
+            if (dC && trc != 0.0)
+                dC[myrow] = trc; // the slice that holds the diagonal block (zero before the launch)
+        }
+        else if (myrow < X.NB && lane == 0)
         {
             C.nnzb[myrow] = kept < C.MB ? kept : C.MB;
             atomicMax(&flags[1], kept);
@@ -1521,6 +1553,70 @@ __global__ void __launch_bounds__(TC_THREADS, Cfg::CTAS)
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(TCOLS)
                      : "memory");
+}
+
+// The blocks that the slices of a group kept, moved together row by row.
+// Every block moves to its place or a lower one, past blocks already moved, so
+// a CTA moves as many at a time as it has warps: all read, then all written.
+template <typename T>
+__global__ void __launch_bounds__(256) tc_close_kernel(TcOut<T> C, int NB, const int2 *runs, int slices, int *flags)
+{
+    constexpr int W = 8, V = TB * TB * (int) sizeof(T) / 16 / 32 / 4; // 16-byte words of a lane in a quarter block
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (flags[2] || flags[3]) // the product is void and the runs may be missing
+        return;
+    for (int ib = blockIdx.x; ib < NB; ib += gridDim.x)
+    {
+        const int2 *r = runs + (size_t) ib * slices;
+        int total = 0;
+        for (int s = 0; s < slices; ++s)
+            total += r[s].y;
+        for (int b = 0; b < total; b += W)
+        {
+            const int d = b + warp;
+            int src = d;
+            if (d < total)
+            {
+                int s = 0, pre = 0;
+                while (d >= pre + r[s].y)
+                    pre += r[s++].y;
+                src = r[s].x + d - pre;
+            }
+            const bool move = d < total && src != d;
+            if (!__syncthreads_or(move))
+                continue;
+            const uint4 *from = reinterpret_cast<const uint4 *>(C.pool + ((size_t) ib * C.MB + src) * C.slot) + lane;
+            uint4 *to = reinterpret_cast<uint4 *>(C.pool + ((size_t) ib * C.MB + d) * C.slot) + lane;
+            int kb = 0;
+            for (int h = 0; h < 4; ++h)
+            {
+                uint4 v[V];
+                if (move)
+                {
+#pragma unroll
+                    for (int u = 0; u < V; ++u)
+                        v[u] = from[(h * V + u) * 32];
+                    if (h == 0)
+                        kb = C.indexb[(size_t) ib * C.MB + src];
+                }
+                __syncthreads();
+                if (move)
+                {
+#pragma unroll
+                    for (int u = 0; u < V; ++u)
+                        to[(h * V + u) * 32] = v[u];
+                    if (h == 0 && lane == 0)
+                        C.indexb[(size_t) ib * C.MB + d] = kb;
+                }
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x == 0)
+        {
+            C.nnzb[ib] = total;
+            atomicMax(&flags[1], total);
+        }
+    }
 }
 
 } // namespace
@@ -1581,7 +1677,39 @@ bool tc_launch(B200Context *c, const bml_matrix_ellblock_t *X, bml_matrix_ellblo
     k<<<grid, TC_THREADS, smem, c->stream>>>(
         tc_view<T>(X), TcOut<T>{static_cast<T *>(X2->d_pool), X2->d_indexb, X2->d_nnzb, X2->MB, X2->slot_elems}, tab,
         img, zimg, threshold, rowmax, colmax, dA, dC, flags);
-    return LAUNCH_OK("tc_x2_kernel");
+    if (!LAUNCH_OK("tc_x2_kernel"))
+        return false;
+    if (tab.slices > 1)
+    {
+        tc_close_kernel<T><<<std::min(X->NB, c->sm_count * 8), 256, 0, c->stream>>>(
+            TcOut<T>{static_cast<T *>(X2->d_pool), X2->d_indexb, X2->d_nnzb, X2->MB, X2->slot_elems}, X->NB, tab.runs,
+            tab.slices, flags);
+        if (!LAUNCH_OK("tc_close_kernel"))
+            return false;
+    }
+    return true;
+}
+
+// CTAs that share a group's waves: with fewer groups than CTAs (up to 16^3
+// blocks in the 8-bit split) a group per CTA leaves most of the SMs idle.
+// Rounds of the grid times the time of an item in units of a whole group's
+// waves, each slice setting its tables up anew (about a tenth of them).
+// Blocks are placed before it is known which earlier ones are kept, so X2 must
+// have room for every block column that the widest group touches.
+static int tc_slices(int ngroups, int grid, int waves, bool room)
+{
+    int best = 1;
+    double cost = 0.0;
+    for (int s = 1; room && s <= std::min(waves, 32); ++s)
+    {
+        const double c = ((ngroups * (long long) s + grid - 1) / grid) * (0.1 + 1.0 / s);
+        if (s == 1 || c < cost)
+        {
+            best = s;
+            cost = c;
+        }
+    }
+    return best;
 }
 
 // The split of the tensor-core X^2: 0 FP16 hi/lo with FP32 accumulation, 1
@@ -1666,9 +1794,11 @@ bool eb_multiply_x2_tc(bml_matrix_ellblock_t *X, bml_matrix_ellblock_t *X2, doub
     tab.pcap = std::max(hf[7], 1);
     tab.wcap = (tab.kcap + tiles - 1) / tiles;
     auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
+    tab.slices = tc_slices(ngroups, grid, tab.wcap, tab.kcap <= X2->MB);
     const size_t J = tab.jcap, K = tab.kcap, P = tab.pcap, W = tab.wcap, g = grid;
-    const size_t sz[9] = {g * J * 4, g * J * 8, g * J, g * (J + 1) * 4, g * K * 4, g * K * 4,
-                          g * P * 4, g * P * 16, g * (W + 1) * 4};
+    const size_t sz[10] = {g * J * 4, g * J * 8, g * J, g * (J + 1) * 4, g * K * 4, g * K * 4,
+                           g * P * 4, g * P * 16, g * (W + 1) * 4,
+                           tab.slices > 1 ? (size_t) NB * tab.slices * sizeof(int2) : 0};
     size_t tab_bytes = 0;
     for (size_t s : sz)
         tab_bytes += al(s);
@@ -1711,10 +1841,12 @@ bool eb_multiply_x2_tc(bml_matrix_ellblock_t *X, bml_matrix_ellblock_t *X2, doub
         tab.ptile = reinterpret_cast<int *>(take(6));
         tab.list = reinterpret_cast<uint4 *>(take(7));
         tab.wstart = reinterpret_cast<int *>(take(8));
+        tab.runs = reinterpret_cast<int2 *>(take(9));
     }
     if (!CUDA_OK(cudaMemsetAsync(flags, 0, 64, c->stream)) ||
         !CUDA_OK(cudaMemsetAsync(zimg, 0, TC_ZERO_BYTES, c->stream)) ||
         !CUDA_OK(cudaMemsetAsync(dA, 0, (size_t) 2 * NB * sizeof(double), c->stream)) ||
+        (tab.slices > 1 && !CUDA_OK(cudaMemsetAsync(tab.runs, 0, sz[9], c->stream))) ||
         (i8 && !CUDA_OK(cudaMemsetAsync(rowmax, 0, 2 * n_scalar * sizeof(unsigned long long), c->stream))))
         return false;
     const int sgrid = (int) std::min((long long) NB * MB, (long long) c->sm_count * 32);
