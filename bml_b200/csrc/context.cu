@@ -120,6 +120,14 @@ B200Context *b200_ctx()
 
 void *b200_scratch(size_t bytes)
 {
+    void *p = b200_scratch_try(bytes);
+    if (!p && b200_ctx())
+        b200_set_error(BML_B200_ERR_ALLOC, "device scratch of %zu bytes", bytes);
+    return p;
+}
+
+void *b200_scratch_try(size_t bytes)
+{
     B200Context *c = b200_ctx();
     if (!c)
         return nullptr;
@@ -135,7 +143,6 @@ void *b200_scratch(size_t bytes)
     if (cudaMallocAsync(&c->scratch, want, c->stream) != cudaSuccess)
     {
         cudaGetLastError();
-        b200_set_error(BML_B200_ERR_ALLOC, "device scratch of %zu bytes", want);
         c->scratch = nullptr;
         return nullptr;
     }

@@ -1,0 +1,1546 @@
+// Tile form of the unordered X^2 of a symmetric ELLPACK matrix: the same
+// result set as the unordered kernel's symmetric form (ellpack_x2_fast.cu;
+// ellpack/bml_multiply_ellpack_typed.c:252-333), with the products formed by
+// FP64 tensor instructions (mma.sync m8n8k4) on 8 x 8 tiles.
+//
+// Why.  The shared-memory accumulator of the unordered kernel is bound by the
+// shared atomics: 0.39 T products/s on the 40^3 lattice's wide iterate, 2 % of
+// the FP64 pipe.  The matrices of this path are local in row order (bands, and
+// runs along x on a lattice), so rows i..i+7 touch nearly the same columns and
+// X packs into 8 x 8 tiles that are a fifth to a half full.  Multiplying the
+// padded tiles costs 5 to 20 times the products of the sparse form, at 37
+// TFLOP/s (18.5 T products/s) and with the sums in registers.
+//
+// X is symmetric, so X^2 = X X^T and C(I,K) = sum_J X(I,J) X(K,J)^T: both
+// operands are tiles of block rows, stored once, in the order in which a
+// warp's lanes hold them (element (r, c) of a tile at 2 (4 r + c % 4) + c / 4,
+// the A fragments of the two k-steps next to each other, so a tile is 16 bytes
+// per lane; as the second operand of X X^T the same order is the B fragment).
+//
+// Work unit: a group is 32 rows (4 tile rows).  A group lists the tile columns
+// J that any of its 4 tile rows touches, with a 4-bit mask and room for four
+// tiles, and a bitmap over J ranked by word.  One warp forms the 32 x 32 block
+// C(G,H), H >= G: it intersects the bitmaps of G and H, and for every common J
+// multiplies the pairs of tiles present (up to 16, two m8n8k4 each) into 16
+// accumulator tiles (64 registers a lane).  The tiles travel through a ring in
+// shared memory, each lane copying (cp.async) what it will read, two columns
+// ahead: from registers loaded one column ahead the kernel waited for L2 (12
+// warps per SM, 29.0 ms on the 40^3 iterate; the ring frees registers for 16
+// warps, 24.3 ms).  Groups of 16 rows would load more tiles per product, of 64
+// would not fit the registers.
+//
+// The kept entries of a block (|c| > threshold, or the diagonal) are packed:
+// 32 row masks and the kept values, in a pool, with the block's place in a
+// table [G][H - G].  Nothing is ordered between warps.  A second kernel
+// writes the rows of C: for a group it walks the blocks (H, G), H <= G,
+// transposed, and then (G, H), so every row comes out in ascending column
+// order, exactly symmetric, and without a sort.
+//
+// The masked product (the adjoint's C = A B at a given pattern) runs on the
+// same kernel, the second operand packed as rows of its transpose, the blocks
+// those that hold an entry of the pattern.
+//
+// Measured against the sparse form on one B200: X^2 of the 40^3 lattice's wide
+// iterate (rows of 825) 65.0 -> 21.3 ms, first X^2 of that lattice (rows of
+// 113) 6.3 -> 2.5 ms, FP32 on 26999 rows 2.08 -> 0.84 ms, a chain of 4096 rows
+// of 340 746 -> 148 us, of 512 rows of 33 74 -> 62 us; the adjoint of 3
+// iterations on the 16^3 lattice 32 -> 21 ms with the host's share.
+// At 40^3 the MMAs that have both tiles take 9.0 ms of the product kernel's 18,
+// those in a pair with only one about 2; the rest is the handling of a common
+// column (4.4 products on average there, 7.8 at 30^3).
+#include "device_util.cuh"
+
+#include <algorithm>
+#include <climits>
+#include <cstring>
+#include <type_traits>
+
+using namespace b200;
+
+namespace {
+
+constexpr int GR = 32;             // rows of a group
+constexpr int PT = 256;            // threads of the per-row and checking kernels
+// A group's rows are read by a warp each and written by 32 warps: with 8 warps
+// a group, the 128 groups of a 4096-row chain took 64 us to pack and 36 us to
+// write (22 and 18 us so); 2000 groups gain a few per cent.
+constexpr int FT = 1024, RT = 1024;
+constexpr int TW = 4;              // warps of a product CTA
+constexpr int TMIN = 4;            // CTAs per SM: 128 registers a thread
+constexpr int SG = 48, SC = 32;    // a patch of blocks (G, H - G)
+constexpr int TS = 3;              // common tile columns whose tiles a warp has in flight or in use
+constexpr int QCAP = 128;          // common tile columns a warp lists at a time (at least 32)
+constexpr int WARP_SMEM = TS * 4096 + QCAP * 8;
+constexpr size_t TL_SMALL = 40960; // place in the context's small buffers
+
+// The tile form runs when its tile products, at TILE_COST sparse products
+// each, are fewer than the sparse form's (X^2 of random band patterns, tile
+// form against sparse form in us, by sparse products per tile product: 0.33
+// 3880 to 7360 / 3840, 0.64 2050 / 2110, 1.45 (2000 rows) 167 to 185 / 134,
+// 1.88 847 / 1770, 1.94 370 / 807, 5.3 140 / 475; lattices have 8 to 70).
+constexpr double TILE_COST = 1.5;
+constexpr long long LAZY_BYTES = 128 << 20; // most tile places of a matrix laid out without counting them
+
+struct TileFlags
+{
+    unsigned long long products; // sum over rows of width^2 (the sparse form's products, X symmetric)
+    unsigned long long tiles2;   // sum over tile rows of tiles^2 (tile products)
+    unsigned long long pool;     // words of the packed result taken
+    int entries;                 // (group, J) entries of X
+    int reach;                   // largest |column - row|
+    int bad;                     // a row length or column out of range
+    int odd;                     // an entry not finite, or a row of zeros only: not for this form
+    int asym;
+    int next;                    // work item counter
+    int full;                    // the pool ran out
+    int overflow, max_width;
+    int done;                    // CTAs of the row kernel that have finished
+    int blocks;                  // blocks of the masked product
+    double trA, trC;
+};
+
+struct TileArgs
+{
+    const void *Xv; const int *Xi; const int *Xn; int ld; int N; int ncols;
+    int NG, nw;                  // groups; words of a group's bitmap
+    unsigned *bits;              // [NG][nw] union bitmap over tile columns
+    unsigned short *rank;        // [NG][nw] entries before the word
+    int *eoff;                   // first entry of the group
+    int2 *range;                 // words {first, last} of the group's bitmap that are used
+    int *last;                   // last group H whose block with G can be non-zero
+    unsigned *ent;               // entry << 4 | mask of the tile rows present; its tiles at 4 entry + row
+    unsigned short *entJ;        // tile column of an entry
+    double *tiles;               // 64 doubles per tile, four places per entry
+    int lazy;                    // no counting pass: the fill kernel counts
+    int *tab; int span;          // [NG][span] place of block (G, G + s) in the pool, or -1
+    unsigned long long *pool; unsigned long long cap;
+    void *Cv; int *Ci; int *Cn; int ldc; int Mc;
+    double thr;
+    double *dA, *dC;             // per-group sums of the diagonals of X and X^2
+    TileFlags *flags;
+    // second operand, as rows of its transpose (the sparse X^2: the same lists)
+    const unsigned *bitsB; const unsigned short *rankB; const int *eoffB; const int2 *rangeB;
+    // masked product
+    unsigned *gb;                // [NG][4][nw] bitmaps of the transpose of X, made by its rows
+    const int *Pi; const int *Pn; int ldp; int hw; // pattern; words of a bitmap over groups
+    unsigned *pbits; int *prank; // [NG][hw] groups H with an entry of the pattern, and blocks before the word
+    int2 *pblk;                  // blocks (G, H) of the pattern
+    double *out;                 // 1024 doubles per block
+    int masked, count_only;
+};
+
+// The form does not apply: the kernels after the fill do nothing.
+__device__ __forceinline__ bool declined(const TileFlags *f)
+{
+    return f->bad || f->odd || f->asym || (double) f->tiles2 * TILE_COST > (double) f->products;
+}
+
+// The four tile rows' bitmaps of group G from the stored columns, in shared
+// memory, and which rows are strictly ascending (bit of *order; zero before);
+// false (uniform) when a row or column is out of range.
+__device__ __forceinline__ bool group_bitmaps(const TileArgs &g, int G, unsigned *bm, int *reach, unsigned *order)
+{
+    for (int w = threadIdx.x; w < 4 * g.nw; w += FT)
+        bm[w] = 0u;
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int bad = 0, far = 0;
+    for (int r = warp; r < GR; r += FT / 32)
+    {
+        const int i = G * GR + r;
+        if (i >= g.N)
+            continue;
+        const int n = g.Xn[i];
+        if (n < 0 || n > g.ld)
+        {
+            bad = 1;
+            continue;
+        }
+        unsigned *row = bm + (r >> 3) * g.nw;
+        bool desc = false;
+        for (int p0 = lane; p0 < n; p0 += 128)
+        {
+            int kk[4], next[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+            {
+                const int *at = g.Xi + (size_t) i * g.ld + p0 + 32 * u;
+                kk[u] = p0 + 32 * u < n ? __ldg(at) : i;
+                next[u] = p0 + 32 * u + 1 < n ? __ldg(at + 1) : INT_MAX;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+            {
+                const int k = kk[u];
+                if (p0 + 32 * u >= n)
+                    continue;
+                desc |= next[u] <= k;
+                if (k < 0 || k >= g.ncols)
+                {
+                    bad = 1;
+                    continue;
+                }
+                far = max(far, abs(k - i));
+                const unsigned bit = 1u << ((k >> 3) & 31);
+                if (!(*(volatile unsigned *) &row[k >> 8] & bit))
+                    atomicOr(&row[k >> 8], bit);
+            }
+        }
+        if (order && !__any_sync(FULL, desc) && lane == 0)
+            atomicOr(order, 1u << r);
+    }
+    *reach = far;
+    return __syncthreads_or(bad) == 0;
+}
+
+// Tiles of each tile row and entries of group G (tot[0..4], zero before), and
+// its share of both forms' products and of the reach.
+__device__ __forceinline__ void group_counts(const TileArgs &g, int G, const unsigned *bm, int far, int *tot)
+{
+    int c[5] = {0, 0, 0, 0, 0};
+    for (int w = threadIdx.x; w < g.nw; w += FT)
+    {
+        unsigned any = 0u;
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+        {
+            const unsigned b = bm[a * g.nw + w];
+            c[a] += __popc(b);
+            any |= b;
+        }
+        c[4] += __popc(any);
+    }
+    unsigned long long n2 = 0;
+    if (threadIdx.x < GR && G * GR + threadIdx.x < g.N)
+    {
+        const unsigned long long n = (unsigned long long) g.Xn[G * GR + threadIdx.x];
+        n2 = n * n;
+    }
+    for (int o = 16; o; o >>= 1)
+    {
+#pragma unroll
+        for (int a = 0; a < 5; ++a)
+            c[a] += __shfl_xor_sync(FULL, c[a], o);
+        n2 += __shfl_xor_sync(FULL, n2, o);
+        far = max(far, __shfl_xor_sync(FULL, far, o));
+    }
+    if ((threadIdx.x & 31) == 0)
+    {
+#pragma unroll
+        for (int a = 0; a < 5; ++a)
+            if (c[a])
+                atomicAdd(&tot[a], c[a]);
+        if (n2)
+            atomicAdd(&g.flags->products, n2);
+        if (far > *(volatile int *) &g.flags->reach)
+            atomicMax(&g.flags->reach, far);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        unsigned long long t2 = 0;
+        for (int a = 0; a < 4; ++a)
+            t2 += (unsigned long long) tot[a] * tot[a];
+        atomicAdd(&g.flags->tiles2, t2);
+    }
+}
+
+// Counts: tiles, entries and the products of both forms.
+__global__ void __launch_bounds__(FT) tile_count_kernel(TileArgs g)
+{
+    extern __shared__ unsigned bm[];
+    __shared__ int tot[5];
+    for (int G = blockIdx.x; G < g.NG; G += gridDim.x)
+    {
+        if (threadIdx.x < 5)
+            tot[threadIdx.x] = 0;
+        int far = 0;
+        if (!group_bitmaps(g, G, bm, &far, nullptr))
+        {
+            if (threadIdx.x == 0)
+                atomicExch(&g.flags->bad, 1);
+            return;
+        }
+        group_counts(g, G, bm, far, tot);
+        if (threadIdx.x == 0)
+        {
+            atomicAdd(&g.flags->entries, tot[4]);
+        }
+        __syncthreads();
+    }
+}
+
+__device__ __forceinline__ int tile_at(int r, int c) { return 2 * (4 * r + (c & 3)) + (c >> 2); }
+
+// Lists, zero-filled tiles and the scatter of group G's entries.  Rows in
+// ascending order have distinct columns and are stored; other rows are added
+// (duplicate columns add up, as they do in the sparse form).
+template <typename T> __global__ void __launch_bounds__(FT) tile_fill_kernel(TileArgs g)
+{
+    extern __shared__ unsigned bm[]; // [4][nw] bitmaps | [nw] entries before the word
+    int *before = reinterpret_cast<int *>(bm + 4 * g.nw);
+    __shared__ int wsum[FT / 32];
+    __shared__ int run, place;
+    __shared__ unsigned order; // rows in strictly ascending order
+    __shared__ int2 used;
+    __shared__ double diag[GR];
+    __shared__ int tot[5];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    for (int G = blockIdx.x; G < g.NG; G += gridDim.x)
+    {
+        if (tid == 0)
+        {
+            run = 0;
+            order = 0u;
+            used = make_int2(INT_MAX, -1);
+        }
+        if (tid < 5)
+            tot[tid] = 0;
+        int far = 0;
+        if (g.gb)
+        {
+            for (int w = tid; w < 4 * g.nw; w += FT)
+                bm[w] = g.gb[(size_t) G * 4 * g.nw + w];
+            __syncthreads();
+        }
+        else if (!group_bitmaps(g, G, bm, &far, &order))
+        {
+            if (tid == 0)
+                atomicExch(&g.flags->bad, 1);
+            return;
+        }
+        if (g.lazy)
+            group_counts(g, G, bm, far, tot);
+        for (int s = tid; s < g.span; s += FT)
+            g.tab[(size_t) G * g.span + s] = -1;
+        if (tid == 0 && !g.masked)
+            g.dC[G] = 0.0;
+        // entries before every word (block prefix, FT words at a time)
+        for (int w0 = 0; w0 < g.nw; w0 += FT)
+        {
+            const int w = w0 + tid;
+            const unsigned any =
+                w < g.nw ? bm[w] | bm[g.nw + w] | bm[2 * g.nw + w] | bm[3 * g.nw + w] : 0u;
+            const int n = __popc(any);
+            int sum = n;
+            for (int o = 1; o < 32; o <<= 1)
+            {
+                const int u = __shfl_up_sync(FULL, sum, o);
+                if (lane >= o)
+                    sum += u;
+            }
+            if (lane == 31)
+                wsum[warp] = sum;
+            __syncthreads();
+            int base = run;
+            for (int v = 0; v < warp; ++v)
+                base += wsum[v];
+            if (w < g.nw)
+            {
+                g.bits[(size_t) G * g.nw + w] = any;
+                g.rank[(size_t) G * g.nw + w] = (unsigned short) (base + sum - n);
+                before[w] = base + sum - n;
+                if (any)
+                {
+                    atomicMin(&used.x, w);
+                    atomicMax(&used.y, w);
+                }
+            }
+            __syncthreads();
+            if (tid == FT - 1)
+                run = base + sum;
+            __syncthreads();
+        }
+        if (tid == 0)
+        {
+            place = atomicAdd(&g.flags->entries, run);
+            g.eoff[G] = place;
+            g.range[G] = used.y < 0 ? make_int2(0, -1) : used; // an empty group intersects nothing
+        }
+        __syncthreads();
+        const int e0 = place, ne = run;
+        for (int w = tid; w < g.nw; w += FT)
+        {
+            unsigned b[4];
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+                b[a] = bm[a * g.nw + w];
+            unsigned any = b[0] | b[1] | b[2] | b[3];
+            for (int e = e0 + before[w]; any; ++e)
+            {
+                const int q = __ffs(any) - 1;
+                any &= any - 1;
+                unsigned m = 0u;
+#pragma unroll
+                for (int a = 0; a < 4; ++a)
+                    m |= ((b[a] >> q) & 1u) << a;
+                g.ent[e] = (unsigned) e << 4 | m;
+                g.entJ[e] = (unsigned short) (w * 32 + q);
+            }
+        }
+        __syncthreads();
+        double2 *z = reinterpret_cast<double2 *>(g.tiles + (size_t) e0 * 256);
+        for (int p = tid; p < ne * 128; p += FT)
+            if (g.ent[e0 + (p >> 7)] >> ((p >> 5) & 3) & 1u)
+                z[p] = make_double2(0.0, 0.0);
+        __syncthreads();
+        if (g.gb) // the transpose's entries are placed by tile_scatter_kernel
+            continue;
+        int odd = 0;
+        for (int r = warp; r < GR; r += FT / 32)
+        {
+            const int i = G * GR + r;
+            if (i >= g.N)
+            {
+                if (lane == 0)
+                    diag[r] = 0.0;
+                continue;
+            }
+            const int n = g.Xn[i];
+            const T *xv = static_cast<const T *>(g.Xv) + (size_t) i * g.ld;
+            const int *xi = g.Xi + (size_t) i * g.ld;
+            const bool sorted = order >> r & 1u;
+            const int a = r >> 3;
+            bool some = false;
+            double d = 0.0;
+            for (int p0 = lane; p0 < n; p0 += 128)
+            {
+                int kk[4];
+                T vv[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                {
+                    const int p = p0 + 32 * u;
+                    kk[u] = p < n ? __ldg(xi + p) : 0;
+                    vv[u] = p < n ? __ldg(xv + p) : T(0);
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                {
+                    if (p0 + 32 * u >= n)
+                        continue;
+                    const int k = kk[u];
+                    const double v = (double) vv[u];
+                    odd |= !(fabs(v) <= 1.7976931348623157e308);
+                    some |= v != 0.0;
+                    if (k == i)
+                        d += v;
+                    const int w = k >> 8;
+                    const unsigned below = (1u << ((k >> 3) & 31)) - 1u;
+                    const unsigned any = bm[w] | bm[g.nw + w] | bm[2 * g.nw + w] | bm[3 * g.nw + w];
+                    const int t = 4 * (e0 + before[w] + __popc(any & below)) + a;
+                    double *at = g.tiles + (size_t) t * 64 + tile_at(r & 7, k & 7);
+                    if (sorted)
+                        *at = v;
+                    else
+                        atomicAdd(at, v);
+                }
+            }
+            // a stored row of zeros touches its diagonal without a sign of it in the tiles
+            odd |= n > 0 && !__any_sync(FULL, some) && !g.masked;
+            for (int o = 16; o; o >>= 1)
+                d += __shfl_xor_sync(FULL, d, o);
+            if (lane == 0)
+                diag[r] = d;
+        }
+        if (__syncthreads_or(odd) && tid == 0)
+            atomicExch(&g.flags->odd, 1);
+        if (warp == 0 && !g.masked)
+        {
+            double d = diag[lane];
+            for (int o = 16; o; o >>= 1)
+                d += __shfl_xor_sync(FULL, d, o);
+            if (lane == 0)
+                g.dA[G] = d;
+        }
+        __syncthreads();
+    }
+}
+
+// Every tile (I, J), J >= I, against tile (J, I): equal bits, or no tile and
+// zeros.  Also the last group H that has a column in common with G.
+__global__ void __launch_bounds__(PT) tile_sym_kernel(TileArgs g)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ int lastH;
+    if (g.flags->bad)
+        return;
+    for (int G = blockIdx.x; G < g.NG; G += gridDim.x)
+    {
+        if (threadIdx.x == 0)
+            lastH = G;
+        __syncthreads();
+        const int2 rg = g.range[G];
+        int ne = 0;
+        if (rg.y >= 0)
+            ne = g.rank[(size_t) G * g.nw + rg.y] + __popc(g.bits[(size_t) G * g.nw + rg.y]);
+        int last = G, asym = 0;
+        for (int e = warp; e < ne; e += PT / 32)
+        {
+            const unsigned en = g.ent[g.eoff[G] + e];
+            const int J = g.entJ[g.eoff[G] + e];
+            const int H = J >> 2;
+            const int2 rh = H < g.NG ? g.range[H] : make_int2(0, -1);
+            if (rh.y >= 0)
+            {
+                // the last tile column of group H
+                const unsigned b = g.bits[(size_t) H * g.nw + rh.y];
+                last = max(last, (rh.y * 32 + 31 - __clz(b)) >> 2);
+            }
+            if (J < 4 * G)
+                continue;
+            const double2 *tp = reinterpret_cast<const double2 *>(g.tiles) + (size_t) (en >> 4) * 128 + lane;
+            for (int a = 0; a < 4; ++a)
+            {
+                if (!(en >> a & 1u))
+                    continue;
+                const double2 x = tp[32 * a];
+                const int I = 4 * G + a;
+                double m0 = 0.0, m1 = 0.0;
+                const unsigned b = rh.y >= 0 ? g.bits[(size_t) H * g.nw + (I >> 5)] : 0u;
+                if (b >> (I & 31) & 1u)
+                {
+                    const int f = g.eoff[H] + g.rank[(size_t) H * g.nw + (I >> 5)] + __popc(b & ((1u << (I & 31)) - 1u));
+                    const unsigned fn = g.ent[f];
+                    const int u = J & 3;
+                    if (fn >> u & 1u)
+                    {
+                        const double *q = g.tiles + (size_t) (4 * (fn >> 4) + u) * 64;
+                        const int r = lane >> 2, c = lane & 3;
+                        m0 = q[tile_at(c, r)];
+                        m1 = q[tile_at(c + 4, r)];
+                    }
+                }
+                asym |= x.x != m0 || x.y != m1;
+            }
+        }
+        for (int o = 16; o; o >>= 1)
+            last = max(last, __shfl_xor_sync(FULL, last, o));
+        if (lane == 0)
+            atomicMax(&lastH, last);
+        asym = __syncthreads_or(asym);
+        if (threadIdx.x == 0)
+        {
+            g.last[G] = min(lastH, g.NG - 1);
+            if (asym)
+                atomicExch(&g.flags->asym, 1);
+        }
+        __syncthreads();
+    }
+}
+
+template <typename T> __device__ __forceinline__ bool over(T x, double thr);
+template <> __device__ __forceinline__ bool over<double>(double x, double thr) { return fabs(x) > thr; }
+template <> __device__ __forceinline__ bool over<float>(float x, double thr) { return fabsf(x) > (float) thr; }
+
+#define TILE_BITS(E)                                                                                                    \
+    "{\n\t.reg .pred p0, p1, p2, p3;\n\t.reg .b32 t;\n\t"                                                             \
+    "and.b32 t, " E ", 1;\n\tsetp.ne.b32 p0, t, 0;\n\tand.b32 t, " E ", 2;\n\tsetp.ne.b32 p1, t, 0;\n\t"               \
+    "and.b32 t, " E ", 4;\n\tsetp.ne.b32 p2, t, 0;\n\tand.b32 t, " E ", 8;\n\tsetp.ne.b32 p3, t, 0;\n\t"
+
+// The tiles present of one entry into a stage, 16 bytes per lane each.  An
+// entry has room for four tiles, so a tile's place is the entry's plus a
+// constant.
+__device__ __forceinline__ void copy_tiles(unsigned dst, const double2 *tiles, unsigned en)
+{
+    asm volatile(TILE_BITS("%2")
+                 "@p0 cp.async.cg.shared.global [%0], [%1], 16;\n\t"
+                 "@p1 cp.async.cg.shared.global [%0 + 512], [%1 + 512], 16;\n\t"
+                 "@p2 cp.async.cg.shared.global [%0 + 1024], [%1 + 1024], 16;\n\t"
+                 "@p3 cp.async.cg.shared.global [%0 + 1536], [%1 + 1536], 16;\n\t}" ::"r"(dst),
+                 "l"(tiles + (size_t) (en >> 4) * 128), "r"(en)
+                 : "memory");
+}
+
+// The same tiles from the stage (each lane reads what it copied).
+__device__ __forceinline__ void load_tiles(unsigned src, unsigned en, double2 (&f)[4])
+{
+    asm volatile(TILE_BITS("%9")
+                 "@p0 ld.shared.v2.f64 {%0, %1}, [%8];\n\t"
+                 "@p1 ld.shared.v2.f64 {%2, %3}, [%8 + 512];\n\t"
+                 "@p2 ld.shared.v2.f64 {%4, %5}, [%8 + 1024];\n\t"
+                 "@p3 ld.shared.v2.f64 {%6, %7}, [%8 + 1536];\n\t}"
+                 : "+d"(f[0].x), "+d"(f[0].y), "+d"(f[1].x), "+d"(f[1].y), "+d"(f[2].x), "+d"(f[2].y), "+d"(f[3].x),
+                   "+d"(f[3].y)
+                 : "r"(src), "r"(en)
+                 : "memory");
+}
+
+#define TILE_MMA(P, C0, C1, AX, BX) \
+    "@" P " mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {" C0 ", " C1 "}, {" AX "}, {" BX "}, {" C0 ", " C1 "};\n\t"
+
+// A tile of the first operand against two adjacent ones of the second, where
+// present; the first k-step of both before the second of either, so that no
+// MMA waits for the one before it.
+__device__ __forceinline__ void mul_pair(unsigned bit0, unsigned bit1, const double2 &A, const double2 &B0,
+                                         const double2 &B1, double (&c0)[2], double (&c1)[2])
+{
+    asm volatile("{\n\t.reg .pred p0, p1;\n\tsetp.ne.b32 p0, %10, 0;\n\tsetp.ne.b32 p1, %11, 0;\n\t"
+                 TILE_MMA("p0", "%0", "%1", "%4", "%6") TILE_MMA("p1", "%2", "%3", "%4", "%8")
+                 TILE_MMA("p0", "%0", "%1", "%5", "%7") TILE_MMA("p1", "%2", "%3", "%5", "%9") "}"
+                 : "+d"(c0[0]), "+d"(c0[1]), "+d"(c1[0]), "+d"(c1[1])
+                 : "d"(A.x), "d"(A.y), "d"(B0.x), "d"(B0.y), "d"(B1.x), "d"(B1.y), "r"(bit0), "r"(bit1));
+}
+
+// An MMA whose predicate is off still takes its cycles of the tensor pipe (75 %
+// busy with half of its instructions off, when only the rows of the first
+// operand were branched over), so pairs without a tile are branched over too:
+// the masks are mostly runs.  X^2 of the 40^3 iterate: 24.3 ms with a branch
+// per row, 21.9 per pair, 24.8 per tile, 22.2 with a jump on the second mask,
+// 36.0 with a jump on both (225 straight pieces miss the instruction cache).
+__device__ __forceinline__ void mul_tiles(unsigned ea, unsigned eb, const double2 (&A)[4], const double2 (&B)[4],
+                                          double (&acc)[4][4][2])
+{
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+        if (ea >> a & 1u)
+        {
+            if (eb & 3u)
+                mul_pair(eb & 1u, eb & 2u, A[a], B[0], B[1], acc[a][0], acc[a][1]);
+            if (eb & 12u)
+                mul_pair(eb & 4u, eb & 8u, A[a], B[2], B[3], acc[a][2], acc[a][3]);
+        }
+}
+
+// Blocks C(G, H): one warp each, TW consecutive H per CTA (they share G's
+// tiles in L1).
+template <typename T, bool MASKED> __global__ void __launch_bounds__(TW * 32, TMIN) tile_x2_kernel(TileArgs g)
+{
+    extern __shared__ __align__(16) unsigned char tsm[]; // per warp: stages[TS][8 tiles] | queue[QCAP]
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (MASKED ? g.flags->odd : declined(g.flags))
+        return;
+    uint2 *qu = reinterpret_cast<uint2 *>(tsm + warp * WARP_SMEM + TS * 4096);
+    const unsigned stage0 = (unsigned) __cvta_generic_to_shared(tsm + warp * WARP_SMEM) + lane * 16;
+    const double2 *tiles = reinterpret_cast<const double2 *>(g.tiles) + lane;
+    // blocks in patches of SG x SC of (G, H - G), claimed by warps: the blocks in flight read a compact set of
+    // groups from L2
+    const int pc = (g.span + SC - 1) / SC;
+    const int items = MASKED ? g.flags->blocks : (g.NG + SG - 1) / SG * pc * (SG * SC);
+    for (;;)
+    {
+        int it = 0;
+        if (lane == 0)
+            it = atomicAdd(&g.flags->next, 1);
+        it = __shfl_sync(FULL, it, 0);
+        if (it >= items)
+            break;
+        int G, H, s = 0;
+        if (MASKED)
+        {
+            const int2 e = g.pblk[it];
+            G = e.x;
+            H = e.y;
+        }
+        else
+        {
+            const int patch = it / (SG * SC), in = it % (SG * SC);
+            G = patch / pc * SG + in % SG;
+            s = patch % pc * SC + in / SG;
+            H = G + s;
+            if (G >= g.NG || s >= g.span || H > g.last[G])
+                continue;
+        }
+        const int2 ra = g.range[G], rb = g.rangeB[H];
+        const int wlo = max(ra.x, rb.x), whi = min(ra.y, rb.y);
+        const int ea0 = g.eoff[G], eb0 = g.eoffB[H];
+        double acc[4][4][2];
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+                acc[a][b][0] = acc[a][b][1] = 0.0;
+        bool any = false;
+        double2 A[4], Bf[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+            A[a] = Bf[a] = make_double2(0.0, 0.0);
+        int n = 0, w0 = wlo;
+        unsigned a = 0u, b = 0u, c = 0u, xa = 0u, xb = 0u;
+        for (;;)
+        {
+            // common tile columns into the queue, as many as fit; a lane holds one word of the bitmaps
+            while (!__any_sync(FULL, c != 0u) && w0 <= whi)
+            {
+                const int w = w0 + lane;
+                c = 0u;
+                if (w <= whi)
+                {
+                    a = __ldg(g.bits + (size_t) G * g.nw + w);
+                    b = __ldg(g.bitsB + (size_t) H * g.nw + w);
+                    xa = g.rank[(size_t) G * g.nw + w];
+                    xb = g.rankB[(size_t) H * g.nw + w];
+                    c = a & b;
+                }
+                w0 += 32;
+            }
+            const bool end = !__any_sync(FULL, c != 0u);
+            if (!end)
+            {
+                any = true;
+                const int cnt = __popc(c);
+                int pre = cnt;
+                for (int o = 1; o < 32; o <<= 1)
+                {
+                    const int u = __shfl_up_sync(FULL, pre, o);
+                    if (lane >= o)
+                        pre += u;
+                }
+                const bool fits = n + pre <= QCAP; // a prefix of the lanes
+                const int nfit = __popc(__ballot_sync(FULL, fits));
+                if (fits)
+                {
+                    int at = n + pre - cnt;
+                    while (c)
+                    {
+                        const unsigned below = (c & (0u - c)) - 1u;
+                        qu[at++].x = (xa + __popc(a & below)) | (xb + __popc(b & below)) << 16;
+                        c &= c - 1;
+                    }
+                }
+                if (nfit)
+                    n += __shfl_sync(FULL, pre, nfit - 1);
+                __syncwarp();
+                if (!__any_sync(FULL, c != 0u) && w0 <= whi && n + 32 <= QCAP)
+                    continue; // room for more
+            }
+            // the entries' tiles through the ring, TS - 1 columns ahead
+            __syncwarp();
+            for (int t = lane; t < n; t += 32)
+            {
+                const unsigned q = qu[t].x;
+                qu[t] = make_uint2(__ldg(g.ent + ea0 + (q & 0xffffu)), __ldg(g.ent + eb0 + (q >> 16)));
+            }
+            __syncwarp();
+            auto issue = [&](int t) {
+                if (t < n)
+                {
+                    const uint2 e = qu[t];
+                    const unsigned st = stage0 + (t % TS) * 4096;
+                    copy_tiles(st, tiles, e.x);
+                    copy_tiles(st + 2048, tiles, e.y);
+                }
+                asm volatile("cp.async.commit_group;" ::: "memory");
+            };
+#pragma unroll
+            for (int t = 0; t < TS - 1; ++t)
+                issue(t);
+            for (int t = 0; t < n; ++t)
+            {
+                asm volatile("cp.async.wait_group %0;" ::"n"(TS - 2) : "memory");
+                const uint2 e = qu[t];
+                const unsigned st = stage0 + (t % TS) * 4096;
+                load_tiles(st, e.x, A);
+                load_tiles(st + 2048, e.y, Bf);
+                issue(t + TS - 1); // into the stage of column t - 1, whose loads have been used
+                mul_tiles(e.x, e.y, A, Bf, acc);
+            }
+            n = 0;
+            __syncwarp();
+            if (end)
+                break;
+        }
+        if (MASKED)
+        {
+            double *o = g.out + (size_t) it * 1024 + (lane >> 2) * 32 + 2 * (lane & 3);
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int b = 0; b < 4; ++b)
+                    *reinterpret_cast<double2 *>(o + a * 256 + 8 * b) = make_double2(acc[a][b][0], acc[a][b][1]);
+            continue;
+        }
+        if (!any)
+            continue;
+
+        // keep, pack, and place in the pool
+        const bool dg = G == H;
+        const int q4 = lane >> 2;
+        unsigned mask[4];
+        int pre[4], total = 0;
+        double dsum = 0.0;
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+        {
+            const int r = 8 * a + q4, i = G * GR + r;
+            const bool live = dg && i < g.N && g.Xn[i] > 0; // the diagonal is touched
+            unsigned m = 0u;
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                {
+                    const int c = 8 * b + 2 * (lane & 3) + h;
+                    const T x = (T) acc[a][b][h];
+                    bool keep = over<T>(x, g.thr);
+                    if (dg)
+                    {
+                        keep = c == r ? live : keep && c > r;
+                        if (c == r && live)
+                            dsum += (double) x;
+                    }
+                    m |= (keep ? 1u : 0u) << c;
+                }
+            m |= __shfl_xor_sync(FULL, m, 1);
+            m |= __shfl_xor_sync(FULL, m, 2);
+            mask[a] = m;
+            const int cnt = __popc(m);
+            int p = cnt;
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1)
+            {
+                const int u = __shfl_up_sync(FULL, p, o);
+                if (lane >= o)
+                    p += u;
+            }
+            pre[a] = total + p - cnt;
+            total += __shfl_sync(FULL, p, 31);
+        }
+        if (dg)
+        {
+            for (int o = 16; o; o >>= 1)
+                dsum += __shfl_xor_sync(FULL, dsum, o);
+            if (lane == 0)
+                g.dC[G] = dsum;
+        }
+        if (total == 0)
+            continue;
+        const unsigned long long need = 16 + ((unsigned long long) total * sizeof(T) + 7) / 8;
+        unsigned long long at = 0;
+        if (lane == 0)
+            at = atomicAdd(&g.flags->pool, need);
+        at = __shfl_sync(FULL, at, 0);
+        if (at + need > g.cap)
+        {
+            if (lane == 0)
+                atomicExch(&g.flags->full, 1);
+            continue;
+        }
+        unsigned *head = reinterpret_cast<unsigned *>(g.pool + at);
+        T *vals = reinterpret_cast<T *>(g.pool + at + 16);
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+        {
+            if ((lane & 3) == 0)
+                head[8 * a + q4] = mask[a];
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                {
+                    const int c = 8 * b + 2 * (lane & 3) + h;
+                    if (mask[a] >> c & 1u)
+                        vals[pre[a] + __popc(mask[a] & ((1u << c) - 1u))] = (T) acc[a][b][h];
+                }
+        }
+        if (lane == 0)
+            g.tab[(size_t) G * g.span + s] = (int) at;
+    }
+}
+
+// Transpose of a 32 x 32 bit matrix, row `lane` in each lane.
+__device__ __forceinline__ unsigned transpose_bits(unsigned x, int lane)
+{
+    unsigned m = 0x0000ffffu;
+#pragma unroll
+    for (int j = 16; j; j >>= 1)
+    {
+        const unsigned y = __shfl_xor_sync(FULL, x, j);
+        x = (lane & j) ? ((x & ~m) | ((y & ~m) >> j)) : ((x & m) | ((y & m) << j));
+        m ^= m << (j >> 1);
+    }
+    return x;
+}
+
+// Rows of C: one CTA per group.  Shared memory: the group's blocks in column
+// order ({place, column group * 2 + transposed}), at most 2 span of them.
+template <typename T> __global__ void __launch_bounds__(RT) tile_rows_kernel(TileArgs g)
+{
+    extern __shared__ int2 blk[];
+    constexpr int W = RT / 32;
+    __shared__ int cnt[W][32];
+    __shared__ int wtot[W];
+    __shared__ int nblk;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (declined(g.flags) || g.flags->full)
+        return;
+    for (int G = blockIdx.x; G < g.NG; G += gridDim.x)
+    {
+        // candidates in column order: (G - span + 1 + c, G) transposed for c < span, then (G, G + c - span)
+        if (tid == 0)
+            nblk = 0;
+        __syncthreads();
+        for (int c0 = 0; c0 < 2 * g.span; c0 += RT)
+        {
+            const int c = c0 + tid;
+            int at = -1, key = 0;
+            if (c < g.span)
+            {
+                const int H = G - g.span + 1 + c;
+                if (H >= 0)
+                    at = g.tab[(size_t) H * g.span + (G - H)];
+                key = H * 2 + 1;
+            }
+            else if (c < 2 * g.span)
+            {
+                const int H = G + c - g.span;
+                if (H < g.NG)
+                    at = g.tab[(size_t) G * g.span + (c - g.span)];
+                key = H * 2;
+            }
+            const unsigned bal = __ballot_sync(FULL, at >= 0);
+            if (lane == 0)
+                wtot[warp] = __popc(bal);
+            __syncthreads();
+            int pos = nblk, all = 0;
+            for (int v = 0; v < W; ++v)
+            {
+                pos += v < warp ? wtot[v] : 0;
+                all += wtot[v];
+            }
+            if (at >= 0)
+                blk[pos + __popc(bal & lanemask_lt())] = make_int2(at, key);
+            __syncthreads();
+            if (tid == 0)
+                nblk += all;
+            __syncthreads();
+        }
+        const int nb = nblk;
+        const int per = (nb + W - 1) / W;
+        const int b0 = min(nb, warp * per), b1 = min(nb, b0 + per);
+        // the masks of output rows (lane = row), transposed blocks strictly below the diagonal
+        auto masks = [&](int2 e, unsigned &own, unsigned &out) {
+            own = __ldg(reinterpret_cast<const unsigned *>(g.pool + e.x) + lane);
+            if (e.y & 1)
+                out = transpose_bits((e.y >> 1) == G ? own & ~(1u << lane) : own, lane);
+            else
+                out = own;
+        };
+        int c = 0;
+        for (int b = b0; b < b1; ++b)
+        {
+            unsigned own, out;
+            masks(blk[b], own, out);
+            c += __popc(out);
+        }
+        cnt[warp][lane] = c;
+        __syncthreads();
+        int off = 0, total = 0;
+        for (int v = 0; v < W; ++v)
+        {
+            off += v < warp ? cnt[v][lane] : 0;
+            total += cnt[v][lane];
+        }
+        const int i0 = G * GR;
+        for (int b = b0; b < b1; ++b)
+        {
+            const int2 e = blk[b];
+            unsigned own, out;
+            masks(e, own, out);
+            const T *vals = reinterpret_cast<const T *>(g.pool + e.x + 16);
+            int p = __popc(own);
+            for (int o = 1; o < 32; o <<= 1)
+            {
+                const int u = __shfl_up_sync(FULL, p, o);
+                if (lane >= o)
+                    p += u;
+            }
+            p -= __popc(own); // values before row `lane` of the block
+            const bool tr = e.y & 1;
+            const int k = (e.y >> 1) * GR + lane;
+#pragma unroll 8
+            for (int r = 0; r < 32; ++r)
+            {
+                const unsigned mr = __shfl_sync(FULL, out, r);
+                const int o = __shfl_sync(FULL, off, r), pr = __shfl_sync(FULL, p, r);
+                if (mr >> lane & 1u)
+                {
+                    const int q = o + __popc(mr & lanemask_lt());
+                    const T x = tr ? vals[p + __popc(own & ((1u << r) - 1u))] : vals[pr + __popc(mr & lanemask_lt())];
+                    if (q < g.Mc)
+                    {
+                        static_cast<T *>(g.Cv)[(size_t) (i0 + r) * g.ldc + q] = x;
+                        g.Ci[(size_t) (i0 + r) * g.ldc + q] = k;
+                    }
+                }
+            }
+            off += __popc(out);
+        }
+        if (warp == 0)
+        {
+            const int i = i0 + lane;
+            if (i < g.N)
+                g.Cn[i] = min(total, g.Mc);
+            int w = total;
+            for (int o = 16; o; o >>= 1)
+                w = max(w, __shfl_xor_sync(FULL, w, o));
+            if (lane == 0)
+            {
+                if (w > *(volatile int *) &g.flags->max_width)
+                    atomicMax(&g.flags->max_width, w);
+                if (w > g.Mc)
+                    atomicExch(&g.flags->overflow, 1);
+            }
+        }
+        __syncthreads();
+    }
+    // the traces, summed over groups in a fixed order by the CTA that finishes last
+    __shared__ double part[2][W];
+    __shared__ int fin;
+    if (tid == 0)
+        fin = atomicAdd(&g.flags->done, 1) == (int) gridDim.x - 1;
+    __syncthreads();
+    if (!fin)
+        return;
+    double a = 0.0, d = 0.0;
+    for (int G = tid; G < g.NG; G += RT)
+    {
+        a += g.dA[G];
+        d += g.dC[G];
+    }
+    for (int o = 16; o; o >>= 1)
+    {
+        a += __shfl_xor_sync(FULL, a, o);
+        d += __shfl_xor_sync(FULL, d, o);
+    }
+    if (lane == 0)
+    {
+        part[0][warp] = a;
+        part[1][warp] = d;
+    }
+    __syncthreads();
+    if (tid == 0)
+    {
+        for (int v = 1; v < W; ++v)
+        {
+            a += part[0][v];
+            d += part[1][v];
+        }
+        g.flags->trA = a;
+        g.flags->trC = d;
+    }
+}
+
+// -------------------------------------------------------------------------
+// Masked product C = A B at P's pattern: the second operand's tiles are those
+// of its transpose, so a block is again a product of two group rows, and only
+// the blocks that hold an entry of P are formed, whole, and read from.
+// -------------------------------------------------------------------------
+
+// Bitmaps of the transpose's groups from B's rows; one warp per row.
+__global__ void __launch_bounds__(PT) tile_tbits_kernel(TileArgs g)
+{
+    const int lane = threadIdx.x & 31, warps = (gridDim.x * PT) >> 5;
+    for (int j = (blockIdx.x * PT + threadIdx.x) >> 5; j < g.N; j += warps)
+    {
+        const int n = g.Xn[j];
+        if (n < 0 || n > g.ld)
+        {
+            if (lane == 0)
+                atomicExch(&g.flags->bad, 1);
+            continue;
+        }
+        if (lane == 0 && n)
+            atomicAdd(&g.flags->products, (unsigned long long) n * n);
+        const unsigned bit = 1u << ((j >> 3) & 31);
+        for (int p = lane; p < n; p += 32)
+        {
+            const int k = g.Xi[(size_t) j * g.ld + p];
+            if (k < 0 || k >= g.ncols)
+            {
+                atomicExch(&g.flags->bad, 1);
+                continue;
+            }
+            unsigned *w = g.gb + (size_t) (k >> 3) * g.nw + (j >> 8);
+            if (!(*(volatile unsigned *) w & bit))
+                atomicOr(w, bit);
+        }
+    }
+}
+
+// Entries of the transpose's groups, and its share of the tile products.
+__global__ void __launch_bounds__(PT) tile_tcount_kernel(TileArgs g)
+{
+    __shared__ int tot[5];
+    for (int G = blockIdx.x; G < g.NG; G += gridDim.x)
+    {
+        if (threadIdx.x < 5)
+            tot[threadIdx.x] = 0;
+        __syncthreads();
+        int c[5] = {0, 0, 0, 0, 0};
+        for (int w = threadIdx.x; w < g.nw; w += PT)
+        {
+            unsigned any = 0u;
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+            {
+                const unsigned b = g.gb[((size_t) G * 4 + a) * g.nw + w];
+                c[a] += __popc(b);
+                any |= b;
+            }
+            c[4] += __popc(any);
+        }
+#pragma unroll
+        for (int a = 0; a < 5; ++a)
+            if (c[a])
+                atomicAdd(&tot[a], c[a]);
+        __syncthreads();
+        if (threadIdx.x == 0)
+        {
+            unsigned long long t2 = 0;
+            for (int a = 0; a < 4; ++a)
+                t2 += (unsigned long long) tot[a] * tot[a];
+            atomicAdd(&g.flags->tiles2, t2);
+            atomicAdd(&g.flags->entries, tot[4]);
+        }
+        __syncthreads();
+    }
+}
+
+// B's entries into the transpose's tiles; one warp per row of B.
+template <typename T> __global__ void __launch_bounds__(PT) tile_scatter_kernel(TileArgs g)
+{
+    const int lane = threadIdx.x & 31, warps = (gridDim.x * PT) >> 5;
+    for (int j = (blockIdx.x * PT + threadIdx.x) >> 5; j < g.N; j += warps)
+    {
+        const int n = g.Xn[j];
+        const T *xv = static_cast<const T *>(g.Xv) + (size_t) j * g.ld;
+        const int *xi = g.Xi + (size_t) j * g.ld;
+        bool desc = false;
+        for (int p = lane; p + 1 < n; p += 32)
+            desc |= xi[p + 1] <= xi[p];
+        const bool sorted = !__any_sync(FULL, desc);
+        const int w = j >> 8;
+        const unsigned below = (1u << ((j >> 3) & 31)) - 1u;
+        bool odd = false;
+        for (int p = lane; p < n; p += 32)
+        {
+            const int k = xi[p], G = k >> 5;
+            const double v = (double) xv[p];
+            odd |= !(fabs(v) <= 1.7976931348623157e308);
+            const size_t at = (size_t) G * g.nw + w;
+            const size_t t = 4 * (size_t) (g.eoff[G] + g.rank[at] + __popc(g.bits[at] & below)) + ((k >> 3) & 3);
+            double *to = g.tiles + t * 64 + tile_at(k & 7, j & 7);
+            if (sorted)
+                *to = v;
+            else
+                atomicAdd(to, v);
+        }
+        if (__any_sync(FULL, odd) && lane == 0)
+            atomicExch(&g.flags->odd, 1);
+    }
+}
+
+// Groups H with an entry of P in the rows of G: counted (count_only), or
+// listed with their ranks.  Shared memory: bitmap[hw].
+__global__ void __launch_bounds__(PT) tile_pattern_kernel(TileArgs g)
+{
+    extern __shared__ unsigned pb[];
+    __shared__ int sum, base;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    for (int G = blockIdx.x; G < g.NG; G += gridDim.x)
+    {
+        for (int w = tid; w < g.hw; w += PT)
+            pb[w] = 0u;
+        if (tid == 0)
+            sum = 0;
+        __syncthreads();
+        for (int r = warp; r < GR; r += PT / 32)
+        {
+            const int i = G * GR + r;
+            const int n = i < g.N ? g.Pn[i] : 0;
+            if (n < 0 || n > g.ldp || n > g.Mc)
+            {
+                if (lane == 0)
+                    atomicExch(&g.flags->bad, 1);
+                continue;
+            }
+            for (int p = lane; p < n; p += 32)
+            {
+                const int k = g.Pi[(size_t) i * g.ldp + p];
+                if (k < 0 || k >= g.ncols)
+                    atomicExch(&g.flags->bad, 1);
+                else if (!(*(volatile unsigned *) &pb[k >> 10] >> ((k >> 5) & 31) & 1u))
+                    atomicOr(&pb[k >> 10], 1u << ((k >> 5) & 31));
+            }
+        }
+        __syncthreads();
+        int c = 0;
+        for (int w = tid; w < g.hw; w += PT)
+            c += __popc(pb[w]);
+        if (c)
+            atomicAdd(&sum, c);
+        __syncthreads();
+        if (tid == 0)
+            base = atomicAdd(&g.flags->blocks, sum);
+        __syncthreads();
+        if (!g.count_only && warp == 0)
+        {
+            int at = base;
+            for (int w0 = 0; w0 < g.hw; w0 += 32)
+            {
+                const int w = w0 + lane;
+                unsigned b = w < g.hw ? pb[w] : 0u;
+                const int n = __popc(b);
+                int pre = n;
+                for (int o = 1; o < 32; o <<= 1)
+                {
+                    const int u = __shfl_up_sync(FULL, pre, o);
+                    if (lane >= o)
+                        pre += u;
+                }
+                if (w < g.hw)
+                {
+                    g.pbits[(size_t) G * g.hw + w] = b;
+                    g.prank[(size_t) G * g.hw + w] = at + pre - n;
+                }
+                for (int e = at + pre - n; b; b &= b - 1, ++e)
+                    g.pblk[e] = make_int2(G, w * 32 + __ffs(b) - 1);
+                at += __shfl_sync(FULL, pre, 31);
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// Row i of C: P's columns with their sums; one warp per row.
+template <typename T> __global__ void __launch_bounds__(PT) tile_gather_kernel(TileArgs g)
+{
+    const int lane = threadIdx.x & 31, warps = (gridDim.x * PT) >> 5;
+    if (g.flags->odd)
+        return;
+    for (int i = (blockIdx.x * PT + threadIdx.x) >> 5; i < g.N; i += warps)
+    {
+        const int n = g.Pn[i], G = i >> 5;
+        for (int p = lane; p < n; p += 32)
+        {
+            const int k = g.Pi[(size_t) i * g.ldp + p];
+            const size_t w = (size_t) G * g.hw + (k >> 10);
+            const int e = g.prank[w] + __popc(g.pbits[w] & ((1u << ((k >> 5) & 31)) - 1u));
+            static_cast<T *>(g.Cv)[(size_t) i * g.ldc + p] = (T) g.out[(size_t) e * 1024 + (i & 31) * 32 + (k & 31)];
+            g.Ci[(size_t) i * g.ldc + p] = k;
+        }
+        if (lane == 0)
+            g.Cn[i] = n;
+    }
+}
+
+template <typename T> bool tile_masked_typed(TileArgs a, TileArgs b, bool *taken)
+{
+    B200Context *c = b200_ctx();
+    if (!c)
+        return false;
+    unsigned char *small = static_cast<unsigned char *>(c->d_small) + TL_SMALL;
+    TileFlags *hf = reinterpret_cast<TileFlags *>(static_cast<unsigned char *>(c->pinned) + TL_SMALL);
+    a.flags = b.flags = reinterpret_cast<TileFlags *>(small);
+    const int NG = a.NG, nw = a.nw;
+    const int per = std::min(NG, c->sm_count * 8);
+    const size_t smemC = (size_t) 4 * nw * sizeof(unsigned), smemF = (size_t) 5 * nw * sizeof(unsigned);
+    const size_t smemP = (size_t) a.hw * sizeof(unsigned);
+    auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        const size_t o = at;
+        at = al(at + bytes);
+        return o;
+    };
+    const size_t o_gb = take((size_t) NG * 4 * nw * sizeof(unsigned));
+    const size_t o_bits = take((size_t) 2 * NG * nw * sizeof(unsigned));
+    const size_t o_rank = take((size_t) 2 * NG * nw * sizeof(unsigned short));
+    const size_t o_eoff = take((size_t) 2 * NG * sizeof(int)), o_range = take((size_t) 2 * NG * sizeof(int2));
+    const size_t o_pb = take((size_t) NG * a.hw * sizeof(unsigned)), o_pr = take((size_t) NG * a.hw * sizeof(int));
+    const size_t fixed = at;
+    unsigned char *scr = nullptr;
+    // the counts, then the layout; a larger arena loses the transpose's bitmaps, which are then made again
+    for (int attempt = 0; attempt < 2; ++attempt)
+    {
+        const bool grown = attempt && (size_t) at > c->scratch_bytes;
+        if (attempt && !grown)
+            break;
+        scr = static_cast<unsigned char *>(b200_scratch_try(attempt ? at : fixed));
+        if (!scr)
+            return true; // the sparse form takes less
+        b.gb = reinterpret_cast<unsigned *>(scr + o_gb);
+        if (!CUDA_OK(cudaMemsetAsync(b.gb, 0, (size_t) NG * 4 * nw * sizeof(unsigned), c->stream)) ||
+            !CUDA_OK(cudaMemsetAsync(small, 0, sizeof(TileFlags), c->stream)))
+            return false;
+        tile_tbits_kernel<<<std::min(b200_ceil_div(b.N, PT / 32), c->sm_count * 8), PT, 0, c->stream>>>(b);
+        if (!LAUNCH_OK("tile_tbits_kernel"))
+            return false;
+        if (attempt)
+            break;
+        tile_tcount_kernel<<<per, PT, 0, c->stream>>>(b);
+        if (!LAUNCH_OK("tile_tcount_kernel"))
+            return false;
+        tile_count_kernel<<<per, FT, smemC, c->stream>>>(a);
+        if (!LAUNCH_OK("tile_count_kernel"))
+            return false;
+        a.count_only = 1;
+        tile_pattern_kernel<<<per, PT, smemP, c->stream>>>(a);
+        if (!LAUNCH_OK("tile_pattern_kernel") ||
+            !CUDA_OK(cudaMemcpyAsync(hf, small, sizeof(TileFlags), cudaMemcpyDeviceToHost, c->stream)) || !b200_sync())
+            return false;
+        if (hf->bad || hf->entries >= (1 << 28) || (double) hf->tiles2 * TILE_COST > (double) hf->products)
+            return true;
+        take(0);
+        const size_t o_ent = take((size_t) hf->entries * sizeof(unsigned));
+        const size_t o_entJ = take((size_t) hf->entries * sizeof(unsigned short));
+        const size_t o_tiles = take((size_t) hf->entries * 2048);
+        const size_t o_blk = take((size_t) hf->blocks * sizeof(int2));
+        const size_t o_out = take((size_t) hf->blocks * 8192);
+        if (at > ((size_t) 64 << 30))
+            return true;
+        a.ent = reinterpret_cast<unsigned *>(o_ent); // offsets until the arena is settled
+        a.entJ = reinterpret_cast<unsigned short *>(o_entJ);
+        a.tiles = reinterpret_cast<double *>(o_tiles);
+        a.pblk = reinterpret_cast<int2 *>(o_blk);
+        a.out = reinterpret_cast<double *>(o_out);
+    }
+    auto place = [&](auto *&p) { p = reinterpret_cast<std::decay_t<decltype(p)>>(scr + reinterpret_cast<size_t>(p)); };
+    place(a.ent);
+    place(a.entJ);
+    place(a.tiles);
+    place(a.pblk);
+    place(a.out);
+    b.ent = a.ent;
+    b.entJ = a.entJ;
+    b.tiles = a.tiles;
+    a.bits = reinterpret_cast<unsigned *>(scr + o_bits);
+    a.rank = reinterpret_cast<unsigned short *>(scr + o_rank);
+    a.eoff = reinterpret_cast<int *>(scr + o_eoff);
+    a.range = reinterpret_cast<int2 *>(scr + o_range);
+    a.bitsB = b.bits = a.bits + (size_t) NG * nw;
+    a.rankB = b.rank = a.rank + (size_t) NG * nw;
+    a.eoffB = b.eoff = a.eoff + NG;
+    a.rangeB = b.range = a.range + NG;
+    a.pbits = reinterpret_cast<unsigned *>(scr + o_pb);
+    a.prank = reinterpret_cast<int *>(scr + o_pr);
+    a.count_only = 0;
+    if (!CUDA_OK(cudaMemsetAsync(small, 0, sizeof(TileFlags), c->stream)))
+        return false;
+    tile_fill_kernel<T><<<per, FT, smemF, c->stream>>>(a);
+    if (!LAUNCH_OK("tile_fill_kernel"))
+        return false;
+    tile_fill_kernel<T><<<per, FT, smemF, c->stream>>>(b);
+    if (!LAUNCH_OK("tile_fill_kernel"))
+        return false;
+    tile_scatter_kernel<T><<<std::min(b200_ceil_div(b.N, PT / 32), c->sm_count * 8), PT, 0, c->stream>>>(b);
+    if (!LAUNCH_OK("tile_scatter_kernel"))
+        return false;
+    tile_pattern_kernel<<<per, PT, smemP, c->stream>>>(a);
+    if (!LAUNCH_OK("tile_pattern_kernel"))
+        return false;
+    const size_t smemQ = (size_t) TW * WARP_SMEM;
+    if (!CUDA_OK(cudaFuncSetAttribute(tile_x2_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int) smemQ)))
+        return false;
+    tile_x2_kernel<T, true><<<c->sm_count * TMIN, TW * 32, smemQ, c->stream>>>(a);
+    if (!LAUNCH_OK("tile_x2_kernel"))
+        return false;
+    tile_gather_kernel<T><<<std::min(b200_ceil_div(a.N, PT / 32), c->sm_count * 8), PT, 0, c->stream>>>(a);
+    if (!LAUNCH_OK("tile_gather_kernel") ||
+        !CUDA_OK(cudaMemcpyAsync(hf, small, sizeof(TileFlags), cudaMemcpyDeviceToHost, c->stream)) || !b200_sync())
+        return false;
+    *taken = !hf->odd && !hf->bad;
+    return true;
+}
+
+template <typename T>
+bool tile_x2_typed(TileArgs g, double *trace, int *required_M, bool *taken, bool *asym, cudaEvent_t *timer)
+{
+    B200Context *c = b200_ctx();
+    if (!c)
+        return false;
+    unsigned char *small = static_cast<unsigned char *>(c->d_small) + TL_SMALL;
+    unsigned char *pin = static_cast<unsigned char *>(c->pinned) + TL_SMALL;
+    TileFlags *hf = reinterpret_cast<TileFlags *>(pin);
+    g.flags = reinterpret_cast<TileFlags *>(small);
+    const int per = (int) std::min<long long>(g.NG, (long long) c->sm_count * 8);
+    const size_t smemC = (size_t) 4 * g.nw * sizeof(unsigned);
+    const size_t smemF = (size_t) 5 * g.nw * sizeof(unsigned); // at most 40 KB
+    if (!CUDA_OK(cudaMemsetAsync(small, 0, sizeof(TileFlags), c->stream)))
+        return false;
+    // Small matrices are laid out for the most tiles they can have, which saves the counting pass and its
+    // round trip; the fill kernel then counts, and the later kernels find the form declined.
+    const long long nbk = b200_ceil_div(g.N, 8);
+    long long entries = std::min((long long) g.NG * nbk, (long long) g.N * g.ld);
+    int span = g.NG;
+    g.lazy = entries * 2048 <= LAZY_BYTES;
+    if (!g.lazy)
+    {
+        tile_count_kernel<<<per, FT, smemC, c->stream>>>(g);
+        if (!LAUNCH_OK("tile_count_kernel") ||
+            !CUDA_OK(cudaMemcpyAsync(pin, small, sizeof(TileFlags), cudaMemcpyDeviceToHost, c->stream)) ||
+            !b200_sync())
+            return false;
+        if (hf->bad || hf->entries <= 0 || hf->entries >= (1 << 28) ||
+            (double) hf->tiles2 * TILE_COST > (double) hf->products)
+            return true;
+        entries = hf->entries;
+        span = std::min(g.NG, 2 * (hf->reach / GR + 1) + 1);
+        // the counters start again at zero: the fill kernel hands out places with them
+        if (!CUDA_OK(cudaMemsetAsync(small, 0, sizeof(TileFlags), c->stream)))
+            return false;
+    }
+    const size_t smemR = (size_t) 2 * span * sizeof(int2);
+    if (smemR > c->smem_optin - 8192)
+        return true;
+    // pool: the kept entries of the upper triangle when no row is wider than M, and a header per block
+    const size_t vals = ((size_t) g.N * ((size_t) g.Mc + 1) / 2 + 1) * sizeof(T) / 8 + 1;
+    const size_t words = vals + (size_t) 17 * g.NG * span;
+    if (words >= ((size_t) 1 << 31))
+        return true;
+    auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        const size_t o = at;
+        at = al(at + bytes);
+        return o;
+    };
+    const size_t o_bits = take((size_t) g.NG * g.nw * sizeof(unsigned));
+    const size_t o_rank = take((size_t) g.NG * g.nw * sizeof(unsigned short));
+    const size_t o_eoff = take((size_t) g.NG * sizeof(int));
+    const size_t o_range = take((size_t) g.NG * sizeof(int2));
+    const size_t o_last = take((size_t) g.NG * sizeof(int));
+    const size_t o_ent = take((size_t) entries * sizeof(unsigned));
+    const size_t o_entJ = take((size_t) entries * sizeof(unsigned short));
+    const size_t o_diag = take((size_t) 2 * g.NG * sizeof(double));
+    const size_t o_tab = take((size_t) g.NG * span * sizeof(int));
+    const size_t o_tiles = take((size_t) entries * 256 * sizeof(double));
+    const size_t o_pool = take(words * 8);
+    if (at > ((size_t) 64 << 30))
+        return true;
+    unsigned char *scr = static_cast<unsigned char *>(b200_scratch_try(at));
+    if (!scr)
+        return true; // the sparse form takes less
+    g.bits = reinterpret_cast<unsigned *>(scr + o_bits);
+    g.rank = reinterpret_cast<unsigned short *>(scr + o_rank);
+    g.eoff = reinterpret_cast<int *>(scr + o_eoff);
+    g.range = reinterpret_cast<int2 *>(scr + o_range);
+    g.last = reinterpret_cast<int *>(scr + o_last);
+    g.ent = reinterpret_cast<unsigned *>(scr + o_ent);
+    g.entJ = reinterpret_cast<unsigned short *>(scr + o_entJ);
+    g.dA = reinterpret_cast<double *>(scr + o_diag);
+    g.dC = g.dA + g.NG;
+    g.tab = reinterpret_cast<int *>(scr + o_tab);
+    g.span = span;
+    g.tiles = reinterpret_cast<double *>(scr + o_tiles);
+    g.pool = reinterpret_cast<unsigned long long *>(scr + o_pool);
+    g.cap = words;
+    g.bitsB = g.bits;
+    g.rankB = g.rank;
+    g.eoffB = g.eoff;
+    g.rangeB = g.range;
+    tile_fill_kernel<T><<<per, FT, smemF, c->stream>>>(g);
+    if (!LAUNCH_OK("tile_fill_kernel"))
+        return false;
+    tile_sym_kernel<<<per, PT, 0, c->stream>>>(g);
+    if (!LAUNCH_OK("tile_sym_kernel"))
+        return false;
+    if (timer && !CUDA_OK(cudaEventRecord(timer[0], c->stream)))
+        return false;
+    const long long items =
+        (long long) ((g.NG + SG - 1) / SG * SG) * ((span + SC - 1) / SC * SC); // counted in an int by the kernel
+    if (items >= 1 << 30)
+        return true;
+    const size_t smemQ = (size_t) TW * WARP_SMEM;
+    if (!CUDA_OK(cudaFuncSetAttribute(tile_x2_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smemQ)))
+        return false;
+    tile_x2_kernel<T, false><<<(int) std::min<long long>((items + TW - 1) / TW, (long long) c->sm_count * TMIN), TW * 32, smemQ,
+                        c->stream>>>(g);
+    if (!LAUNCH_OK("tile_x2_kernel"))
+        return false;
+    if (timer && !CUDA_OK(cudaEventRecord(timer[1], c->stream)))
+        return false;
+    if (smemR > 32768 && !CUDA_OK(cudaFuncSetAttribute(
+                             tile_rows_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smemR)))
+        return false;
+    tile_rows_kernel<T><<<g.NG, RT, smemR, c->stream>>>(g);
+    if (!LAUNCH_OK("tile_rows_kernel"))
+        return false;
+    if (!CUDA_OK(cudaMemcpyAsync(pin, small, sizeof(TileFlags), cudaMemcpyDeviceToHost, c->stream)) || !b200_sync())
+        return false;
+    if (hf->bad || hf->odd || hf->asym || hf->full || (double) hf->tiles2 * TILE_COST > (double) hf->products)
+    {
+        *asym = hf->asym != 0;
+        return true;
+    }
+    *taken = true;
+    if (required_M)
+        *required_M = hf->max_width;
+    if (trace)
+    {
+        trace[0] = hf->trA;
+        trace[1] = hf->trC;
+    }
+    if (hf->overflow)
+    {
+        b200_set_error(BML_B200_ERR_ROW_OVERFLOW, "Number of non-zeroes per row > M, Increase M (need %d, M = %d)",
+                       hf->max_width, g.Mc);
+        return false;
+    }
+    return true;
+}
+
+} // namespace
+
+bool ell_x2_tiles(bml_matrix_ellpack_t *X, bml_matrix_ellpack_t *C, double threshold, double *trace, int *required_M,
+                  bool *taken, bool *asym, cudaEvent_t *timer)
+{
+    *taken = *asym = false;
+    // a place in a group's list is kept in 16 bits
+    const int nbk = b200_ceil_div(X->N, 8);
+    if (!(threshold >= 0.0) || X->N != C->N || X->N < 1 || nbk > 65535)
+        return true;
+    TileArgs g{};
+    g.Xv = X->d_value;
+    g.Xi = X->d_index;
+    g.Xn = X->d_nnz;
+    g.ld = X->ld;
+    g.N = X->N;
+    g.ncols = X->N;
+    g.NG = b200_ceil_div(X->N, GR);
+    g.nw = b200_ceil_div(nbk, 32);
+    g.Cv = C->d_value;
+    g.Ci = C->d_index;
+    g.Cn = C->d_nnz;
+    g.ldc = C->ld;
+    g.Mc = C->M;
+    g.thr = threshold;
+    return X->matrix_precision == double_real ? tile_x2_typed<double>(g, trace, required_M, taken, asym, timer)
+                                              : tile_x2_typed<float>(g, trace, required_M, taken, asym, timer);
+}
+
+bool ell_masked_tiles(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bml_matrix_ellpack_t *P,
+                      bml_matrix_ellpack_t *C, bool *taken)
+{
+    *taken = false;
+    const int nbk = b200_ceil_div(A->N, 8);
+    if (A->N != B->N || A->N != C->N || nbk > 65535)
+        return true;
+    TileArgs a{};
+    a.N = a.ncols = A->N;
+    a.NG = b200_ceil_div(A->N, GR);
+    a.nw = b200_ceil_div(nbk, 32);
+    a.masked = 1;
+    TileArgs b = a;
+    a.Xv = A->d_value;
+    a.Xi = A->d_index;
+    a.Xn = A->d_nnz;
+    a.ld = A->ld;
+    b.Xv = B->d_value;
+    b.Xi = B->d_index;
+    b.Xn = B->d_nnz;
+    b.ld = B->ld;
+    a.Pi = P->d_index;
+    a.Pn = P->d_nnz;
+    a.ldp = P->ld;
+    a.hw = b200_ceil_div(a.NG, 32);
+    a.Cv = C->d_value;
+    a.Ci = C->d_index;
+    a.Cn = C->d_nnz;
+    a.ldc = C->ld;
+    a.Mc = C->M;
+    return A->matrix_precision == double_real ? tile_masked_typed<double>(a, b, taken)
+                                              : tile_masked_typed<float>(a, b, taken);
+}

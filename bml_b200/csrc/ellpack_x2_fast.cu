@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(256) sym_check_kernel(FastArgs g)
 
 // -------------------------------------------------------------------------
 // Product kernel.
-// Shared memory: acc[tile] (T) | touched bits[tile/32] (TOUCH) | cur[lda] (int)
+// Shared memory: acc[tile] (T) | cur[lda] (int)
 // -------------------------------------------------------------------------
 template <typename T> __device__ __forceinline__ bool above(T x, double thr);
 template <> __device__ __forceinline__ bool above<double>(double x, double thr) { return fabs(x) > thr; }
@@ -810,6 +810,13 @@ size_t fast_smem_budget(const B200Context *c)
     return b - sizeof(FastMisc) - 64;
 }
 
+// Whether the product kernel is to be timed (its events exist).
+bool kernel_timer()
+{
+    return g_time_kernel &&
+           (g_kev[0] || (CUDA_OK(cudaEventCreate(&g_kev[0])) && CUDA_OK(cudaEventCreate(&g_kev[1]))));
+}
+
 template <typename T, bool TOUCH> auto fast_kernel()
 {
     return fast_x2_kernel<T, FX_W, FX_U, FX_MINB, TOUCH>;
@@ -921,8 +928,7 @@ bool fast_multiply_typed(FastArgs g, double *trace, int *required_M, bool touch)
         b200_set_error(BML_B200_ERR_UNSUPPORTED, "multiply: the unordered kernel does not fit the device");
         return false;
     }
-    const bool timed = g_time_kernel && (g_kev[0] || (CUDA_OK(cudaEventCreate(&g_kev[0])) &&
-                                                        CUDA_OK(cudaEventCreate(&g_kev[1]))));
+    const bool timed = kernel_timer();
     if (timed && !CUDA_OK(cudaEventRecord(g_kev[0], c->stream)))
         return false;
     kern<<<c->sm_count * occ, FX_W * 32, smemK, c->stream>>>(g);
@@ -1033,6 +1039,20 @@ bool ell_multiply_unordered(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bm
     // the touched columns are needed where untouched zeros could pass the
     // keep rule (threshold < 0 or NaN) or the pre-threshold width is checked
     const bool touch = check_pre || !(threshold >= 0.0);
+    if (g.sym_try && !touch)
+    {
+        bool taken = false, asym = false;
+        const bool timed = kernel_timer();
+        const bool ok = ell_x2_tiles(A, C, threshold, trace, required_M, &taken, &asym, timed ? g_kev : nullptr);
+        if (taken || !ok)
+        {
+            g_last_symmetric = taken;
+            g_last_kernel_ms = -1.0f;
+            return !(timed && taken && !CUDA_OK(cudaEventElapsedTime(&g_last_kernel_ms, g_kev[0], g_kev[1]))) && ok;
+        }
+        if (asym)
+            g.sym_try = 0;
+    }
     return A->matrix_precision == double_real ? fast_multiply_typed<double>(g, trace, required_M, touch)
                                               : fast_multiply_typed<float>(g, trace, required_M, touch);
 }
@@ -1057,6 +1077,18 @@ bool ell_multiply_masked(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bml_m
         C->mirror = MIRROR_SYNCED;
     *taken = true;
     g_last_dense = false;
+    {
+        bool tiles = false;
+        const bool ok = ell_masked_tiles(A, B, P, C, &tiles);
+        if (tiles)
+        {
+            g_last_symmetric = false;
+            g_last_kernel_ms = -1.0f;
+            ell_mark_device(C);
+        }
+        if (tiles || !ok)
+            return ok;
+    }
     FastArgs g{};
     g.Av = A->d_value; g.Ai = A->d_index; g.An = A->d_nnz; g.lda = A->ld; g.NA = A->N;
     g.Bv = B->d_value; g.Bi = B->d_index; g.Bn = B->d_nnz; g.ldb = B->ld; g.NB = B->N;

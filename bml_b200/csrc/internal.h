@@ -109,6 +109,9 @@ struct B200Context
 B200Context *b200_ctx();
 // Device scratch of at least `bytes`, valid until the next call that grows it.
 void *b200_scratch(size_t bytes);
+// The same without a status when the memory is not there, for forms that have
+// another to leave the call to (the arena is empty then).
+void *b200_scratch_try(size_t bytes);
 // Synchronise the library stream; false (error recorded) on failure.
 bool b200_sync();
 
@@ -151,6 +154,16 @@ bool ell_x2_exact();
 bool ell_unordered_fits(const bml_matrix_ellpack_t *A);
 bool ell_multiply_unordered(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bml_matrix_ellpack_t *C,
                             double threshold, double *trace, int *required_M, bool check_pre);
+// The tile form of the unordered X^2 (ellpack_tiles.cu): symmetric X whose rows
+// pack well into 8 x 8 tiles, threshold >= 0.  Leaves *taken false, with no
+// status set, where it does not apply (*asym: X was found not to be
+// symmetric); timer (nullable): events recorded around the product kernel.
+bool ell_x2_tiles(bml_matrix_ellpack_t *X, bml_matrix_ellpack_t *C, double threshold, double *trace, int *required_M,
+                  bool *taken, bool *asym, cudaEvent_t *timer);
+// The tile form of the masked product below; *taken false, with no status
+// set, where it does not apply.
+bool ell_masked_tiles(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bml_matrix_ellpack_t *P,
+                      bml_matrix_ellpack_t *C, bool *taken);
 // C = A*B at P's pattern (the masked form of the unordered product): row i
 // of C lists P's row i columns in P's order with the sums of their products
 // (0 where there are none), no threshold.  *taken is false, with no status

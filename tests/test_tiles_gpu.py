@@ -1,0 +1,197 @@
+"""The tile form of the unordered symmetric X^2 (8 x 8 tiles, groups of 32
+rows) against the C restatement, at the sizes where its tiles, groups and
+bitmap words end: within 1e-12 of S = sum |x_ij x_jk| (FP32: 2 n 2^-24, n
+products per entry), patterns equal except at the threshold, rows ascending,
+the result exactly symmetric, the traces of the same bound."""
+import numpy as np
+import pytest
+import torch
+
+import bml_b200 as B
+import x2check
+
+pytestmark = [pytest.mark.gpu, pytest.mark.unordered]
+SINGLE, DOUBLE = 1, 2
+
+
+def _banded(N, band, density, seed, empty=(), dtype=np.float64):
+    """Symmetric matrix of a band, each pair present with the given
+    probability, rows and columns in `empty` without entries."""
+    rng = np.random.default_rng(seed)
+    D = np.zeros((N, N), dtype)
+    for d in range(0, min(band, N - 1) + 1):
+        x = rng.standard_normal(N - d).astype(dtype) * (rng.random(N - d) < (density if d else 1.0))
+        i = np.arange(N - d)
+        D[i, i + d] = x
+        D[i + d, i] = x
+    D[list(empty), :] = 0
+    D[:, list(empty)] = 0
+    return D
+
+
+def _rows(D, M, shuffle, seed):
+    N = D.shape[0]
+    rng = np.random.default_rng(seed)
+    v, ix, nz = np.zeros((N, M), D.dtype), np.zeros((N, M), np.int32), np.zeros(N, np.int32)
+    for i in range(N):
+        c = np.flatnonzero(D[i])
+        if shuffle:
+            rng.shuffle(c)
+        v[i, :len(c)], ix[i, :len(c)], nz[i] = D[i, c], c, len(c)
+    return v.reshape(-1), ix.reshape(-1), nz
+
+
+def _x2(arrs, N, M, M2, thr, prec):
+    X = B.Ellpack.from_arrays(*arrs, N, M, prec)
+    Y = B.Ellpack(N, M2, prec)
+    st, tr = B.multiply_x2(X, Y, thr)
+    return st, tr, Y.download()
+
+
+def _dense(arrs, N, M):
+    v, ix, nz = arrs
+    D = np.zeros((N, N))
+    for i in range(N):
+        D[i, ix[i * M:i * M + nz[i]]] = v[i * M:i * M + nz[i]]
+    return D
+
+
+def _check(O, D, shuffle, thr, prec, M2=None):
+    N = D.shape[0]
+    M = max(1, int((D != 0).sum(1).max()))
+    M2 = M2 or N
+    arrs = _rows(D, M, shuffle, 3)
+    ref, tr_ref, _ = O.rest_x2(*arrs, N, M, thr, M2, prec)
+    av = np.abs(arrs[0].astype(np.float64))
+    S, _, _ = O.rest_x2(av, arrs[1], arrs[2], N, M, -1.0, M2, DOUBLE)
+    st, tr, got = _x2(arrs, N, M, M2, thr, prec)
+    assert st == B.OK
+    n = int(arrs[2].max())
+    eps = 1e-12 if prec == DOUBLE else 2.0 * n * 2.0 ** -24
+    x2check.compare(got, ref, S, M2, M2, M2, thr, eps)
+    assert x2check.rows_sorted(got, M2)
+    G = _dense(got, N, M2)
+    assert np.array_equal(G, G.T)
+    Sd = np.trace(_dense(S, N, M2))
+    assert abs(tr[0] - tr_ref[0]) <= eps * max(1.0, np.abs(np.diag(D)).sum())
+    assert abs(tr[1] - tr_ref[1]) <= max(eps, 1e-5 if prec == SINGLE else 0.0) * max(Sd, 1e-300)
+
+
+# N at the ends of tiles (8), groups (32) and words of the bitmaps (256 rows);
+# bands inside one tile, across groups, and the whole matrix
+CASES = [(1, 0, 1.0, ()), (7, 3, 0.6, ()), (8, 8, 0.9, ()), (9, 2, 1.0, ()), (31, 5, 0.7, (3, 4)),
+         (32, 31, 0.5, ()), (33, 33, 0.4, (0, 32)), (65, 9, 0.5, tuple(range(24, 64))), (256, 40, 0.8, ()),
+         (257, 40, 0.5, (256,)), (300, 299, 0.3, ()), (513, 300, 0.9, ()), (1000, 20, 1.0, ())]
+
+
+@pytest.mark.parametrize("prec", [DOUBLE, SINGLE], ids=["fp64", "fp32"])
+@pytest.mark.parametrize("shuffle", [False, True], ids=["ascending", "any_order"])
+@pytest.mark.parametrize("N,band,density,empty", CASES)
+def test_tiles_against_restatement(N, band, density, empty, shuffle, prec):
+    from oracle import oracle as O
+    D = _banded(N, band, density, N + band, empty, np.float64 if prec == DOUBLE else np.float32)
+    for thr in (0.0, 1e-2):
+        _check(O, D, shuffle, thr, prec)
+    assert B.lib.bml_b200_last_x2_symmetric() == 1
+
+
+def test_tiles_long_lists():
+    """More common tile columns than a warp lists at a time (1024: 8192 columns)."""
+    N, M = 8400, 8400
+    rng = np.random.default_rng(0)
+    D = np.zeros((N, N))
+    D[:8, :] = rng.standard_normal((8, N))
+    D = D + D.T
+    D[np.arange(N), np.arange(N)] = 1.0
+    arrs = _rows(D, M, False, 0)
+    st, tr, got = _x2(arrs, N, M, N, 1e-9, DOUBLE)
+    assert st == B.OK
+    Dt = torch.from_numpy(D).cuda()  # the FP64 dense product as the oracle
+    want, S = Dt @ Dt, Dt.abs() @ Dt.abs()
+    G = torch.from_numpy(_dense(got, N, N)).cuda()
+    tol = 1e-12 * S + torch.where(G == 0, 1e-9, 0.0)  # an entry at the threshold may be dropped
+    assert bool(((G - want).abs() <= tol).all())
+    assert abs(tr[1] - float(want.trace())) <= 1e-12 * float(S.trace())
+
+
+def test_matrices_the_tile_form_leaves_to_the_sparse_one():
+    """Infinite entries, a stored row of zeros and an asymmetric entry give
+    the full form's result."""
+    N = 200
+    D = _banded(N, 20, 0.8, 1)
+    M = int((D != 0).sum(1).max())
+    base = _rows(D, M, False, 0)
+    v, ix, nz = base
+    inf = v.copy()
+    inf[5 * M + int(np.flatnonzero(ix[5 * M:5 * M + nz[5]] == 5)[0])] = np.inf
+    zero = v.copy()
+    row = np.repeat(np.arange(N), M)
+    zero[(row == 7) | (ix == 7)] = 0.0
+    asym = v.copy()
+    asym[9 * M] += 1.0
+    for vals in (inf, zero, asym):
+        st, tr, got = _x2((vals, ix, nz), N, M, N, 1e-5, DOUBLE)
+        old = B.lib.bml_b200_set_x2_symmetric(0)
+        st0, tr0, want = _x2((vals, ix, nz), N, M, N, 1e-5, DOUBLE)
+        B.lib.bml_b200_set_x2_symmetric(old)
+        assert st == st0 == B.OK
+        assert np.array_equal(got[2], want[2])
+        assert np.array_equal(got[1], want[1])
+        np.testing.assert_allclose(got[0], want[0], rtol=1e-9, atol=1e-12)
+
+
+@pytest.mark.parametrize("M2", [40, 76], ids=["pool_runs_out", "rows_too_wide"])
+def test_tiles_row_overflow(M2):
+    """A result row wider than M (81 here) is reported, rows hold at most M
+    entries of the product and the traces are whole.  With M2 = 40 the pool of
+    packed blocks runs out and the sparse form completes the call."""
+    N = 300
+    D = _banded(N, 20, 1.0, 2)
+    M = int((D != 0).sum(1).max())
+    arrs = _rows(D, M, False, 0)
+    B.lib.bml_b200_set_verbose(0)
+    try:
+        st, tr, got = _x2(arrs, N, M, M2, 0.0, DOUBLE)
+    finally:
+        B.lib.bml_b200_set_verbose(1)
+        B.clear_error()
+    assert st == B.ERR_ROW_OVERFLOW
+    X2 = D @ D
+    assert tr[1] == pytest.approx(np.trace(X2), rel=1e-12)
+    for i in range(N):
+        n = int(got[2][i])
+        assert 0 < n <= M2
+        k = got[1][i * M2:i * M2 + n]
+        np.testing.assert_allclose(got[0][i * M2:i * M2 + n], X2[i, k], rtol=0, atol=1e-11)
+    if M2 == 76:
+        assert B.lib.bml_b200_last_required_M() == 81
+
+
+@pytest.mark.parametrize("L,radius", [(6, 2), (7, 3)])
+def test_masked_tiles_unsymmetric_weights(L, radius):
+    """The adjoint's masked products on tiles (the second operand through its
+    transpose): weights that are not symmetric, so neither are the gradients
+    that the products take; against the ordered form's gradient (whole
+    products, restricted), as test_adjoint_gpu.py does, to 1e-10."""
+    import ctypes as C
+    N, MH = L ** 3, 128
+    v, ix, nz = B.gen_lattice(L, radius, N, MH, 4)
+    M = N
+    pad = lambda a: np.pad(a.reshape(N, MH), ((0, 0), (0, M - MH)))[:, :M].reshape(-1)  # noqa: E731
+    v, ix = pad(v), pad(ix)
+    vv = np.random.default_rng(1).uniform(-0.01, 0.01, N * M)
+    grads = []
+    for exact in (0, 1):
+        old = B.lib.bml_b200_set_x2_exact(exact)
+        H = B.Ellpack.from_arrays(v, ix, nz, N, M)
+        V = B.Ellpack.from_arrays(vv, ix, nz, N, M)
+        dH = B.Ellpack(N, M)
+        loss = C.c_double()
+        B.check(B.lib.bml_b200_sp2_adjoint(H.h, V.h, 1e-5, N / 2.0, 6, 2, M, dH.h, C.byref(loss)))
+        grads.append((loss.value, dH.download()))
+        B.lib.bml_b200_set_x2_exact(old)
+    (l0, (g0, i0, n0)), (l1, (g1, i1, n1)) = grads
+    assert l0 == pytest.approx(l1, rel=1e-10)
+    mask = (np.arange(M)[None, :] < nz[:, None]).reshape(-1)
+    assert np.array_equal(n0, n1) and np.array_equal(i0[mask], i1[mask])
+    assert np.abs(g0[mask] - g1[mask]).max() <= 1e-10 * np.abs(g1[mask]).max()
