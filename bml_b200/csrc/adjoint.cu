@@ -202,64 +202,6 @@ Mat step_back(bml_matrix_t *Xn, const Mat &G, int branch, double threshold, bml_
     return Gn;
 }
 
-// Rows of H whose Gershgorin discs reach emax (h + r) and emin (h - r),
-// computed on the host mirror with the device kernel's arithmetic.
-template <typename T>
-void gershgorin_rows(bml_matrix_ellpack_t *H, int *kmax, int *kmin)
-{
-    const T *v = static_cast<const T *>(H->value);
-    double best_hi = -HUGE_VAL, best_lo = HUGE_VAL;
-    *kmax = *kmin = 0;
-    for (int i = 0; i < H->N; ++i)
-    {
-        T radius = T(0), d = T(0);
-        for (int p = 0; p < H->nnz[i]; ++p)
-        {
-            const int k = H->index[(size_t) i * H->M + p];
-            const T x = v[(size_t) i * H->M + p];
-            if (k == i)
-                d = x;
-            else
-                radius = (T) ((double) radius + (double) fabs(x));
-        }
-        const double hi = (double) (T) (d + radius), lo = (double) (T) (d - radius);
-        if (hi > best_hi)
-        {
-            best_hi = hi;
-            *kmax = i;
-        }
-        if (lo < best_lo)
-        {
-            best_lo = lo;
-            *kmin = i;
-        }
-    }
-}
-
-// dH row `row` += c * (1 on the diagonal, sgn * sign(H_rj) elsewhere).
-template <typename T>
-void add_disc_gradient(bml_matrix_ellpack_t *H, bml_matrix_ellpack_t *dH, int row, double c, double sgn)
-{
-    const T *hv = static_cast<const T *>(H->value);
-    T *gv = static_cast<T *>(dH->value);
-    for (int p = 0; p < dH->nnz[row]; ++p)
-    {
-        const int k = dH->index[(size_t) row * dH->M + p];
-        double s = 0.0;
-        if (k == row)
-            s = 1.0;
-        else
-            for (int q = 0; q < H->nnz[row]; ++q)
-                if (H->index[(size_t) row * H->M + q] == k)
-                {
-                    const T x = hv[(size_t) row * H->M + q];
-                    s = sgn * (x > T(0) ? 1.0 : (x < T(0) ? -1.0 : 0.0));
-                    break;
-                }
-        gv[(size_t) row * dH->M + p] = (T) ((double) gv[(size_t) row * dH->M + p] + c * s);
-    }
-}
-
 } // namespace
 
 extern "C" int bml_b200_sp2_adjoint(bml_matrix_t *H, bml_matrix_t *V, double threshold, double occupation,
@@ -365,23 +307,9 @@ extern "C" int bml_b200_sp2_adjoint(bml_matrix_t *H, bml_matrix_t *V, double thr
     double sc = -1.0 / d;
     float scf = (float) sc;
     bml_scale_inplace(prec == double_real ? (void *) &sc : (void *) &scf, dH);
-    if (err() || !ell_to_host(He) || !ell_to_host(De))
+    // the bounds' own dependence on H, on the device: neither matrix goes to the host
+    if (err() || !ell_disc_gradient(He, De, (trG - gx) / d, gx / d))
         return err();
-    int kmax = 0, kmin = 0;
-    const double a = (trG - gx) / d, b = gx / d;
-    if (prec == double_real)
-    {
-        gershgorin_rows<double>(He, &kmax, &kmin);
-        add_disc_gradient<double>(He, De, kmax, a, 1.0);
-        add_disc_gradient<double>(He, De, kmin, b, -1.0);
-    }
-    else
-    {
-        gershgorin_rows<float>(He, &kmax, &kmin);
-        add_disc_gradient<float>(He, De, kmax, a, 1.0);
-        add_disc_gradient<float>(He, De, kmin, b, -1.0);
-    }
-    ell_mark_host(De);
     if (loss)
         *loss = L;
     return BML_B200_OK;

@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <climits>
+#include <cmath>
 #include <cstring>
 
 using namespace b200;
@@ -1362,6 +1363,126 @@ bool ell_transpose_new(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B)
                        B->M);
         return false;
     }
+    return true;
+}
+
+namespace {
+
+// The first rows with the largest hi and the smallest lo (row 0 when none
+// compares, as with NaN).  Launch <<<1, 1024>>>.
+__global__ void __launch_bounds__(1024) disc_rows_kernel(const double *hi, const double *lo, int n, int *rows)
+{
+    __shared__ double bv[32];
+    __shared__ int bi[32];
+    for (int side = 0; side < 2; ++side)
+    {
+        const double *x = side ? lo : hi;
+        const double sg = side ? -1.0 : 1.0;
+        double best = -HUGE_VAL;
+        int at = INT_MAX;
+        for (int i = threadIdx.x; i < n; i += 1024)
+            if (sg * x[i] > best)
+            {
+                best = sg * x[i];
+                at = i;
+            }
+        auto join = [&](double v, int k) {
+            if (v > best || (v == best && k < at))
+            {
+                best = v;
+                at = k;
+            }
+        };
+        for (int o = 16; o; o >>= 1)
+        {
+            const double v = __shfl_xor_sync(FULL, best, o);
+            join(v, __shfl_xor_sync(FULL, at, o));
+        }
+        if ((threadIdx.x & 31) == 0)
+        {
+            bv[threadIdx.x >> 5] = best;
+            bi[threadIdx.x >> 5] = at;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0)
+        {
+            for (int w = 1; w < 32; ++w)
+                join(bv[w], bi[w]);
+            rows[side] = at == INT_MAX ? 0 : at;
+        }
+        __syncthreads();
+    }
+}
+
+// dH's rows rows[0] and rows[1] += c (1 on the diagonal, sgn sign(H_rj)
+// elsewhere), with (c, sgn) = (a, 1) and (b, -1).  One CTA.
+template <typename T>
+__global__ void __launch_bounds__(256) disc_gradient_kernel(const T *Hv, const int *Hi, const int *Hn, int ldh, T *Gv,
+                                                            const int *Gi, const int *Gn, int ldg, const int *rows,
+                                                            double a, double b)
+{
+    for (int side = 0; side < 2; ++side)
+    {
+        const int r = rows[side];
+        const double c = side ? b : a, sgn = side ? -1.0 : 1.0;
+        const size_t rg = (size_t) r * ldg, rh = (size_t) r * ldh;
+        const int ng = Gn[r], nh = Hn[r];
+        for (int p = threadIdx.x; p < ng; p += 256)
+        {
+            const int k = Gi[rg + p];
+            double s = 0.0;
+            if (k == r)
+                s = 1.0;
+            else
+                for (int q = 0; q < nh; ++q)
+                    if (Hi[rh + q] == k)
+                    {
+                        const T x = Hv[rh + q];
+                        s = sgn * (x > T(0) ? 1.0 : (x < T(0) ? -1.0 : 0.0));
+                        break;
+                    }
+            Gv[rg + p] = (T) ((double) Gv[rg + p] + c * s);
+        }
+        __syncthreads(); // the two rows may be one
+    }
+}
+
+} // namespace
+
+bool ell_disc_gradient(bml_matrix_ellpack_t *H, bml_matrix_ellpack_t *dH, double a, double b)
+{
+    B200Context *c = b200_ctx();
+    if (!c || !ell_to_device(H) || !ell_to_device(dH))
+        return false;
+    double *hi = static_cast<double *>(b200_scratch((size_t) 2 * H->N * sizeof(double) + 2 * sizeof(int)));
+    if (!hi)
+        return false;
+    double *lo = hi + H->N;
+    int *rows = reinterpret_cast<int *>(lo + H->N);
+    const int grid = max(1, min(b200_ceil_div(H->N, 32 * GER_WARPS), c->sm_count * 8));
+    const bool dbl = H->matrix_precision == double_real;
+    if (dbl)
+        gershgorin_kernel<double><<<grid, GER_WARPS * 32, 0, c->stream>>>(static_cast<const double *>(H->d_value),
+                                                                          H->d_index, H->d_nnz, H->ld, H->N, hi, lo);
+    else
+        gershgorin_kernel<float><<<grid, GER_WARPS * 32, 0, c->stream>>>(static_cast<const float *>(H->d_value),
+                                                                         H->d_index, H->d_nnz, H->ld, H->N, hi, lo);
+    if (!LAUNCH_OK("gershgorin_kernel"))
+        return false;
+    disc_rows_kernel<<<1, 1024, 0, c->stream>>>(hi, lo, H->N, rows);
+    if (!LAUNCH_OK("disc_rows_kernel"))
+        return false;
+    if (dbl)
+        disc_gradient_kernel<double><<<1, 256, 0, c->stream>>>(
+            static_cast<const double *>(H->d_value), H->d_index, H->d_nnz, H->ld, static_cast<double *>(dH->d_value),
+            dH->d_index, dH->d_nnz, dH->ld, rows, a, b);
+    else
+        disc_gradient_kernel<float><<<1, 256, 0, c->stream>>>(
+            static_cast<const float *>(H->d_value), H->d_index, H->d_nnz, H->ld, static_cast<float *>(dH->d_value),
+            dH->d_index, dH->d_nnz, dH->ld, rows, a, b);
+    if (!LAUNCH_OK("disc_gradient_kernel"))
+        return false;
+    ell_mark_device(dH);
     return true;
 }
 

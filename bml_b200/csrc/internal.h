@@ -200,6 +200,9 @@ bool ell_trace_mult(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, double *tr
 bool ell_transpose_new(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B);
 bool ell_copy(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B);
 bool ell_gershgorin(bml_matrix_ellpack_t *A, double *bounds);
+// dH += a d(emax)/dH + b d(emin)/dH, emax and emin H's Gershgorin bounds (the
+// discs of the first rows that reach them; |x| at 0 has derivative 0).
+bool ell_disc_gradient(bml_matrix_ellpack_t *H, bml_matrix_ellpack_t *dH, double a, double b);
 bool ell_sum_squares(bml_matrix_ellpack_t *A, double *result);
 bool ell_fnorm2(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, double *result);
 bool ell_convert(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B); // any precisions, same entries
