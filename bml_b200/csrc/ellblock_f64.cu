@@ -511,9 +511,9 @@ bool eb_multiply_f64(bml_matrix_ellblock_t *A, bml_matrix_ellblock_t *B, bml_mat
     size_t spill = 0;
     for (int attempt = 0; attempt < 2; ++attempt)
     {
-        unsigned char *scr = static_cast<unsigned char *>(b200_scratch(fixed + spill * 8192));
+        unsigned char *scr = static_cast<unsigned char *>(b200_scratch_try(fixed + spill * 8192));
         if (!scr)
-            return false;
+            return true; // the accumulating form asks for what it needs
         g.rowT = reinterpret_cast<unsigned short *>(scr + o_row);
         g.colT = reinterpret_cast<unsigned short *>(scr + o_col);
         g.list = reinterpret_cast<unsigned short *>(scr + o_list);
