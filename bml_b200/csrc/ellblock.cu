@@ -714,7 +714,7 @@ template <typename T> __device__ double block_norm_inf(const T *x, int ne, doubl
 
 // copy B <- A (same partition).  The CTAs of a grid column share a block row's
 // blocks: with a row per CTA, the 343 rows of a 7^3 block lattice left most of
-// an SM's threads idle (226 us for 250 MB, 85 us with the rows shared).
+// an SM's threads idle (226 us for 250 MB, 94 us with the rows shared).
 template <typename T> __global__ void eb_copy_kernel(EbView<T> A, EbView<T> B, int *overflow)
 {
     for (int ib = blockIdx.x; ib < A.NB; ib += gridDim.x)
@@ -872,7 +872,8 @@ __global__ void eb_add_kernel(EbView<T> A, EbView<T> B, double alpha, double bet
 // until the CTA knows which of its eight are kept.  The eight go to positions
 // at or below their own in the list, and A's blocks still to be read lie
 // above, so the sum is again written in place.  (One block at a time with the
-// merge in one thread: 294 us for 7^3 block rows of up to 91 blocks.)
+// merge in one thread: 294 us for 7^3 block rows of up to 91 blocks, 158 us
+// so.)
 template <typename T>
 __global__ void __launch_bounds__(256) eb_add_warp_kernel(EbView<T> A, EbView<T> B, double alpha, double beta, double thr,
                                                         int *scr, int cap, int *overflow)

@@ -47,7 +47,8 @@ struct DenseFlags
 };
 
 // image[i * ld + col] += value for every stored entry (duplicates add up, as
-// they do in the sparse products); rows padded with zeros.  One warp per row.
+// they do in the sparse products; a strictly ascending row has none and is
+// stored); rows padded with zeros.  One warp per row.
 template <typename T>
 __global__ void __launch_bounds__(256) dense_scatter_kernel(const T *v, const int *ix, const int *nz, int ldE, int nrows,
                                                             int ncols, T *img, size_t ld, unsigned char *pat,
@@ -64,6 +65,11 @@ __global__ void __launch_bounds__(256) dense_scatter_kernel(const T *v, const in
                 atomicExch(&flags->bad_input, 1);
             continue;
         }
+        bool desc = false;
+#pragma unroll 4
+        for (int p = lane; p + 1 < n; p += 32)
+            desc |= ix[(size_t) i * ldE + p + 1] <= ix[(size_t) i * ldE + p];
+        const bool sorted = !__any_sync(FULL, desc);
         for (int p = lane; p < n; p += 32)
         {
             const int c = ix[(size_t) i * ldE + p];
@@ -72,7 +78,10 @@ __global__ void __launch_bounds__(256) dense_scatter_kernel(const T *v, const in
                 atomicExch(&flags->bad_input, 1);
                 continue;
             }
-            atomicAdd(&img[(size_t) i * ld + c], v[(size_t) i * ldE + p]);
+            if (sorted)
+                img[(size_t) i * ld + c] = v[(size_t) i * ldE + p];
+            else
+                atomicAdd(&img[(size_t) i * ld + c], v[(size_t) i * ldE + p]);
             if (pat)
                 pat[(size_t) c * ld + i] = 1; // pattern of B, transposed: pat[col * ld + row]
         }
@@ -266,7 +275,7 @@ __global__ void __launch_bounds__(DTHREADS, 1) dense_gemm_f64_kernel(const doubl
 #pragma unroll
         for (int n = 0; n < 4; ++n)
             acc[m][n][0] = acc[m][n][1] = 0.0;
-    const int steps = Kp / DK; // a multiple of 8
+    const int steps = Kp / DK;
     for (int s = 0; s < GS - 1; ++s)
     {
         fetch(s);
@@ -447,13 +456,14 @@ bool dense_typed(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bml_matrix_el
     }
     const dim3 grid((unsigned) (ld / DT), (unsigned) (ld / DT));
     const int *asym = same ? &flags->asym : nullptr;
+    const int kp = b200_round_up(B->N, DK); // the images are zero from there on (N >= 1024)
     if constexpr (std::is_same<T, double>::value)
     {
         const size_t smemG = GS * GSTAGE * sizeof(double);
         if (!CUDA_OK(cudaFuncSetAttribute(dense_gemm_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int) smemG)))
             return false;
-        dense_gemm_f64_kernel<<<grid, DTHREADS, smemG, c->stream>>>(DA, DB, DC, ld, (int) ld, asym);
+        dense_gemm_f64_kernel<<<grid, DTHREADS, smemG, c->stream>>>(DA, DB, DC, ld, kp, asym);
     }
     else
     {
@@ -461,7 +471,7 @@ bool dense_typed(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bml_matrix_el
         if (!CUDA_OK(cudaFuncSetAttribute(dense_gemm_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int) smemG)))
             return false;
-        dense_gemm_kernel<T><<<grid, DTHREADS, smemG, c->stream>>>(DA, DB, DC, ld, (int) ld, asym);
+        dense_gemm_kernel<T><<<grid, DTHREADS, smemG, c->stream>>>(DA, DB, DC, ld, kp, asym);
     }
     if (!LAUNCH_OK("dense_gemm_kernel"))
         return false;

@@ -40,6 +40,12 @@
 // same kernel, the second operand packed as rows of its transpose, the blocks
 // those that hold an entry of the pattern.
 //
+// The general product (A B, and X^2 of an X that is not symmetric) packs the
+// second operand the same way, forms the blocks (G, H) with H on both sides of
+// G, and writes rows from them alone.  The columns that a row touches, which
+// A B's width check and the diagonal's keep rule ask for, come from the OR of
+// the bitmaps of B's rows.
+//
 // Measured against the sparse form on one B200: X^2 of the 40^3 lattice's wide
 // iterate (rows of 825) 65.0 -> 21.3 ms, first X^2 of that lattice (rows of
 // 113) 6.3 -> 2.5 ms, FP32 on 26999 rows 2.08 -> 0.84 ms, a chain of 4096 rows
@@ -87,7 +93,7 @@ struct TileFlags
     unsigned long long tiles2;   // sum over tile rows of tiles^2 (tile products)
     unsigned long long pool;     // words of the packed result taken
     int entries;                 // (group, J) entries of X
-    int reach;                   // largest |column - row|
+    int reach, reachB;           // largest |column - row|; of the second operand
     int bad;                     // a row length or column out of range
     int odd;                     // an entry not finite, or a row of zeros only: not for this form
     int asym;
@@ -117,7 +123,7 @@ struct TileArgs
     void *Cv; int *Ci; int *Cn; int ldc; int Mc;
     double thr;
     double *dA, *dC;             // per-group sums of the diagonals of X and X^2
-    TileFlags *flags;
+    TileFlags *flags, *host;     // host: pinned, written by the row kernel's last CTA
     // second operand, as rows of its transpose (the sparse X^2: the same lists)
     const unsigned *bitsB; const unsigned short *rankB; const int *eoffB; const int2 *rangeB;
     // masked product
@@ -127,7 +133,21 @@ struct TileArgs
     int2 *pblk;                  // blocks (G, H) of the pattern
     double *out;                 // 1024 doubles per block
     int masked, count_only;
+    // general product
+    int general, back;           // blocks (G, G - back + s), s < span
+    unsigned *rowbits; int rw;   // [N][rw] bitmaps of B's rows
+    int *touched;                // rows of C whose diagonal is touched
+    int reach, check_pre;
 };
+
+// The flags as they are in L2, into the host's copy (complete when the kernel
+// is); one warp.
+__device__ __forceinline__ void tell_host(const TileArgs &g, int lane)
+{
+    static_assert(sizeof(TileFlags) <= 32 * sizeof(int), "a word per lane");
+    if (lane < (int) (sizeof(TileFlags) / sizeof(int)))
+        reinterpret_cast<volatile int *>(g.host)[lane] = reinterpret_cast<const volatile int *>(g.flags)[lane];
+}
 
 // The form does not apply: the kernels after the fill do nothing.
 __device__ __forceinline__ bool declined(const TileFlags *f)
@@ -437,7 +457,7 @@ template <typename T> __global__ void __launch_bounds__(FT) tile_fill_kernel(Til
                 }
             }
             // a stored row of zeros touches its diagonal without a sign of it in the tiles
-            odd |= n > 0 && !__any_sync(FULL, some) && !g.masked;
+            odd |= n > 0 && !__any_sync(FULL, some) && !g.masked && !g.general;
             for (int o = 16; o; o >>= 1)
                 d += __shfl_xor_sync(FULL, d, o);
             if (lane == 0)
@@ -602,10 +622,13 @@ __device__ __forceinline__ void mul_tiles(unsigned ea, unsigned eb, const double
         }
 }
 
-// Blocks C(G, H): one warp each, TW consecutive H per CTA (they share G's
-// tiles in L1).
-template <typename T, bool MASKED> __global__ void __launch_bounds__(TW * 32, TMIN) tile_x2_kernel(TileArgs g)
+// Blocks C(G, H), one warp each: H >= G of a symmetric square, those that hold
+// an entry of the pattern, or H on both sides of G.
+constexpr int TILE_SQUARE = 0, TILE_MASKED = 1, TILE_GENERAL = 2;
+
+template <typename T, int MODE> __global__ void __launch_bounds__(TW * 32, TMIN) tile_x2_kernel(TileArgs g)
 {
+    constexpr bool MASKED = MODE == TILE_MASKED, GENERAL = MODE == TILE_GENERAL;
     extern __shared__ __align__(16) unsigned char tsm[]; // per warp: stages[TS][8 tiles] | queue[QCAP]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (MASKED ? g.flags->odd : declined(g.flags))
@@ -637,8 +660,8 @@ template <typename T, bool MASKED> __global__ void __launch_bounds__(TW * 32, TM
             const int patch = it / (SG * SC), in = it % (SG * SC);
             G = patch / pc * SG + in % SG;
             s = patch % pc * SC + in / SG;
-            H = G + s;
-            if (G >= g.NG || s >= g.span || H > g.last[G])
+            H = GENERAL ? G - g.back + s : G + s;
+            if (G >= g.NG || s >= g.span || (GENERAL ? H < 0 || H >= g.NG : H > g.last[G]))
                 continue;
         }
         const int2 ra = g.range[G], rb = g.rangeB[H];
@@ -763,7 +786,7 @@ template <typename T, bool MASKED> __global__ void __launch_bounds__(TW * 32, TM
         for (int a = 0; a < 4; ++a)
         {
             const int r = 8 * a + q4, i = G * GR + r;
-            const bool live = dg && i < g.N && g.Xn[i] > 0; // the diagonal is touched
+            const bool live = dg && i < g.N && (GENERAL ? g.touched[i] : g.Xn[i]) > 0; // the diagonal is touched
             unsigned m = 0u;
 #pragma unroll
             for (int b = 0; b < 4; ++b)
@@ -775,7 +798,7 @@ template <typename T, bool MASKED> __global__ void __launch_bounds__(TW * 32, TM
                     bool keep = over<T>(x, g.thr);
                     if (dg)
                     {
-                        keep = c == r ? live : keep && c > r;
+                        keep = c == r ? live : keep && (GENERAL || c > r);
                         if (c == r && live)
                             dsum += (double) x;
                     }
@@ -863,18 +886,29 @@ template <typename T> __global__ void __launch_bounds__(RT) tile_rows_kernel(Til
     __shared__ int nblk;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (declined(g.flags) || g.flags->full)
+    {
+        if (blockIdx.x == 0 && warp == 0)
+            tell_host(g, lane);
         return;
+    }
     for (int G = blockIdx.x; G < g.NG; G += gridDim.x)
     {
         // candidates in column order: (G - span + 1 + c, G) transposed for c < span, then (G, G + c - span)
         if (tid == 0)
             nblk = 0;
         __syncthreads();
-        for (int c0 = 0; c0 < 2 * g.span; c0 += RT)
+        for (int c0 = 0; c0 < (g.general ? g.span : 2 * g.span); c0 += RT)
         {
             const int c = c0 + tid;
             int at = -1, key = 0;
-            if (c < g.span)
+            if (g.general)
+            {
+                const int H = G - g.back + c;
+                if (c < g.span && H >= 0 && H < g.NG)
+                    at = g.tab[(size_t) G * g.span + c];
+                key = H * 2;
+            }
+            else if (c < g.span)
             {
                 const int H = G - g.span + 1 + c;
                 if (H >= 0)
@@ -988,7 +1022,11 @@ template <typename T> __global__ void __launch_bounds__(RT) tile_rows_kernel(Til
     __shared__ double part[2][W];
     __shared__ int fin;
     if (tid == 0)
+    {
+        __threadfence(); // this CTA's width and overflow come before its count
         fin = atomicAdd(&g.flags->done, 1) == (int) gridDim.x - 1;
+        __threadfence();
+    }
     __syncthreads();
     if (!fin)
         return;
@@ -1018,6 +1056,12 @@ template <typename T> __global__ void __launch_bounds__(RT) tile_rows_kernel(Til
         }
         g.flags->trA = a;
         g.flags->trC = d;
+        __threadfence();
+    }
+    if (warp == 0)
+    {
+        __syncwarp();
+        tell_host(g, lane);
     }
 }
 
@@ -1043,6 +1087,7 @@ __global__ void __launch_bounds__(PT) tile_tbits_kernel(TileArgs g)
         if (lane == 0 && n)
             atomicAdd(&g.flags->products, (unsigned long long) n * n);
         const unsigned bit = 1u << ((j >> 3) & 31);
+        int far = 0;
         for (int p = lane; p < n; p += 32)
         {
             const int k = g.Xi[(size_t) j * g.ld + p];
@@ -1051,10 +1096,15 @@ __global__ void __launch_bounds__(PT) tile_tbits_kernel(TileArgs g)
                 atomicExch(&g.flags->bad, 1);
                 continue;
             }
+            far = max(far, abs(k - j));
             unsigned *w = g.gb + (size_t) (k >> 3) * g.nw + (j >> 8);
             if (!(*(volatile unsigned *) w & bit))
                 atomicOr(w, bit);
         }
+        for (int o = 16; o; o >>= 1)
+            far = max(far, __shfl_xor_sync(FULL, far, o));
+        if (lane == 0 && far > *(volatile int *) &g.flags->reachB)
+            atomicMax(&g.flags->reachB, far);
     }
 }
 
@@ -1133,19 +1183,19 @@ template <typename T> __global__ void __launch_bounds__(PT) tile_scatter_kernel(
 
 // Groups H with an entry of P in the rows of G: counted (count_only), or
 // listed with their ranks.  Shared memory: bitmap[hw].
-__global__ void __launch_bounds__(PT) tile_pattern_kernel(TileArgs g)
+__global__ void __launch_bounds__(FT) tile_pattern_kernel(TileArgs g)
 {
     extern __shared__ unsigned pb[];
     __shared__ int sum, base;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     for (int G = blockIdx.x; G < g.NG; G += gridDim.x)
     {
-        for (int w = tid; w < g.hw; w += PT)
+        for (int w = tid; w < g.hw; w += FT)
             pb[w] = 0u;
         if (tid == 0)
             sum = 0;
         __syncthreads();
-        for (int r = warp; r < GR; r += PT / 32)
+        for (int r = warp; r < GR; r += FT / 32)
         {
             const int i = G * GR + r;
             const int n = i < g.N ? g.Pn[i] : 0;
@@ -1166,7 +1216,7 @@ __global__ void __launch_bounds__(PT) tile_pattern_kernel(TileArgs g)
         }
         __syncthreads();
         int c = 0;
-        for (int w = tid; w < g.hw; w += PT)
+        for (int w = tid; w < g.hw; w += FT)
             c += __popc(pb[w]);
         if (c)
             atomicAdd(&sum, c);
@@ -1276,7 +1326,7 @@ template <typename T> bool tile_masked_typed(TileArgs a, TileArgs b, bool *taken
         if (!LAUNCH_OK("tile_count_kernel"))
             return false;
         a.count_only = 1;
-        tile_pattern_kernel<<<per, PT, smemP, c->stream>>>(a);
+        tile_pattern_kernel<<<per, FT, smemP, c->stream>>>(a);
         if (!LAUNCH_OK("tile_pattern_kernel") ||
             !CUDA_OK(cudaMemcpyAsync(hf, small, sizeof(TileFlags), cudaMemcpyDeviceToHost, c->stream)) || !b200_sync())
             return false;
@@ -1327,14 +1377,14 @@ template <typename T> bool tile_masked_typed(TileArgs a, TileArgs b, bool *taken
     tile_scatter_kernel<T><<<std::min(b200_ceil_div(b.N, PT / 32), c->sm_count * 8), PT, 0, c->stream>>>(b);
     if (!LAUNCH_OK("tile_scatter_kernel"))
         return false;
-    tile_pattern_kernel<<<per, PT, smemP, c->stream>>>(a);
+    tile_pattern_kernel<<<per, FT, smemP, c->stream>>>(a);
     if (!LAUNCH_OK("tile_pattern_kernel"))
         return false;
     const size_t smemQ = (size_t) TW * WARP_SMEM;
-    if (!CUDA_OK(cudaFuncSetAttribute(tile_x2_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (!CUDA_OK(cudaFuncSetAttribute(tile_x2_kernel<T, TILE_MASKED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int) smemQ)))
         return false;
-    tile_x2_kernel<T, true><<<c->sm_count * TMIN, TW * 32, smemQ, c->stream>>>(a);
+    tile_x2_kernel<T, TILE_MASKED><<<c->sm_count * TMIN, TW * 32, smemQ, c->stream>>>(a);
     if (!LAUNCH_OK("tile_x2_kernel"))
         return false;
     tile_gather_kernel<T><<<std::min(b200_ceil_div(a.N, PT / 32), c->sm_count * 8), PT, 0, c->stream>>>(a);
@@ -1342,6 +1392,223 @@ template <typename T> bool tile_masked_typed(TileArgs a, TileArgs b, bool *taken
         !CUDA_OK(cudaMemcpyAsync(hf, small, sizeof(TileFlags), cudaMemcpyDeviceToHost, c->stream)) || !b200_sync())
         return false;
     *taken = !hf->odd && !hf->bad;
+    return true;
+}
+
+// -------------------------------------------------------------------------
+// General product: which columns a row touches.
+// -------------------------------------------------------------------------
+
+// Bitmaps over columns of B's rows (zero before); one warp per row.
+__global__ void __launch_bounds__(PT) tile_rowbits_kernel(TileArgs g)
+{
+    const int lane = threadIdx.x & 31, warps = (gridDim.x * PT) >> 5;
+    for (int j = (blockIdx.x * PT + threadIdx.x) >> 5; j < g.N; j += warps)
+    {
+        const int n = g.Xn[j];
+        for (int p = lane; p < n; p += 32)
+        {
+            const int k = g.Xi[(size_t) j * g.ld + p];
+            atomicOr(&g.rowbits[(size_t) j * g.rw + (k >> 5)], 1u << (k & 31));
+        }
+    }
+}
+
+// Row i of C touches the OR of the bitmaps of the rows of B that A's row i
+// names: its width against M (check_pre), and whether it holds the diagonal.
+// One warp per row, 128 words (16 bytes a lane) of the row's window (g.reach
+// columns on each side) at a time.
+__global__ void __launch_bounds__(PT) tile_touch_kernel(TileArgs g)
+{
+    const int lane = threadIdx.x & 31, warps = (gridDim.x * PT) >> 5;
+    for (int i = (blockIdx.x * PT + threadIdx.x) >> 5; i < g.N; i += warps)
+    {
+        const int n = g.Xn[i];
+        const int lo = max(0, i - g.reach) >> 7, hi = min(g.N - 1, i + g.reach) >> 7; // in words of 128 columns
+        int width = 0;
+        bool diag = false;
+        for (int w0 = lo; w0 <= hi; w0 += 32)
+        {
+            const int w = w0 + lane;
+            uint4 any = make_uint4(0u, 0u, 0u, 0u);
+            for (int p0 = 0; p0 < n; p0 += 32)
+            {
+                const int mine = p0 + lane < n ? g.Xi[(size_t) i * g.ld + p0 + lane] : 0;
+                const int m = min(32, n - p0);
+#pragma unroll 8
+                for (int t = 0; t < m; ++t)
+                {
+                    const int j = __shfl_sync(FULL, mine, t);
+                    if (w <= hi)
+                    {
+                        const uint4 b = __ldg(reinterpret_cast<const uint4 *>(g.rowbits + (size_t) j * g.rw) + w);
+                        any.x |= b.x;
+                        any.y |= b.y;
+                        any.z |= b.z;
+                        any.w |= b.w;
+                    }
+                }
+            }
+            width += __popc(any.x) + __popc(any.y) + __popc(any.z) + __popc(any.w);
+            const int q = (i >> 5) & 3;
+            diag |= w == i >> 7 && ((q == 0 ? any.x : q == 1 ? any.y : q == 2 ? any.z : any.w) >> (i & 31) & 1u);
+        }
+        for (int o = 16; o; o >>= 1)
+            width += __shfl_xor_sync(FULL, width, o);
+        diag = __any_sync(FULL, diag);
+        if (lane == 0)
+        {
+            g.touched[i] = diag;
+            if (g.check_pre && width > g.Mc)
+                atomicExch(&g.flags->overflow, 1);
+        }
+    }
+}
+
+template <typename T>
+bool tile_general_typed(TileArgs a, TileArgs b, double *trace, int *required_M, bool *taken, cudaEvent_t *timer)
+{
+    B200Context *c = b200_ctx();
+    if (!c)
+        return false;
+    unsigned char *small = static_cast<unsigned char *>(c->d_small) + TL_SMALL;
+    TileFlags *hf = reinterpret_cast<TileFlags *>(static_cast<unsigned char *>(c->pinned) + TL_SMALL);
+    a.flags = b.flags = reinterpret_cast<TileFlags *>(small);
+    a.host = hf;
+    const int NG = a.NG, nw = a.nw;
+    const int per = std::min(NG, c->sm_count * 8);
+    const int rows = std::min(b200_ceil_div(a.N, PT / 32), c->sm_count * 8);
+    const size_t smemC = (size_t) 4 * nw * sizeof(unsigned), smemF = (size_t) 5 * nw * sizeof(unsigned);
+    auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        const size_t o = at;
+        at = al(at + bytes);
+        return o;
+    };
+    const size_t n_gb = (size_t) NG * 4 * nw * sizeof(unsigned), n_rb = (size_t) b.N * b.rw * sizeof(unsigned);
+    const size_t o_gb = take(n_gb), o_rb = take(n_rb);
+    const size_t o_bits = take((size_t) 2 * NG * nw * sizeof(unsigned));
+    const size_t o_rank = take((size_t) 2 * NG * nw * sizeof(unsigned short));
+    const size_t o_eoff = take((size_t) 2 * NG * sizeof(int)), o_range = take((size_t) 2 * NG * sizeof(int2));
+    const size_t o_touched = take((size_t) a.N * sizeof(int)), o_diag = take((size_t) 2 * NG * sizeof(double));
+    const size_t fixed = at;
+    size_t o_ent = 0, o_entJ = 0, o_tiles = 0, o_tab = 0, o_pool = 0;
+    unsigned char *scr = nullptr;
+    int reach = 0;
+    // the counts, then the layout; a larger arena loses B's bitmaps, which are then made again
+    for (int attempt = 0; attempt < 2; ++attempt)
+    {
+        if (attempt && at <= c->scratch_bytes)
+            break;
+        scr = static_cast<unsigned char *>(b200_scratch_try(attempt ? at : fixed));
+        if (!scr)
+            return true; // the sparse form takes less
+        b.gb = reinterpret_cast<unsigned *>(scr + o_gb);
+        b.rowbits = reinterpret_cast<unsigned *>(scr + o_rb);
+        if (!CUDA_OK(cudaMemsetAsync(b.gb, 0, n_gb, c->stream)) ||
+            !CUDA_OK(cudaMemsetAsync(b.rowbits, 0, n_rb, c->stream)) ||
+            !CUDA_OK(cudaMemsetAsync(small, 0, sizeof(TileFlags), c->stream)))
+            return false;
+        tile_tbits_kernel<<<rows, PT, 0, c->stream>>>(b);
+        if (!LAUNCH_OK("tile_tbits_kernel"))
+            return false;
+        if (attempt)
+            break;
+        tile_tcount_kernel<<<per, PT, 0, c->stream>>>(b);
+        if (!LAUNCH_OK("tile_tcount_kernel"))
+            return false;
+        tile_count_kernel<<<per, FT, smemC, c->stream>>>(a);
+        if (!LAUNCH_OK("tile_count_kernel") ||
+            !CUDA_OK(cudaMemcpyAsync(hf, small, sizeof(TileFlags), cudaMemcpyDeviceToHost, c->stream)) || !b200_sync())
+            return false;
+        if (hf->bad || hf->entries <= 0 || hf->entries >= (1 << 28) ||
+            (double) hf->tiles2 * TILE_COST > (double) hf->products)
+            return true;
+        const long long entries = hf->entries;
+        reach = std::min(a.N, hf->reach + hf->reachB);
+        a.back = std::min(NG - 1, reach / GR + 1);
+        a.span = 2 * a.back + 1;
+        const size_t words = (size_t) a.N * a.Mc * sizeof(T) / 8 + 1 + (size_t) 17 * NG * a.span;
+        if ((size_t) a.span * sizeof(int2) > c->smem_optin - 8192 || words >= ((size_t) 1 << 31) ||
+            (long long) ((NG + SG - 1) / SG * SG) * ((a.span + SC - 1) / SC * SC) >= 1 << 30)
+            return true;
+        o_ent = take((size_t) entries * sizeof(unsigned));
+        o_entJ = take((size_t) entries * sizeof(unsigned short));
+        o_tiles = take((size_t) entries * 2048);
+        o_tab = take((size_t) NG * a.span * sizeof(int));
+        o_pool = take(words * 8);
+        a.cap = words;
+        if (at > ((size_t) 64 << 30))
+            return true;
+    }
+    a.ent = b.ent = reinterpret_cast<unsigned *>(scr + o_ent);
+    a.entJ = b.entJ = reinterpret_cast<unsigned short *>(scr + o_entJ);
+    a.tiles = b.tiles = reinterpret_cast<double *>(scr + o_tiles);
+    a.bits = reinterpret_cast<unsigned *>(scr + o_bits);
+    a.rank = reinterpret_cast<unsigned short *>(scr + o_rank);
+    a.eoff = reinterpret_cast<int *>(scr + o_eoff);
+    a.range = reinterpret_cast<int2 *>(scr + o_range);
+    a.bitsB = b.bits = a.bits + (size_t) NG * nw;
+    a.rankB = b.rank = a.rank + (size_t) NG * nw;
+    a.eoffB = b.eoff = a.eoff + NG;
+    a.rangeB = b.range = a.range + NG;
+    a.touched = reinterpret_cast<int *>(scr + o_touched);
+    a.dA = reinterpret_cast<double *>(scr + o_diag);
+    a.dC = a.dA + NG;
+    a.tab = reinterpret_cast<int *>(scr + o_tab);
+    a.pool = reinterpret_cast<unsigned long long *>(scr + o_pool);
+    a.rowbits = b.rowbits;
+    a.reach = reach;
+    if (!CUDA_OK(cudaMemsetAsync(small, 0, sizeof(TileFlags), c->stream)))
+        return false;
+    tile_rowbits_kernel<<<rows, PT, 0, c->stream>>>(b);
+    if (!LAUNCH_OK("tile_rowbits_kernel"))
+        return false;
+    tile_touch_kernel<<<rows, PT, 0, c->stream>>>(a);
+    if (!LAUNCH_OK("tile_touch_kernel"))
+        return false;
+    tile_fill_kernel<T><<<per, FT, smemF, c->stream>>>(a);
+    if (!LAUNCH_OK("tile_fill_kernel"))
+        return false;
+    tile_fill_kernel<T><<<per, FT, smemF, c->stream>>>(b);
+    if (!LAUNCH_OK("tile_fill_kernel"))
+        return false;
+    tile_scatter_kernel<T><<<rows, PT, 0, c->stream>>>(b);
+    if (!LAUNCH_OK("tile_scatter_kernel"))
+        return false;
+    const size_t smemQ = (size_t) TW * WARP_SMEM;
+    const size_t smemR = (size_t) a.span * sizeof(int2);
+    if (!CUDA_OK(cudaFuncSetAttribute(tile_x2_kernel<T, TILE_GENERAL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int) smemQ)) ||
+        (smemR > 32768 && !CUDA_OK(cudaFuncSetAttribute(
+                              tile_rows_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smemR))) ||
+        (timer && !CUDA_OK(cudaEventRecord(timer[0], c->stream))))
+        return false;
+    tile_x2_kernel<T, TILE_GENERAL><<<c->sm_count * TMIN, TW * 32, smemQ, c->stream>>>(a);
+    if (!LAUNCH_OK("tile_x2_kernel"))
+        return false;
+    if (timer && !CUDA_OK(cudaEventRecord(timer[1], c->stream)))
+        return false;
+    tile_rows_kernel<T><<<NG, RT, smemR, c->stream>>>(a);
+    if (!LAUNCH_OK("tile_rows_kernel") || !b200_sync())
+        return false;
+    if (hf->bad || hf->odd || hf->full)
+        return true;
+    *taken = true;
+    if (required_M)
+        *required_M = hf->max_width;
+    if (trace)
+    {
+        trace[0] = hf->trA;
+        trace[1] = hf->trC;
+    }
+    if (hf->overflow)
+    {
+        b200_set_error(BML_B200_ERR_ROW_OVERFLOW, "Number of non-zeroes per row > M, Increase M (need %d, M = %d)",
+                       hf->max_width, a.Mc);
+        return false;
+    }
     return true;
 }
 
@@ -1355,6 +1622,7 @@ bool tile_x2_typed(TileArgs g, double *trace, int *required_M, bool *taken, bool
     unsigned char *pin = static_cast<unsigned char *>(c->pinned) + TL_SMALL;
     TileFlags *hf = reinterpret_cast<TileFlags *>(pin);
     g.flags = reinterpret_cast<TileFlags *>(small);
+    g.host = hf;
     const int per = (int) std::min<long long>(g.NG, (long long) c->sm_count * 8);
     const size_t smemC = (size_t) 4 * g.nw * sizeof(unsigned);
     const size_t smemF = (size_t) 5 * g.nw * sizeof(unsigned); // at most 40 KB
@@ -1444,9 +1712,9 @@ bool tile_x2_typed(TileArgs g, double *trace, int *required_M, bool *taken, bool
     if (items >= 1 << 30)
         return true;
     const size_t smemQ = (size_t) TW * WARP_SMEM;
-    if (!CUDA_OK(cudaFuncSetAttribute(tile_x2_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smemQ)))
+    if (!CUDA_OK(cudaFuncSetAttribute(tile_x2_kernel<T, TILE_SQUARE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smemQ)))
         return false;
-    tile_x2_kernel<T, false><<<(int) std::min<long long>((items + TW - 1) / TW, (long long) c->sm_count * TMIN), TW * 32, smemQ,
+    tile_x2_kernel<T, TILE_SQUARE><<<(int) std::min<long long>((items + TW - 1) / TW, (long long) c->sm_count * TMIN), TW * 32, smemQ,
                         c->stream>>>(g);
     if (!LAUNCH_OK("tile_x2_kernel"))
         return false;
@@ -1456,9 +1724,7 @@ bool tile_x2_typed(TileArgs g, double *trace, int *required_M, bool *taken, bool
                              tile_rows_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smemR)))
         return false;
     tile_rows_kernel<T><<<g.NG, RT, smemR, c->stream>>>(g);
-    if (!LAUNCH_OK("tile_rows_kernel"))
-        return false;
-    if (!CUDA_OK(cudaMemcpyAsync(pin, small, sizeof(TileFlags), cudaMemcpyDeviceToHost, c->stream)) || !b200_sync())
+    if (!LAUNCH_OK("tile_rows_kernel") || !b200_sync())
         return false;
     if (hf->bad || hf->odd || hf->asym || hf->full || (double) hf->tiles2 * TILE_COST > (double) hf->products)
     {
@@ -1543,4 +1809,40 @@ bool ell_masked_tiles(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bml_matr
     a.Mc = C->M;
     return A->matrix_precision == double_real ? tile_masked_typed<double>(a, b, taken)
                                               : tile_masked_typed<float>(a, b, taken);
+}
+
+bool ell_general_tiles(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bml_matrix_ellpack_t *C, double threshold,
+                       double *trace, int *required_M, bool check_pre, bool *taken, cudaEvent_t *timer)
+{
+    *taken = false;
+    const int nbk = b200_ceil_div(A->N, 8);
+    if (!(threshold >= 0.0) || A->N != B->N || A->N != C->N || nbk > 65535)
+        return true;
+    TileArgs a{};
+    a.N = a.ncols = A->N;
+    a.NG = b200_ceil_div(A->N, GR);
+    a.nw = b200_ceil_div(nbk, 32);
+    a.rw = b200_ceil_div(A->N, 128) * 4; // rows of 16-byte words
+    if ((size_t) a.N * a.rw * sizeof(unsigned) > ((size_t) 2 << 30)) // bitmaps of B's rows: N up to 131072
+        return true;
+    a.general = 1;
+    a.thr = threshold;
+    TileArgs b = a;
+    b.masked = 1;
+    a.Xv = A->d_value;
+    a.Xi = A->d_index;
+    a.Xn = A->d_nnz;
+    a.ld = A->ld;
+    b.Xv = B->d_value;
+    b.Xi = B->d_index;
+    b.Xn = B->d_nnz;
+    b.ld = B->ld;
+    a.Cv = C->d_value;
+    a.Ci = C->d_index;
+    a.Cn = C->d_nnz;
+    a.ldc = C->ld;
+    a.Mc = C->M;
+    a.check_pre = check_pre ? 1 : 0;
+    return A->matrix_precision == double_real ? tile_general_typed<double>(a, b, trace, required_M, taken, timer)
+                                              : tile_general_typed<float>(a, b, trace, required_M, taken, timer);
 }

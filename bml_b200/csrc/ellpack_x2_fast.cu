@@ -1039,19 +1039,24 @@ bool ell_multiply_unordered(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bm
     // the touched columns are needed where untouched zeros could pass the
     // keep rule (threshold < 0 or NaN) or the pre-threshold width is checked
     const bool touch = check_pre || !(threshold >= 0.0);
+    // on tiles: the symmetric square, or the general product where there is no symmetry to use
+    const bool timed = kernel_timer();
+    bool taken = false, ok = true;
     if (g.sym_try && !touch)
     {
-        bool taken = false, asym = false;
-        const bool timed = kernel_timer();
-        const bool ok = ell_x2_tiles(A, C, threshold, trace, required_M, &taken, &asym, timed ? g_kev : nullptr);
-        if (taken || !ok)
-        {
-            g_last_symmetric = taken;
-            g_last_kernel_ms = -1.0f;
-            return !(timed && taken && !CUDA_OK(cudaEventElapsedTime(&g_last_kernel_ms, g_kev[0], g_kev[1]))) && ok;
-        }
+        bool asym = false;
+        ok = ell_x2_tiles(A, C, threshold, trace, required_M, &taken, &asym, timed ? g_kev : nullptr);
         if (asym)
             g.sym_try = 0;
+    }
+    const bool square = taken;
+    if (ok && !taken && !g.sym_try)
+        ok = ell_general_tiles(A, B, C, threshold, trace, required_M, check_pre, &taken, timed ? g_kev : nullptr);
+    if (taken || !ok)
+    {
+        g_last_symmetric = square;
+        g_last_kernel_ms = -1.0f;
+        return !(timed && taken && !CUDA_OK(cudaEventElapsedTime(&g_last_kernel_ms, g_kev[0], g_kev[1]))) && ok;
     }
     return A->matrix_precision == double_real ? fast_multiply_typed<double>(g, trace, required_M, touch)
                                               : fast_multiply_typed<float>(g, trace, required_M, touch);

@@ -160,6 +160,10 @@ bool ell_multiply_unordered(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bm
 // symmetric); timer (nullable): events recorded around the product kernel.
 bool ell_x2_tiles(bml_matrix_ellpack_t *X, bml_matrix_ellpack_t *C, double threshold, double *trace, int *required_M,
                   bool *taken, bool *asym, cudaEvent_t *timer);
+// The tile form of the unordered A*B (and X^2 whatever its symmetry) of square
+// matrices of one N, threshold >= 0; check_pre as for ell_multiply_unordered.
+bool ell_general_tiles(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bml_matrix_ellpack_t *C, double threshold,
+                       double *trace, int *required_M, bool check_pre, bool *taken, cudaEvent_t *timer);
 // The tile form of the masked product below; *taken false, with no status
 // set, where it does not apply.
 bool ell_masked_tiles(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bml_matrix_ellpack_t *P,

@@ -195,3 +195,68 @@ def test_masked_tiles_unsymmetric_weights(L, radius):
     mask = (np.arange(M)[None, :] < nz[:, None]).reshape(-1)
     assert np.array_equal(n0, n1) and np.array_equal(i0[mask], i1[mask])
     assert np.abs(g0[mask] - g1[mask]).max() <= 1e-10 * np.abs(g1[mask]).max()
+
+
+def _random_band(N, band, density, seed, empty, dtype):
+    rng = np.random.default_rng(seed)
+    i, j = np.indices((N, N))
+    D = np.where((abs(i - j) <= band) & (rng.random((N, N)) < density), rng.standard_normal((N, N)), 0.0).astype(dtype)
+    D[list(empty), :] = 0
+    return D
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("square", [False, True], ids=["ab", "x2_not_symmetric"])
+@pytest.mark.parametrize("N,ba,bb,density,empty", [
+    (1, 0, 0, 1.0, ()), (9, 2, 8, 0.9, (3,)), (32, 31, 5, 0.8, ()), (33, 4, 33, 0.7, (0, 32)),
+    (257, 30, 60, 0.6, tuple(range(32, 64))), (400, 399, 20, 0.5, ()), (900, 12, 80, 0.9, ())])
+def test_general_tiles(N, ba, bb, density, empty, square, dtype):
+    """A*B and X^2 of matrices that are not symmetric, rows in any order: the
+    kept entries and the diagonal where some product touches it, against the
+    dense FP64 product; and the refusal of a row that touches more than M
+    columns although fewer are kept."""
+    prec = "double_real" if dtype == np.float64 else "single_real"
+    Da = _random_band(N, ba, density, 1, empty, dtype)
+    Db = Da if square else _random_band(N, bb, density, 2, empty, dtype)
+    if N > 8:  # a diagonal that nothing touches
+        Da[5, :] = 0
+        Db = Da if square else Db
+    pa, pb = (Da != 0).astype(float), (Db != 0).astype(float)
+    want, S = Da.astype(float) @ Db.astype(float), abs(Da.astype(float)) @ abs(Db.astype(float))
+    touched = pa @ pb > 0
+    thr = 0.5
+    n = int((Da != 0).sum(1).max()) or 1
+    tol = (1e-12 if dtype == np.float64 else 2.0 * n * 2.0 ** -24) * S
+    keep = abs(want) > thr
+    np.fill_diagonal(keep, touched.diagonal())
+    ma, mb = (max(1, int((d != 0).sum(1).max())) for d in (Da, Db))
+    A = B.Ellpack.from_arrays(*_rows(Da, ma, True, 3), N, ma, prec)
+    Bm = A if square else B.Ellpack.from_arrays(*_rows(Db, mb, False, 4), N, mb, prec)
+    wide = max(1, int(touched.sum(1).max()))
+    for M, status in ((wide, B.OK), (wide - 1, B.ERR_ROW_OVERFLOW)):
+        if M < 1 or (square and status != B.OK):
+            continue
+        Cm = B.Ellpack(N, M, prec)
+        B.lib.bml_b200_set_verbose(0)
+        if square:
+            st, tr = B.multiply_x2(A, Cm, thr)
+            assert abs(tr[0] - np.trace(Da.astype(float))) <= 1e-12 * max(1.0, abs(np.diag(Da)).sum())
+            assert abs(tr[1] - np.trace(want)) <= (1e-12 if dtype == np.float64 else 1e-5) * max(np.trace(S), 1e-300)
+        else:
+            B.lib.bml_multiply_AB(A.h, Bm.h, Cm.h, thr)
+            st = B.last_error()
+        B.clear_error()
+        B.lib.bml_b200_set_verbose(1)
+        assert st == status
+        if status != B.OK:
+            continue
+        got = Cm.download()
+        assert x2check.rows_sorted(got, M)
+        v, ix, nz = got[0].reshape(N, M), got[1].reshape(N, M), got[2]
+        G, K = np.zeros((N, N)), np.zeros((N, N), bool)
+        for i in range(N):
+            G[i, ix[i, :nz[i]]], K[i, ix[i, :nz[i]]] = v[i, :nz[i]], True
+        sure = abs(abs(want) - thr) > tol + 1e-300
+        sure |= np.eye(N, dtype=bool)
+        assert np.array_equal(K[sure], keep[sure])
+        assert (abs(G - want)[K] <= (tol + 1e-300)[K] + (abs(want)[K] * 2.0 ** -24 if dtype == np.float32 else 0)).all()
