@@ -29,7 +29,7 @@
 // the device): only blocks kb >= ib are formed, each stored also at its
 // mirrored place, so C is exactly symmetric.
 //
-// Measured (X^2 of the radius-2 block lattice, FP64): 11^3 blocks 6.2 -> 1.97
+// Measured (X^2 of the radius-2 block lattice, FP64): 11^3 blocks 6.2 -> 1.93
 // ms, 6^3 blocks 1.65 -> 0.37 ms.  At 11^3 the stores of the result alone take
 // 0.35 ms; the products of one triangle 0.93 ms at 37 TFLOP/s, the rest is the
 // latency of the first loads of a block (4.2 pairs on average).
@@ -97,9 +97,12 @@ __global__ void __launch_bounds__(PT) f64_table_kernel(F64Args g)
     }
 }
 
-// X against its transpose: blocks (ib, jb), jb >= ib, one warp each.
-__global__ void __launch_bounds__(PT) f64_sym_kernel(F64Args g)
+// X against its transpose: blocks (ib, jb), jb >= ib, one warp each, the
+// mirrored block through shared memory (its column reads in place: 100 us
+// against 68 at 11^3 blocks).
+__global__ void __launch_bounds__(128) f64_sym_kernel(F64Args g)
 {
+    __shared__ double t[4][32][33];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int ib = blockIdx.x; ib < g.NB; ib += gridDim.x)
     {
@@ -107,7 +110,7 @@ __global__ void __launch_bounds__(PT) f64_sym_kernel(F64Args g)
             return;
         const int n = g.An[ib];
         int bad = 0;
-        for (int p = warp; p < n; p += PT / 32)
+        for (int p = warp; p < n; p += 4)
         {
             const int jb = g.Ai[(size_t) ib * g.MA + p];
             const int s = g.rowT[(size_t) jb * g.NB + ib];
@@ -118,11 +121,16 @@ __global__ void __launch_bounds__(PT) f64_sym_kernel(F64Args g)
             }
             if (jb < ib)
                 continue;
-            const double *x = g.Ap + ((size_t) ib * g.MA + p) * 1024;
-            const double *y = g.Ap + ((size_t) jb * g.MA + s) * 1024;
-#pragma unroll 8
+            const double *x = g.Ap + ((size_t) ib * g.MA + p) * 1024 + lane;
+            const double *y = g.Ap + ((size_t) jb * g.MA + s) * 1024 + lane;
+#pragma unroll 16
             for (int r = 0; r < 32; ++r)
-                bad |= x[r * 32 + lane] != y[lane * 32 + r];
+                t[warp][r][lane] = y[r * 32];
+            __syncwarp();
+#pragma unroll 16
+            for (int r = 0; r < 32; ++r)
+                bad |= x[r * 32] != t[warp][lane][r];
+            __syncwarp();
         }
         if (__any_sync(FULL, bad) && lane == 0)
             atomicExch(&g.flags->asym, 1);
@@ -244,6 +252,7 @@ template <bool SYM> __global__ void __launch_bounds__(FW * 32, FMIN) f64_numeric
             const int qm = SYM && !diag ? g.where[(size_t) kb * g.NB + ib] : 0;
             double *mir = SYM ? (diag ? dst : place_of(g, kb, qm)) : nullptr;
             double mx = 0.0, tr = 0.0;
+            int npairs = 0;
             // two halves of 16 columns: room for the sum and for the product of one pair
             for (int half = 0; half < 2; ++half)
             {
@@ -253,8 +262,10 @@ template <bool SYM> __global__ void __launch_bounds__(FW * 32, FMIN) f64_numeric
 #pragma unroll
                     for (int b = 0; b < 2; ++b)
                         acc[a][b][0] = acc[a][b][1] = part[a][b][0] = part[a][b][1] = 0.0;
-                int n = 0;
-                for (int p0 = 0;; p0 += 32)
+                // the second half finds the list as the first left it, if it held all pairs
+                const bool listed = half && na <= PAIRS;
+                int n = listed ? npairs : 0;
+                for (int p0 = listed ? na : 0;; p0 += 32)
                 {
                     // pairs of the next 32 left blocks: slot in row ib, slot of the right block
                     const int p = p0 + lane;
@@ -271,6 +282,7 @@ template <bool SYM> __global__ void __launch_bounds__(FW * 32, FMIN) f64_numeric
                     {
                         __syncwarp();
                         const int steps = 4 * n;
+                        npairs = n;
                         double2 A0[4], A1[4], B0[2], B1[2];
                         auto load = [&](int step, double2(&A)[4], double2(&Bf)[2]) {
                             const unsigned e = qu[step >> 2];
@@ -534,7 +546,7 @@ bool eb_multiply_f64(bml_matrix_ellblock_t *A, bml_matrix_ellblock_t *B, bml_mat
             return false;
         if (g.square)
         {
-            f64_sym_kernel<<<rows, PT, 0, c->stream>>>(g);
+            f64_sym_kernel<<<rows, 128, 0, c->stream>>>(g);
             if (!LAUNCH_OK("f64_sym_kernel"))
                 return false;
         }
