@@ -467,10 +467,10 @@ def formed_fraction(X, n, sample=400, seed=0):
 
 
 # ncu capture of one X^2 call on the 30^3 lattice's SP2 iterate (bench.py
-# --profile, 18.57 G reference product terms; profiles/x2_symmetric_lattice30.md):
+# --profile, 18.57 G reference product terms; profiles/x2_tiles_lattice30.md):
 # the product kernel's dram__bytes_read.sum + dram__bytes_write.sum
 NCU_X2_PRODUCTS = 18570945128
-NCU_X2_KERNEL_DRAM = 1111612672 + 169511936
+NCU_X2_KERNEL_DRAM = 2796406784 + 115515136
 
 
 def x2_roofline(B, H, info):
@@ -517,24 +517,21 @@ def x2_roofline(B, H, info):
             "peak_source": src,
             "traffic": NCU_X2_KERNEL_DRAM / NCU_X2_PRODUCTS * P,
             "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of the product kernel "
-                              "(fast_x2_kernel, symmetric form) on the 30^3 case (bench.py --profile: 1.28 GB for "
+                              "(tile_x2_kernel, symmetric form) on the 30^3 case (bench.py --profile: 2.91 GB for "
                               "18.57 G reference product terms), scaled by this call's product terms",
-            "kernel": "fast_x2_kernel (symmetric form: columns k >= i), one ELLPACK X^2 on the SP2 iterate of "
+            "kernel": "tile_x2_kernel (symmetric form: blocks H >= G), one ELLPACK X^2 on the SP2 iterate of "
                       "iteration %d; kernel_seconds by CUDA events around it on the library stream" % (SP2_ITERS - 1),
             "kernel_seconds": t_k, "x2_call_seconds": t_call, "symmetric_form": bool(symmetric),
             "nnz_x": int(nnz_x), "nnz_x2": int(nnz_x2), "products_reference": P,
             "products_formed": int(formed), "products_formed_share": frac_formed,
             "reference_products_per_s": P / t_call,
             "fp64_gflops_formed": 2.0 * formed / t_k / 1e9,
-            "compute_frac": 2.0 * formed / t_k / 1e12 / (FP64_NOMINAL_TFLOPS / 2),
-            "compute_frac_of": "nominal FP64 %.0f TFLOP/s halved (each product is a multiply and a separate "
-                               "atomic add)" % FP64_NOMINAL_TFLOPS,
-            "busiest_unit": {"unit": "L1/shared-memory pipe (l1tex__throughput)", "busy_pct": 92.6,
-                             "shared_atomic_wavefronts_share": 0.59, "l2_pct": 23.5, "dram_pct_of_elapsed": None,
-                             "source": "ncu --set full of fast_x2_kernel on the 30^3 case (bench.py --profile): the "
-                                       "kernel is bound by its shared-memory atomic adds (59% of the shared "
-                                       "wavefronts), neither by HBM bytes nor by FP64 flops"},
-            "gathered_gbs": 12.0 * formed / t_k / 1e9}
+            "compute_frac": 2.0 * formed / t_k / 1e12 / FP64_NOMINAL_TFLOPS,
+            "compute_frac_of": "nominal FP64 %.0f TFLOP/s, counting the products of stored entries only (the 8 x 8 "
+                               "tiles also multiply their zeros)" % FP64_NOMINAL_TFLOPS,
+            "busiest_unit": {"unit": "FP64 tensor pipe (sm__pipe_tensor_subpipe_dmma_cycles_active)",
+                             "busy_pct": 78.1, "l2_pct": 33.9, "dram_pct": 5.3,
+                             "source": "ncu of tile_x2_kernel on the 30^3 case (bench.py --profile)"}}
 
 
 # ---------------------------------------------------------------------------
@@ -571,7 +568,7 @@ def _ref_setup():
     threads = _omp_env()
     from oracle import oracle as O
     if not O.available():
-        raise RuntimeError("oracle/_ref is not built")
+        return None
     import numpy as np
     # the oracle's own copy of the seeded generator: this process never loads
     # the library under test
@@ -584,8 +581,14 @@ def _ref_setup():
     return O, H, D, X2, threads
 
 
+REF_MISSING = "the reference library is not built (oracle/_ref; its sources are needed to build it)"
+
+
 def cpu_baseline():
-    O, H, D, X2, threads = _ref_setup()
+    setup = _ref_setup()
+    if setup is None:
+        return {"unavailable": REF_MISSING}
+    O, H, D, X2, threads = setup
     t0 = time.perf_counter()
     ref_sp2(O, H, D, X2, SP2_ITERS)
     dt = time.perf_counter() - t0
@@ -597,7 +600,10 @@ def cpu_baseline():
 def run_reference(args, rank, world):
     if rank != 0:
         return None
-    O, H, D, X2, threads = _ref_setup()
+    setup = _ref_setup()
+    if setup is None:
+        return {"impl": "reference", "unavailable": REF_MISSING}
+    O, H, D, X2, threads = setup
     warm, steps = args.warmup, args.steps
     for _ in range(warm):
         ref_sp2(O, H, D, X2, SP2_ITERS)
@@ -981,9 +987,10 @@ def ellblock_leg(reps=3):
            "nnz_h": int(nnz_h), "nnz_x2": int(B.lib.bml_b200_nnz(Xt)), "block_products": P,
            "fp64_tflops": flops / te / 1e12,
            "fp64_ceiling_tflops": FP64_NOMINAL_TFLOPS,
-           "fp64_ceiling": "nominal B200 FP64 %.0f TFLOP/s: the library's default (unordered) form sums each "
-                           "block product by fused multiply-adds; the ordered form (bml_b200_set_x2_exact(1)) "
-                           "rounds every multiply and add separately, as the reference, at half that "
+           "fp64_ceiling": "nominal B200 FP64 %.0f TFLOP/s; fp64_tflops counts every block product, and the "
+                           "default (unordered) form of a symmetric X, as here, computes one triangle of them, so "
+                           "its limit is twice that; the ordered form (bml_b200_set_x2_exact(1)) rounds every "
+                           "multiply and add separately, as the reference, at half the "
                            "ceiling" % FP64_NOMINAL_TFLOPS,
            "tc_tflops": 3 * flops / tt / 1e12, "tc_peak_tflops": tc_peak,
            "tc_tflops_note": "three block products (hi*hi, hi*lo, lo*hi) per block pair over the measured "

@@ -9,7 +9,11 @@
 // tr C the sum of the pre-threshold diagonal values of C.  Unlike the ordered
 // tiers (ellpack_multiply.cu), the products of one C[i,k] are added in no
 // fixed order and a row's kept columns come out in ascending column order.
-// Every product a*b is still a separately rounded multiply followed by one
+// This file holds the sparse form.  Products whose operands pack into 8 x 8
+// tiles run on the tile form (ellpack_tiles.cu, which says where the line
+// lies), filled matrices on the dense tier (ellpack_dense.cu).
+//
+// Every product a*b is a separately rounded multiply followed by one
 // rounded add, so |C - C_ref| <= (n-1) u sum_j |A_ij B_jk| for a column summed
 // from n products: 1e-12 of that sum for any n below 4500 in FP64.
 //
