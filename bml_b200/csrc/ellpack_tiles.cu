@@ -97,6 +97,7 @@ struct TileFlags
     int bad;                     // a row length or column out of range
     int odd;                     // an entry not finite, or a row of zeros only: not for this form
     int asym;
+    int alone;                   // tiles above the groups' diagonal blocks that have a mirror, less those below
     int next;                    // work item counter
     int full;                    // the pool ran out
     int overflow, max_width;
@@ -152,7 +153,7 @@ __device__ __forceinline__ void tell_host(const TileArgs &g, int lane)
 // The form does not apply: the kernels after the fill do nothing.
 __device__ __forceinline__ bool declined(const TileFlags *f)
 {
-    return f->bad || f->odd || f->asym || (double) f->tiles2 * TILE_COST > (double) f->products;
+    return f->bad || f->odd || f->asym || f->alone || (double) f->tiles2 * TILE_COST > (double) f->products;
 }
 
 // The four tile rows' bitmaps of group G from the stored columns, in shared
@@ -478,69 +479,90 @@ template <typename T> __global__ void __launch_bounds__(FT) tile_fill_kernel(Til
 }
 
 // Every tile (I, J), J >= I, against tile (J, I): equal bits, or no tile and
-// zeros.  Also the last group H that has a column in common with G.
+// zeros.  A tile below its group's diagonal block has a mirror when the tiles
+// there are as many as those above that have one: checking that each has its
+// mirror took the lists of the other group once more.  Also the last group H
+// that has a column in common with G.
 __global__ void __launch_bounds__(PT) tile_sym_kernel(TileArgs g)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    __shared__ int lastH;
+    __shared__ int lastH, alone;
     if (g.flags->bad)
         return;
     for (int G = blockIdx.x; G < g.NG; G += gridDim.x)
     {
         if (threadIdx.x == 0)
+        {
             lastH = G;
+            alone = 0;
+        }
         __syncthreads();
         const int2 rg = g.range[G];
         int ne = 0;
         if (rg.y >= 0)
             ne = g.rank[(size_t) G * g.nw + rg.y] + __popc(g.bits[(size_t) G * g.nw + rg.y]);
-        int last = G, asym = 0;
+        int last = G, asym = 0, mirrors = 0;
         for (int e = warp; e < ne; e += PT / 32)
         {
             const unsigned en = g.ent[g.eoff[G] + e];
             const int J = g.entJ[g.eoff[G] + e];
             const int H = J >> 2;
             const int2 rh = H < g.NG ? g.range[H] : make_int2(0, -1);
+            // the four tile rows of G lie in one word of H's bitmap, its tiles there are consecutive entries
+            const int s0 = (4 * G) & 31;
+            const bool in = H < g.NG && J >= 4 * G;
+            const unsigned b = in ? g.bits[(size_t) H * g.nw + (4 * G >> 5)] : 0u;
+            int f = in ? g.eoff[H] + g.rank[(size_t) H * g.nw + (4 * G >> 5)] + __popc(b & ((1u << s0) - 1u)) : 0;
             if (rh.y >= 0)
             {
                 // the last tile column of group H
-                const unsigned b = g.bits[(size_t) H * g.nw + rh.y];
-                last = max(last, (rh.y * 32 + 31 - __clz(b)) >> 2);
+                const unsigned bl = g.bits[(size_t) H * g.nw + rh.y];
+                last = max(last, (rh.y * 32 + 31 - __clz(bl)) >> 2);
             }
             if (J < 4 * G)
+            {
+                mirrors -= __popc(en & 15u);
                 continue;
+            }
             const double2 *tp = reinterpret_cast<const double2 *>(g.tiles) + (size_t) (en >> 4) * 128 + lane;
+            double2 x[4];
+            double m0[4], m1[4];
+#pragma unroll
             for (int a = 0; a < 4; ++a)
             {
-                if (!(en >> a & 1u))
-                    continue;
-                const double2 x = tp[32 * a];
-                const int I = 4 * G + a;
-                double m0 = 0.0, m1 = 0.0;
-                const unsigned b = rh.y >= 0 ? g.bits[(size_t) H * g.nw + (I >> 5)] : 0u;
-                if (b >> (I & 31) & 1u)
+                x[a] = make_double2(0.0, 0.0);
+                m0[a] = m1[a] = 0.0;
+                const unsigned fn = b >> (s0 + a) & 1u ? g.ent[f++] : 0u;
+                const bool both = fn >> (J & 3) & 1u;
+                if (en >> a & 1u)
                 {
-                    const int f = g.eoff[H] + g.rank[(size_t) H * g.nw + (I >> 5)] + __popc(b & ((1u << (I & 31)) - 1u));
-                    const unsigned fn = g.ent[f];
-                    const int u = J & 3;
-                    if (fn >> u & 1u)
+                    x[a] = tp[32 * a];
+                    if (both)
                     {
-                        const double *q = g.tiles + (size_t) (4 * (fn >> 4) + u) * 64;
+                        mirrors += J >= 4 * G + 4;
+                        const double *q = g.tiles + (size_t) (4 * (fn >> 4) + (J & 3)) * 64;
                         const int r = lane >> 2, c = lane & 3;
-                        m0 = q[tile_at(c, r)];
-                        m1 = q[tile_at(c + 4, r)];
+                        m0[a] = q[tile_at(c, r)];
+                        m1[a] = q[tile_at(c + 4, r)];
                     }
                 }
-                asym |= x.x != m0 || x.y != m1;
             }
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+                asym |= x[a].x != m0[a] || x[a].y != m1[a];
         }
         for (int o = 16; o; o >>= 1)
             last = max(last, __shfl_xor_sync(FULL, last, o));
         if (lane == 0)
+        {
             atomicMax(&lastH, last);
+            atomicAdd(&alone, mirrors);
+        }
         asym = __syncthreads_or(asym);
         if (threadIdx.x == 0)
         {
+            if (alone)
+                atomicAdd(&g.flags->alone, alone);
             g.last[G] = min(lastH, g.NG - 1);
             if (asym)
                 atomicExch(&g.flags->asym, 1);
@@ -1726,9 +1748,9 @@ bool tile_x2_typed(TileArgs g, double *trace, int *required_M, bool *taken, bool
     tile_rows_kernel<T><<<g.NG, RT, smemR, c->stream>>>(g);
     if (!LAUNCH_OK("tile_rows_kernel") || !b200_sync())
         return false;
-    if (hf->bad || hf->odd || hf->asym || hf->full || (double) hf->tiles2 * TILE_COST > (double) hf->products)
+    if (hf->bad || hf->odd || hf->asym || hf->alone || hf->full || (double) hf->tiles2 * TILE_COST > (double) hf->products)
     {
-        *asym = hf->asym != 0;
+        *asym = hf->asym || hf->alone;
         return true;
     }
     *taken = true;

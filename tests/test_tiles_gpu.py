@@ -140,6 +140,23 @@ def test_matrices_the_tile_form_leaves_to_the_sparse_one():
         np.testing.assert_allclose(got[0], want[0], rtol=1e-9, atol=1e-12)
 
 
+@pytest.mark.parametrize("i,j", [(180, 3), (3, 180), (20, 3), (97, 64), (199, 0)])
+def test_an_entry_without_its_mirror(i, j):
+    """An entry outside the band with no mirror, in a tile that has none
+    either, on each side of the diagonal and within a group of 32 rows: X^2 is
+    not formed as X X^T."""
+    N = 200
+    D = _banded(N, 2, 1.0, 3)
+    D[i, j] = 0.5
+    M = N
+    st, tr, got = _x2(_rows(D, M, False, 0), N, M, N, 0.0, DOUBLE)
+    assert st == B.OK
+    S = np.abs(D) @ np.abs(D)
+    assert (np.abs(_dense(got, N, N) - D @ D) <= 1e-12 * S).all()
+    assert tr[1] == pytest.approx(np.trace(D @ D), rel=1e-12)
+    assert B.lib.bml_b200_last_x2_symmetric() == 0
+
+
 @pytest.mark.parametrize("M2", [40, 76], ids=["pool_runs_out", "rows_too_wide"])
 def test_tiles_row_overflow(M2):
     """A result row wider than M (81 here) is reported, rows hold at most M
