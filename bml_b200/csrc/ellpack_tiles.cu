@@ -47,9 +47,9 @@
 // the bitmaps of B's rows.
 //
 // Measured against the sparse form on one B200: X^2 of the 40^3 lattice's wide
-// iterate (rows of 825) 65.0 -> 21.3 ms, first X^2 of that lattice (rows of
-// 113) 6.3 -> 2.5 ms, FP32 on 26999 rows 2.08 -> 0.84 ms, a chain of 4096 rows
-// of 340 746 -> 148 us, of 512 rows of 33 74 -> 62 us; the adjoint of 3
+// iterate (rows of 825) 65.0 -> 21.1 ms, first X^2 of that lattice (rows of
+// 113) 6.3 -> 2.5 ms, FP32 on 26999 rows 2.07 -> 0.82 ms, a chain of 4096 rows
+// of 340 745 -> 132 us, of 512 rows of 33 71 -> 55 us; the adjoint of 3
 // iterations on the 16^3 lattice 32 -> 21 ms with the host's share.
 // At 40^3 the MMAs that have both tiles take 9.0 ms of the product kernel's 18,
 // those in a pair with only one about 2; the rest is the handling of a common
@@ -85,6 +85,12 @@ constexpr size_t TL_SMALL = 40960; // place in the context's small buffers
 // 3880 to 7360 / 3840, 0.64 2050 / 2110, 1.45 (2000 rows) 167 to 185 / 134,
 // 1.88 847 / 1770, 1.94 370 / 807, 5.3 140 / 475; lattices have 8 to 70).
 constexpr double TILE_COST = 1.5;
+// A general product's ten launches and two waits take about 150 us whatever
+// its size, so matrices of fewer rows stay with the sparse form (A*B on
+// lattices, tile form against sparse form in us: 1721 rows 176 / 105, 207 /
+// 150, 202 / 151 and 250 / 274 for 5, 20, 17 and 82 M products; 4089 rows 200
+// / 200 and 287 / 488 for 11 and 90 M; 7993 rows 264 / 303 and 479 / 710).
+constexpr int GENERAL_ROWS = 4096;
 constexpr long long LAZY_BYTES = 128 << 20; // most tile places of a matrix laid out without counting them
 
 struct TileFlags
@@ -1848,7 +1854,7 @@ bool ell_general_tiles(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bml_mat
 {
     *taken = false;
     const int nbk = b200_ceil_div(A->N, 8);
-    if (!(threshold >= 0.0) || A->N != B->N || A->N != C->N || nbk > 65535)
+    if (!(threshold >= 0.0) || A->N < GENERAL_ROWS || A->N != B->N || A->N != C->N || nbk > 65535)
         return true;
     TileArgs a{};
     a.N = a.ncols = A->N;

@@ -226,7 +226,10 @@ def _random_band(N, band, density, seed, empty, dtype):
 @pytest.mark.parametrize("square", [False, True], ids=["ab", "x2_not_symmetric"])
 @pytest.mark.parametrize("N,ba,bb,density,empty", [
     (1, 0, 0, 1.0, ()), (9, 2, 8, 0.9, (3,)), (32, 31, 5, 0.8, ()), (33, 4, 33, 0.7, (0, 32)),
-    (257, 30, 60, 0.6, tuple(range(32, 64))), (400, 399, 20, 0.5, ()), (900, 12, 80, 0.9, ())])
+    (257, 30, 60, 0.6, tuple(range(32, 64))), (400, 399, 20, 0.5, ()), (900, 12, 80, 0.9, ()),
+    # matrices of fewer than 4096 rows take the sparse form
+    (4095, 4, 33, 0.7, ()), (4096, 12, 80, 0.9, ()), (4097, 399, 20, 0.5, (0, 4096)),
+    (4129, 30, 60, 0.6, tuple(range(32, 64)))])
 def test_general_tiles(N, ba, bb, density, empty, square, dtype):
     """A*B and X^2 of matrices that are not symmetric, rows in any order: the
     kept entries and the diagonal where some product touches it, against the
