@@ -308,6 +308,10 @@ __global__ void __launch_bounds__(W * 32, 3) add_map_kernel(T *Av, int *Ai, int 
     const bool use_b = beta > 0.0 || beta < 0.0;
     for (int s = tid; s < MAP_COLS / 8; s += NT)
         reinterpret_cast<uint4 *>(smem)[s] = make_uint4(0u, 0u, 0u, 0u);
+    auto claim = [&](int at) { // marks the place used; true for the first to do so
+        const unsigned bit = (unsigned) USED << 16 * (at & 1);
+        return !(atomicOr(reinterpret_cast<unsigned *>(smem) + (at >> 1), bit) & bit);
+    };
     for (int i = blockIdx.x; i < N; i += gridDim.x)
     {
         const int na = use_a ? An[i] : 0;
@@ -425,12 +429,10 @@ __global__ void __launch_bounds__(W * 32, 3) add_map_kernel(T *Av, int *Ai, int 
                 xx[u] = axpy_d(T(0), alpha, xx[u]);
                 if (kk[u] >= blo && kk[u] <= bhi)
                 {
+                    // of several entries of A in one column (set_element appends to short rows), one takes B's
                     const unsigned short m = map[kk[u] & (MAP_COLS - 1)];
-                    if (m)
-                    {
-                        map[kk[u] & (MAP_COLS - 1)] = m | USED;
-                        xx[u] = axpy_d(xx[u], beta, __ldg(Bv + rb + (m & (USED - 1)) - 1));
-                    }
+                    if (m && !(m & USED) && claim(kk[u] & (MAP_COLS - 1)))
+                        xx[u] = axpy_d(xx[u], beta, __ldg(Bv + rb + m - 1));
                 }
                 keep[u] = __ballot_sync(FULL, p0 + (warp * MAP_U + u) * 32 + lane < na && fabs(xx[u]) > thr_t);
             }

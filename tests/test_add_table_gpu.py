@@ -110,3 +110,25 @@ def test_trace_mult_sized_by_rows(wa, wb):
         want += sum(p)
         size += sum(map(abs, p))
     assert abs(B.lib.bml_trace_mult(A.h, Bm.h) - want) <= 1e-12 * max(size, 1e-300)
+
+
+def test_add_to_a_column_stored_twice():
+    """Two entries of A in one column (bml_set_element appends to rows of at
+    most two entries): B's entry joins the sum once."""
+    import ctypes as C
+    N, M = 40, 8
+    A, Bm = B.Ellpack(N, M), B.Ellpack(N, M)
+    x = C.c_double()
+    for i in range(N):
+        for y in (1.0, 2.0):
+            x.value = y
+            B.lib.bml_set_element(A.h, i, (i + 3) % N, C.byref(x))
+        x.value = 10.0
+        B.lib.bml_set_element(Bm.h, i, (i + 3) % N, C.byref(x))
+    B.lib.bml_add(A.h, Bm.h, 1.0, 0.5, 0.0)
+    B.check()
+    v, ix, nz = A.download()
+    for i in range(N):
+        at = slice(i * M, i * M + nz[i])
+        assert list(ix[at]) == [(i + 3) % N] * 2
+        assert v[at].sum() == 8.0
