@@ -93,6 +93,44 @@ __device__ __forceinline__ int hash_get(const int *keys, const int *pay, unsigne
     return -1;
 }
 
+// Place of column k in the hash, or -1.
+__device__ __forceinline__ int hash_find(const int *keys, unsigned mask, int k)
+{
+    unsigned h = hash_slot(k, mask);
+#pragma unroll 1
+    for (unsigned p = 0; p <= mask; ++p)
+    {
+        const int cur = keys[h];
+        if (cur == k)
+            return (int) h;
+        if (cur == B200_EMPTY_KEY)
+            return -1;
+        h = (h + 1) & mask;
+    }
+    return -1;
+}
+
+// hash_put that tells whether the column was there already.
+__device__ __forceinline__ bool hash_add(int *keys, int *pay, unsigned mask, int k, int v)
+{
+    unsigned h = hash_slot(k, mask);
+    volatile int *vk = keys;
+#pragma unroll 1
+    for (unsigned p = 0; p <= mask; ++p)
+    {
+        int old = vk[h];
+        if (old == B200_EMPTY_KEY)
+            old = atomicCAS(&keys[h], B200_EMPTY_KEY, k);
+        if (old == B200_EMPTY_KEY || old == k)
+        {
+            pay[h] = v;
+            return old == k;
+        }
+        h = (h + 1) & mask;
+    }
+    return false;
+}
+
 } // namespace b200
 
 // Sum of one or two per-row arrays in FP64 with a fixed order (each thread a

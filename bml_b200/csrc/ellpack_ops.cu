@@ -715,12 +715,16 @@ __global__ void diag_kernel(const T *Av, const int *Ai, const int *An, int ld, i
 // (the reference's bml_getVector_ellpack reads B's row i at A's columns,
 // ellpack/bml_trace_ellpack_typed.c:145-158 with
 // ellpack/bml_submatrix_ellpack_typed.c:380-406; a column absent from B's row
-// contributes 0).  Per-row partial sums in FP64.  One warp per row, B's row in
-// a shared-memory hash of 2^logts slots per warp.
+// contributes 0).  Per-row partial sums in FP64.  One warp per row, the hashed
+// matrix's row in a shared-memory hash of 2^logts slots per warp; with
+// hash_a, the roles are exchanged and A is hashed.  A column that a row stores
+// twice (set_element appends to short rows) shows as a key found on insertion
+// or, of the row not hashed, as a place of A's hit twice; such a row is summed
+// by search: every entry of A, against the last of B's in its column.
 template <typename T>
 __global__ void trace_mult_kernel(const T *Av, const int *Ai, const int *An, int lda,
                                   const T *Bv, const int *Bi, const int *Bn, int ldb, int N,
-                                  int logts, double *part)
+                                  int logts, int hash_a, double *part)
 {
     extern __shared__ __align__(128) unsigned char smem[];
     const int TS = 1 << logts;
@@ -731,25 +735,44 @@ __global__ void trace_mult_kernel(const T *Av, const int *Ai, const int *An, int
     const int warps = (gridDim.x * blockDim.x) >> 5;
     for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < N; i += warps)
     {
+        const int na = An[i], nb = Bn[i];
+        const int *ai = Ai + (size_t) i * lda, *bi = Bi + (size_t) i * ldb;
+        const T *av = Av + (size_t) i * lda, *bv = Bv + (size_t) i * ldb;
+        const int *hi = hash_a ? ai : bi, *pi = hash_a ? bi : ai;
+        const T *hv = hash_a ? av : bv, *pv = hash_a ? bv : av;
+        const int nh = hash_a ? na : nb, np = hash_a ? nb : na;
         for (int s = lane; s < TS; s += 32)
             keys[s] = B200_EMPTY_KEY;
         __syncwarp();
-        const int nb = Bn[i];
-        for (int c0 = 0; c0 < nb; c0 += 32)
+        bool twice = false;
+        for (int c0 = 0; c0 < nh; c0 += 32)
         {
             const int p = c0 + lane;
-            if (p < nb)
-                hash_put(keys, pos, mask, Bi[(size_t) i * ldb + p], p);
+            if (p < nh)
+                twice |= hash_add(keys, pos, mask, hi[p], p);
             __syncwarp();
         }
-        __syncwarp();
         double s = 0.0;
-        const int na = An[i];
-        for (int p = lane; p < na; p += 32)
+        for (int p = lane; p < np; p += 32)
         {
-            const int q = hash_get(keys, pos, mask, Ai[(size_t) i * lda + p]);
-            if (q >= 0)
-                s += (double) mul_rn(Av[(size_t) i * lda + p], Bv[(size_t) i * ldb + q]);
+            const int h = hash_find(keys, mask, pi[p]);
+            if (h < 0)
+                continue;
+            const int q = hash_a ? atomicOr(&pos[h], INT_MIN) : pos[h];
+            twice |= q < 0;
+            s += (double) mul_rn(pv[p], hv[q & INT_MAX]);
+        }
+        if (__any_sync(FULL, twice))
+        {
+            s = 0.0;
+            for (int p = lane; p < na; p += 32)
+            {
+                int q = nb - 1;
+                while (q >= 0 && bi[q] != ai[p])
+                    --q;
+                if (q >= 0)
+                    s += (double) mul_rn(av[p], bv[q]);
+            }
         }
         for (int o = 16; o; o >>= 1)
             s += __shfl_xor_sync(FULL, s, o);
@@ -1234,12 +1257,11 @@ bool ell_trace_mult(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, double *tr
     B200Context *c = b200_ctx();
     if (!c || !ell_to_device(A) || !ell_to_device(B))
         return false;
-    // The hash takes the rows of the narrower matrix (the sum is symmetric in
-    // A and B), sized by its widest row where finding that out (a pass over
+    // The hash takes the rows of the narrower matrix, sized by its widest row where finding that out (a pass over
     // the row lengths and a round trip, about 15 us each) is small against the
     // operation: sized by M = 2048, tr(D H) of the 40^3 density matrix took
     // 3.2 ms with 4 warps per SM.
-    int wb = B->M;
+    int wb = B->M, hash_a = 0;
     if ((long long) A->N * (A->M + B->M) >= 1 << 22)
     {
         int wa = A->M;
@@ -1248,11 +1270,8 @@ bool ell_trace_mult(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, double *tr
             return false;
         if (B == A)
             wb = wa;
-        if (wa < wb)
-        {
-            std::swap(A, B);
-            wb = wa;
-        }
+        hash_a = wa < wb;
+        wb = min(wa, wb);
     }
     double *part = static_cast<double *>(b200_scratch((size_t) A->N * sizeof(double)));
     if (!part)
@@ -1277,7 +1296,7 @@ bool ell_trace_mult(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, double *tr
             return false;
         k<<<grid, 32 * warps_per_block, smem, c->stream>>>(
             static_cast<const double *>(A->d_value), A->d_index, A->d_nnz, A->ld,
-            static_cast<const double *>(B->d_value), B->d_index, B->d_nnz, B->ld, A->N, logts, part);
+            static_cast<const double *>(B->d_value), B->d_index, B->d_nnz, B->ld, A->N, logts, hash_a, part);
     }
     else
     {
@@ -1286,7 +1305,7 @@ bool ell_trace_mult(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, double *tr
             return false;
         k<<<grid, 32 * warps_per_block, smem, c->stream>>>(
             static_cast<const float *>(A->d_value), A->d_index, A->d_nnz, A->ld,
-            static_cast<const float *>(B->d_value), B->d_index, B->d_nnz, B->ld, A->N, logts, part);
+            static_cast<const float *>(B->d_value), B->d_index, B->d_nnz, B->ld, A->N, logts, hash_a, part);
     }
     double *out = reinterpret_cast<double *>(static_cast<unsigned char *>(c->d_small) + 3072);
     b200_count_launch(); // trace_mult_kernel

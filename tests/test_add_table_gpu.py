@@ -132,3 +132,31 @@ def test_add_to_a_column_stored_twice():
         at = slice(i * M, i * M + nz[i])
         assert list(ix[at]) == [(i + 3) % N] * 2
         assert v[at].sum() == 8.0
+
+
+@pytest.mark.parametrize("wa,wb", [(20, 300), (300, 20), (2, 300), (40, 40)])
+@pytest.mark.parametrize("twice", ["a", "b"])
+def test_trace_mult_of_columns_stored_twice(wa, wb, twice):
+    """Every entry of A counts once, against the last of B's in its column."""
+    N, M, ncols = 5000, 512, 5000
+    a = _random(N, M, ncols, (wa,), (600,), 7, np.float64)
+    b = _random(N, M, ncols, (wb,), (600,), 8, np.float64)
+    for x in (a, b):
+        for i in range(0, N, 2):  # columns that both store
+            n = min(a[2][i], b[2][i]) // 2
+            if x is b:
+                free = [k for k in b[1][i, n:b[2][i]] if k not in set(a[1][i, :n])]
+                b[1][i, :n], b[1][i, n:n + len(free)] = a[1][i, :n], free
+                b[2][i] = n + len(free)
+    d = a if twice == "a" else b
+    for i in range(0, N, 3):
+        if d[2][i] >= 2:
+            d[1][i, d[2][i] - 1] = d[1][i, 0]
+    A, Bm = (B.Ellpack.from_arrays(*x, N, M) for x in (a, b))
+    want = size = 0.0
+    for i in range(N):
+        y = dict(zip(b[1][i, :b[2][i]].tolist(), b[0][i, :b[2][i]].tolist()))
+        p = [x * y[k] for k, x in zip(a[1][i, :a[2][i]].tolist(), a[0][i, :a[2][i]].tolist()) if k in y]
+        want += sum(p)
+        size += sum(map(abs, p))
+    assert abs(B.lib.bml_trace_mult(A.h, Bm.h) - want) <= 1e-12 * size
