@@ -4,6 +4,7 @@
 #include "device_util.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <cfloat>
 #include <climits>
 #include <cmath>
@@ -715,17 +716,28 @@ __global__ void diag_kernel(const T *Av, const int *Ai, const int *An, int ld, i
 // (the reference's bml_getVector_ellpack reads B's row i at A's columns,
 // ellpack/bml_trace_ellpack_typed.c:145-158 with
 // ellpack/bml_submatrix_ellpack_typed.c:380-406; a column absent from B's row
-// contributes 0).  Per-row partial sums in FP64.  One warp per row, the hashed
-// matrix's row in a shared-memory hash of 2^logts slots per warp; with
-// hash_a, the roles are exchanged and A is hashed.  A column that a row stores
-// twice (set_element appends to short rows) shows as a key found on insertion
-// or, of the row not hashed, as a place of A's hit twice; such a row is summed
-// by search: every entry of A, against the last of B's in its column.
+// contributes 0).  Per-row partial sums in FP64.  One warp per row, the
+// narrower of its two rows in a shared-memory hash of 2^logts slots per warp.
+// A column that a row stores twice (set_element appends to short rows) shows
+// as a key found on insertion or, of the row not hashed, as a place hit twice;
+// such a row is summed by search: every entry of A, against the last of B's
+// in its column.
+//
+// The hash bounds the warps of an SM, so rows go to the first of a few sizes
+// that is at most half full, a launch each: this one sums the rows of more
+// than `done` entries that fit, and where some do not stores the call's number
+// in *beyond.  The next size returns at once unless it finds the number there
+// (an old value that happens to be equal costs it a look at every row).
+// us, sized by M | by the widest row, found in a pass with a wait | so:
+// tr(D H) at 40^3 (rows of 925 and 123, M = 2048) 2712 | 320 | 262; 4096 rows
+// of 33 and 61, M = 1024 31 | 60 | 32; 64000 such rows, M = 64 58 | 95 | 67.
 template <typename T>
 __global__ void trace_mult_kernel(const T *Av, const int *Ai, const int *An, int lda,
                                   const T *Bv, const int *Bi, const int *Bn, int ldb, int N,
-                                  int logts, int hash_a, double *part)
+                                  int logts, int done, const int *need, int *beyond, int call,
+                                  double *part)
 {
+    constexpr int TU = 2, USED = 1 << 30;
     extern __shared__ __align__(128) unsigned char smem[];
     const int TS = 1 << logts;
     const unsigned mask = TS - 1;
@@ -733,9 +745,19 @@ __global__ void trace_mult_kernel(const T *Av, const int *Ai, const int *An, int
     int *keys = reinterpret_cast<int *>(smem) + (size_t) warp * 2 * TS;
     int *pos = keys + TS;
     const int warps = (gridDim.x * blockDim.x) >> 5;
+    if (need && *need != call)
+        return;
     for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < N; i += warps)
     {
         const int na = An[i], nb = Bn[i];
+        const bool hash_a = na < nb;
+        if (min(na, nb) <= done)
+            continue;
+        if (2 * min(na, nb) > TS)
+        {
+            *beyond = call;
+            continue;
+        }
         const int *ai = Ai + (size_t) i * lda, *bi = Bi + (size_t) i * ldb;
         const T *av = Av + (size_t) i * lda, *bv = Bv + (size_t) i * ldb;
         const int *hi = hash_a ? ai : bi, *pi = hash_a ? bi : ai;
@@ -744,23 +766,39 @@ __global__ void trace_mult_kernel(const T *Av, const int *Ai, const int *An, int
         for (int s = lane; s < TS; s += 32)
             keys[s] = B200_EMPTY_KEY;
         __syncwarp();
+        // TU entries per lane loaded before any is looked up
         bool twice = false;
-        for (int c0 = 0; c0 < nh; c0 += 32)
+        for (int c0 = lane; c0 < nh; c0 += 32 * TU)
         {
-            const int p = c0 + lane;
-            if (p < nh)
-                twice |= hash_add(keys, pos, mask, hi[p], p);
-            __syncwarp();
+            int k[TU];
+#pragma unroll
+            for (int u = 0; u < TU; ++u)
+                k[u] = c0 + 32 * u < nh ? __ldg(hi + c0 + 32 * u) : 0;
+#pragma unroll
+            for (int u = 0; u < TU; ++u)
+                if (c0 + 32 * u < nh)
+                    twice |= hash_add(keys, pos, mask, k[u], c0 + 32 * u);
         }
+        __syncwarp();
         double s = 0.0;
-        for (int p = lane; p < np; p += 32)
+        for (int c0 = lane; c0 < np; c0 += 32 * TU)
         {
-            const int h = hash_find(keys, mask, pi[p]);
-            if (h < 0)
-                continue;
-            const int q = hash_a ? atomicOr(&pos[h], INT_MIN) : pos[h];
-            twice |= q < 0;
-            s += (double) mul_rn(pv[p], hv[q & INT_MAX]);
+            int k[TU], q[TU];
+#pragma unroll
+            for (int u = 0; u < TU; ++u)
+                k[u] = c0 + 32 * u < np ? __ldg(pi + c0 + 32 * u) : 0;
+#pragma unroll
+            for (int u = 0; u < TU; ++u)
+            {
+                const int h = c0 + 32 * u < np ? hash_find(keys, mask, k[u]) : -1;
+                q[u] = h < 0 ? -1 : hash_a ? atomicOr(&pos[h], USED) : pos[h];
+                if (h >= 0 && q[u] & USED)
+                    twice = true;
+            }
+#pragma unroll
+            for (int u = 0; u < TU; ++u)
+                if (q[u] >= 0)
+                    s += (double) mul_rn(__ldg(pv + c0 + 32 * u), __ldg(hv + (q[u] & (USED - 1))));
         }
         if (__any_sync(FULL, twice))
         {
@@ -1250,6 +1288,9 @@ bool ell_trace(bml_matrix_ellpack_t *A, double *trace)
     return true;
 }
 
+// Hash sizes (log2): rows of up to 128 entries, of up to 1024, then any width.
+constexpr int TRACE_NARROW = 8, TRACE_WIDE = 11;
+
 bool ell_trace_mult(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, double *trace)
 {
     if (!check_pair(A, B, "trace_mult"))
@@ -1257,58 +1298,47 @@ bool ell_trace_mult(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, double *tr
     B200Context *c = b200_ctx();
     if (!c || !ell_to_device(A) || !ell_to_device(B))
         return false;
-    // The hash takes the rows of the narrower matrix, sized by its widest row where finding that out (a pass over
-    // the row lengths and a round trip, about 15 us each) is small against the
-    // operation: sized by M = 2048, tr(D H) of the 40^3 density matrix took
-    // 3.2 ms with 4 warps per SM.
-    int wb = B->M, hash_a = 0;
-    if ((long long) A->N * (A->M + B->M) >= 1 << 22)
-    {
-        int wa = A->M;
-        long long t;
-        if (!ell_nnz_total(A, &t, &wa) || (B != A && !ell_nnz_total(B, &t, &wb)))
-            return false;
-        if (B == A)
-            wb = wa;
-        hash_a = wa < wb;
-        wb = min(wa, wb);
-    }
     double *part = static_cast<double *>(b200_scratch((size_t) A->N * sizeof(double)));
     if (!part)
         return false;
-    int logts = 5;
-    while ((1 << logts) < 2 * wb)
-        ++logts;
-    int warps_per_block = 4;
-    size_t smem = (size_t) warps_per_block * 2 * (1 << logts) * sizeof(int);
-    while (smem > c->smem_optin && warps_per_block > 1)
-    {
-        warps_per_block >>= 1;
-        smem >>= 1;
-    }
-    if (smem > c->smem_optin)
+    int full = 5; // holds every row at most half full
+    while ((1 << full) < 2 * min(A->M, B->M))
+        ++full;
+    if ((size_t) 2 * sizeof(int) << full > c->smem_optin)
         return ell_trace_mult_wide(A, B, trace);
-    const int grid = min(b200_ceil_div(A->N, warps_per_block), c->sm_count * 16);
-    if (A->matrix_precision == double_real)
+    static std::atomic<int> calls{0};
+    const int call = ++calls;
+    int *beyond = reinterpret_cast<int *>(static_cast<unsigned char *>(c->d_small) + 3072) + 16;
+    const int *need = nullptr;
+    int done = -1;
+    for (int logts : {TRACE_NARROW, TRACE_WIDE, full})
     {
-        auto k = trace_mult_kernel<double>;
-        if (!CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)))
+        if (logts > full)
+            continue;
+        int warps_per_block = 4;
+        while ((size_t) warps_per_block * 2 * sizeof(int) << logts > c->smem_optin)
+            warps_per_block >>= 1;
+        const size_t smem = (size_t) warps_per_block * 2 * sizeof(int) << logts;
+        const int grid = min(b200_ceil_div(A->N, warps_per_block), c->sm_count * 16);
+        auto launch = [&](auto kern, auto *av, auto *bv) {
+            if (!CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)))
+                return false;
+            kern<<<grid, 32 * warps_per_block, smem, c->stream>>>(av, A->d_index, A->d_nnz, A->ld, bv, B->d_index,
+                                                                  B->d_nnz, B->ld, A->N, logts, done, need, beyond, call, part);
+            return LAUNCH_OK("trace_mult_kernel");
+        };
+        if (A->matrix_precision == double_real
+                ? !launch(trace_mult_kernel<double>, static_cast<const double *>(A->d_value),
+                          static_cast<const double *>(B->d_value))
+                : !launch(trace_mult_kernel<float>, static_cast<const float *>(A->d_value),
+                          static_cast<const float *>(B->d_value)))
             return false;
-        k<<<grid, 32 * warps_per_block, smem, c->stream>>>(
-            static_cast<const double *>(A->d_value), A->d_index, A->d_nnz, A->ld,
-            static_cast<const double *>(B->d_value), B->d_index, B->d_nnz, B->ld, A->N, logts, hash_a, part);
-    }
-    else
-    {
-        auto k = trace_mult_kernel<float>;
-        if (!CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)))
-            return false;
-        k<<<grid, 32 * warps_per_block, smem, c->stream>>>(
-            static_cast<const float *>(A->d_value), A->d_index, A->d_nnz, A->ld,
-            static_cast<const float *>(B->d_value), B->d_index, B->d_nnz, B->ld, A->N, logts, hash_a, part);
+        if (logts == full)
+            break;
+        done = 1 << (logts - 1);
+        need = beyond++;
     }
     double *out = reinterpret_cast<double *>(static_cast<unsigned char *>(c->d_small) + 3072);
-    b200_count_launch(); // trace_mult_kernel
     b200_sum_rows_kernel<<<1, 1024, 0, c->stream>>>(part, nullptr, A->N, out);
     if (!LAUNCH_OK("trace_mult kernels"))
         return false;
