@@ -116,12 +116,13 @@ __global__ void __launch_bounds__(256) dense_pattern_kernel(const int *ix, const
 
 // touched[i] = 1 when some stored A[i,j] meets a stored B[j,i]; dA[i] = sum of
 // A's diagonal entries.  One warp per row of A.  In a symmetric square
-// (*asym == 0) an entry that is not zero has its mirror; a row of zeros looks
-// for one in the rows that it names.
+// (*asym == 0) an entry of the image that is not zero has its mirror (a stored
+// one may not: entries of one column add up, perhaps to zero); a row of zeros
+// looks for one in the rows that it names.
 template <typename T>
 __global__ void __launch_bounds__(256) dense_diag_kernel(const T *v, const int *ix, const int *nz, int ldE, int nrows,
                                                          int ncols, const unsigned char *patBt, size_t ld,
-                                                         const int *asym, int *touched, double *dA)
+                                                         const T *img, const int *asym, int *touched, double *dA)
 {
     const bool sym = asym && *asym == 0;
     const int lane = threadIdx.x & 31;
@@ -132,18 +133,19 @@ __global__ void __launch_bounds__(256) dense_diag_kernel(const T *v, const int *
         int hit = 0;
         double d = 0.0;
         if (n >= 0 && n <= ldE)
+        {
+#pragma unroll 4
             for (int p = lane; p < n; p += 32)
+                if (ix[(size_t) i * ldE + p] == i)
+                    d += (double) v[(size_t) i * ldE + p];
+            for (int p0 = 0; p0 < n && !__any_sync(FULL, hit); p0 += 32)
             {
-                const int j = ix[(size_t) i * ldE + p];
-                if (j < 0 || j >= ncols)
-                    continue;
-                const T x = v[(size_t) i * ldE + p];
+                const int j = p0 + lane < n ? ix[(size_t) i * ldE + p0 + lane] : -1;
                 // B[j,i] stored <=> patBt[i * ld + j]
-                if (sym ? x != T(0) : i < ncols && patBt[(size_t) i * ld + j])
-                    hit = 1;
-                if (j == i)
-                    d += (double) x;
+                if (j >= 0 && j < ncols)
+                    hit = sym ? img[(size_t) i * ld + j] != T(0) : i < ncols && patBt[(size_t) i * ld + j];
             }
+        }
         if (sym && n > 0 && n <= ldE && !__any_sync(FULL, hit))
             for (int p = 0; p < n; ++p)
             {
@@ -491,7 +493,8 @@ bool dense_typed(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bml_matrix_el
     if (!LAUNCH_OK("dense_pattern_kernel"))
         return false;
     dense_diag_kernel<T><<<wgrid, 256, 0, c->stream>>>(static_cast<const T *>(A->d_value), A->d_index, A->d_nnz,
-                                                       A->ld, NA, B->N, pat, ld, asym, touched, trace ? dA : nullptr);
+                                                       A->ld, NA, B->N, pat, ld, DA, asym, touched,
+                                                       trace ? dA : nullptr);
     if (!LAUNCH_OK("dense_diag_kernel"))
         return false;
     const dim3 grid((unsigned) (ld / DT), (unsigned) (ld / DT));

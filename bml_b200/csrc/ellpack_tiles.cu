@@ -101,7 +101,7 @@ struct TileFlags
     int entries;                 // (group, J) entries of X
     int reach, reachB;           // largest |column - row|; of the second operand
     int bad;                     // a row length or column out of range
-    int odd;                     // an entry not finite, or a row of zeros only: not for this form
+    int odd;                     // an entry not finite, or a row whose tiles are zero: not for this form
     int asym;
     int alone;                   // tiles above the groups' diagonal blocks that have a mirror, less those below
     int next;                    // work item counter
@@ -428,7 +428,6 @@ template <typename T> __global__ void __launch_bounds__(FT) tile_fill_kernel(Til
             const int *xi = g.Xi + (size_t) i * g.ld;
             const bool sorted = order >> r & 1u;
             const int a = r >> 3;
-            bool some = false;
             double d = 0.0;
             for (int p0 = lane; p0 < n; p0 += 128)
             {
@@ -449,7 +448,6 @@ template <typename T> __global__ void __launch_bounds__(FT) tile_fill_kernel(Til
                     const int k = kk[u];
                     const double v = (double) vv[u];
                     odd |= !(fabs(v) <= 1.7976931348623157e308);
-                    some |= v != 0.0;
                     if (k == i)
                         d += v;
                     const int w = k >> 8;
@@ -463,8 +461,6 @@ template <typename T> __global__ void __launch_bounds__(FT) tile_fill_kernel(Til
                         atomicAdd(at, v);
                 }
             }
-            // a stored row of zeros touches its diagonal without a sign of it in the tiles
-            odd |= n > 0 && !__any_sync(FULL, some) && !g.masked && !g.general;
             for (int o = 16; o; o >>= 1)
                 d += __shfl_xor_sync(FULL, d, o);
             if (lane == 0)
@@ -810,6 +806,7 @@ template <typename T, int MODE> __global__ void __launch_bounds__(TW * 32, TMIN)
         unsigned mask[4];
         int pre[4], total = 0;
         double dsum = 0.0;
+        bool zero = false;
 #pragma unroll
         for (int a = 0; a < 4; ++a)
         {
@@ -828,7 +825,10 @@ template <typename T, int MODE> __global__ void __launch_bounds__(TW * 32, TMIN)
                     {
                         keep = c == r ? live : keep && (GENERAL || c > r);
                         if (c == r && live)
+                        {
                             dsum += (double) x;
+                            zero |= acc[a][b][h] == 0.0;
+                        }
                     }
                     m |= (keep ? 1u : 0u) << c;
                 }
@@ -853,6 +853,10 @@ template <typename T, int MODE> __global__ void __launch_bounds__(TW * 32, TMIN)
                 dsum += __shfl_xor_sync(FULL, dsum, o);
             if (lane == 0)
                 g.dC[G] = dsum;
+            // a row of stored zeros, or of entries that cancel: the tiles of a symmetric square do not tell whether
+            // a product touches its diagonal
+            if (!GENERAL && zero)
+                atomicExch(&g.flags->odd, 1);
         }
         if (total == 0)
             continue;

@@ -82,3 +82,19 @@ def test_dense_tier(N, kind, dtype):
     assert (abs(G - want)[K] <= tol[K] + 1e-300).all()
     if kind == "symmetric":
         assert np.array_equal(G, G.T)
+
+
+def test_entries_of_a_row_that_cancel():
+    """A row whose two entries lie in one column and cancel, nothing stored in
+    its own column: no product touches its diagonal."""
+    N = 1024
+    D = np.random.default_rng(1).standard_normal((N, N))
+    D = D + D.T
+    D[50] = D[:, 50] = 0.0
+    (v, ix, nz), M = _ell(D != 0, D, False)
+    v[50 * M:50 * M + 2], ix[50 * M:50 * M + 2], nz[50] = (1.0, -1.0), 49, 2
+    Y = B.Ellpack(N, N)
+    st, tr = B.multiply_x2(B.Ellpack.from_arrays(v, ix, nz, N, M), Y, 1e-9)
+    assert st == B.OK and B.lib.bml_b200_last_x2_dense() == 1
+    assert Y.download()[2][50] == 0
+    assert abs(tr[1] - np.trace(D @ D)) <= 1e-12 * np.trace(abs(D) @ abs(D))

@@ -140,6 +140,19 @@ def test_matrices_the_tile_form_leaves_to_the_sparse_one():
         np.testing.assert_allclose(got[0], want[0], rtol=1e-9, atol=1e-12)
 
 
+def test_entries_of_a_row_that_cancel():
+    """A row whose two entries lie in one column and cancel, nothing stored in
+    its own column: no product touches its diagonal."""
+    N, M = 200, 20
+    D = _banded(N, 5, 1.0, 3, (50,))
+    v, ix, nz = _rows(D, M, False, 0)
+    v[50 * M:50 * M + 2], ix[50 * M:50 * M + 2], nz[50] = (1.0, -1.0), 49, 2
+    st, tr, got = _x2((v, ix, nz), N, M, N, 1e-9, DOUBLE)
+    assert st == B.OK
+    assert got[2][50] == 0
+    assert tr[1] == pytest.approx(np.trace(D @ D), rel=1e-12)
+
+
 @pytest.mark.parametrize("i,j", [(180, 3), (3, 180), (20, 3), (97, 64), (199, 0)])
 def test_an_entry_without_its_mirror(i, j):
     """An entry outside the band with no mirror, in a tile that has none
