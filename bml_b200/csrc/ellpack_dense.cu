@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(DTHREADS, 1) dense_gemm_f64_kernel(const doubl
 template <typename T> __global__ void __launch_bounds__(256) dense_sym_kernel(const T *A, size_t ld, int *asym)
 {
     __shared__ T t[32][33];
-    if (blockIdx.x < blockIdx.y || *(volatile int *) asym)
+    if (blockIdx.x < blockIdx.y || __syncthreads_or(*(volatile int *) asym)) // other CTAs set it meanwhile
         return;
     const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
     const size_t i0 = (size_t) blockIdx.y * 32, j0 = (size_t) blockIdx.x * 32;
