@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(128) f64_sym_kernel(F64Args g)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int ib = blockIdx.x; ib < g.NB; ib += gridDim.x)
     {
-        if (*(volatile int *) &g.flags->asym)
+        if (__any_sync(FULL, *(volatile int *) &g.flags->asym)) // other warps set it meanwhile
             return;
         const int n = g.An[ib];
         int bad = 0;

@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(256) sym_check_kernel(FastArgs g)
         return;
     for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < g.NB; i += warps)
     {
-        if (*(volatile int *) &g.flags->asym)
+        if (__any_sync(FULL, *(volatile int *) &g.flags->asym)) // other warps set it meanwhile
             return;
         const int ni = g.Bn[i];
         const RowView<T> r = row_of<T>(g, i);
