@@ -150,6 +150,38 @@ void *b200_scratch_try(size_t bytes)
     return c->scratch;
 }
 
+bool b200_device_alloc(void **p, size_t bytes)
+{
+    B200Context *c = b200_ctx();
+    if (!c)
+        return false;
+    for (int attempt = 0; attempt < 3; ++attempt)
+    {
+        if (cudaMallocAsync(p, bytes, c->stream) == cudaSuccess)
+            return true;
+        cudaGetLastError();
+        *p = nullptr;
+        if (attempt == 0)
+        {
+            // the scratch arena gives way to a matrix
+            if (c->scratch)
+                cudaFreeAsync(c->scratch, c->stream);
+            c->scratch = nullptr;
+            c->scratch_bytes = 0;
+        }
+        else
+        {
+            // and so does what the pool keeps of freed ones
+            cudaMemPool_t pool;
+            if (cudaDeviceGetDefaultMemPool(&pool, c->device) == cudaSuccess)
+                cudaMemPoolTrimTo(pool, 0);
+        }
+        if (cudaStreamSynchronize(c->stream) != cudaSuccess)
+            break;
+    }
+    return false;
+}
+
 bool b200_sync()
 {
     B200Context *c = b200_ctx();

@@ -117,15 +117,12 @@ bml_matrix_ellblock_t *eb_alloc_blocks(bml_matrix_precision_t prec, int NB, int 
     bool ok = A->bsize && A->indexb && A->nnzb && A->ptr_value && A->h_pool;
     if (ok)
     {
-        cudaError_t e1 = cudaMallocAsync(&A->d_pool, eb_pool_elems(A) * sz, c->stream);
-        cudaError_t e2 = cudaMallocAsync(reinterpret_cast<void **>(&A->d_indexb), sizeof(int) * (size_t) NB * MB, c->stream);
-        cudaError_t e3 = cudaMallocAsync(reinterpret_cast<void **>(&A->d_nnzb), sizeof(int) * NB, c->stream);
-        cudaError_t e4 = cudaMallocAsync(reinterpret_cast<void **>(&A->d_bsize), sizeof(int) * NB, c->stream);
-        cudaError_t e5 = cudaMallocAsync(reinterpret_cast<void **>(&A->d_boff), sizeof(int) * (NB + 1), c->stream);
-        if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess || e4 != cudaSuccess ||
-            e5 != cudaSuccess)
+        if (!b200_device_alloc(&A->d_pool, eb_pool_elems(A) * sz) ||
+            !b200_device_alloc(reinterpret_cast<void **>(&A->d_indexb), sizeof(int) * (size_t) NB * MB) ||
+            !b200_device_alloc(reinterpret_cast<void **>(&A->d_nnzb), sizeof(int) * NB) ||
+            !b200_device_alloc(reinterpret_cast<void **>(&A->d_bsize), sizeof(int) * NB) ||
+            !b200_device_alloc(reinterpret_cast<void **>(&A->d_boff), sizeof(int) * (NB + 1)))
         {
-            cudaGetLastError();
             b200_set_error(BML_B200_ERR_ALLOC, "ELLBLOCK device arrays NB=%d MB=%d maxbs=%d", NB, MB, maxbs);
             ok = false;
         }
@@ -2576,14 +2573,16 @@ bml_matrix_ellblock_t *eb_from_ellpack(bml_matrix_ellpack_t *E, bml_matrix_preci
         b200_set_error(BML_B200_ERR_UNSUPPORTED, "convert: NB=%d block columns", NB);
         return nullptr;
     }
-    unsigned char *scr = static_cast<unsigned char *>(b200_scratch((size_t) (N + NB + 1) * sizeof(int) + 256));
     int *f = eb_flags(c);
-    if (!scr || !f)
-        return nullptr;
-    int *dcolblk = reinterpret_cast<int *>(scr);
-    int *dboff = dcolblk + N;
-    if (!CUDA_OK(cudaMemcpyAsync(dcolblk, colblk.data(), sizeof(int) * N, cudaMemcpyHostToDevice, c->stream)) ||
-        !CUDA_OK(cudaMemcpyAsync(dboff, boff.data(), sizeof(int) * (NB + 1), cudaMemcpyHostToDevice, c->stream)))
+    int *dcolblk = nullptr, *dboff = nullptr;
+    auto upload = [&]() {
+        dcolblk = static_cast<int *>(b200_scratch((size_t) (N + NB + 1) * sizeof(int) + 256));
+        dboff = dcolblk + N;
+        return dcolblk &&
+               CUDA_OK(cudaMemcpyAsync(dcolblk, colblk.data(), sizeof(int) * N, cudaMemcpyHostToDevice, c->stream)) &&
+               CUDA_OK(cudaMemcpyAsync(dboff, boff.data(), sizeof(int) * (NB + 1), cudaMemcpyHostToDevice, c->stream));
+    };
+    if (!f || !upload())
         return nullptr;
     for (auto kern : {conv_count_kernel<double>})
         if (!CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)))
@@ -2606,6 +2605,11 @@ bml_matrix_ellblock_t *eb_from_ellpack(bml_matrix_ellpack_t *E, bml_matrix_preci
     bml_matrix_ellblock_t *B = eb_alloc_blocks(prec, NB, MB, M, bsize, mode);
     if (!B)
         return nullptr;
+    if (!c->scratch && !upload()) // the arena gave way to B
+    {
+        eb_free(B);
+        return nullptr;
+    }
     bool ok;
     const bool din = E->matrix_precision == double_real, dout = prec == double_real;
     auto set_smem = [&](auto kern) {
@@ -2639,14 +2643,17 @@ bml_matrix_ellpack_t *ell_from_ellblock(bml_matrix_ellblock_t *A, bml_matrix_pre
     for (int ib = 0, r = 0; ib < A->NB; ++ib)
         for (int k = 0; k < A->bsize[ib]; ++k)
             rowblk[r++] = ib;
+    bml_matrix_ellpack_t *E = ell_alloc(prec, N, M, mode, true);
+    if (!E)
+        return nullptr;
     int *drowblk = static_cast<int *>(b200_scratch(sizeof(int) * (size_t) N + 256));
     int *f = eb_flags(c);
     if (!drowblk || !f ||
         !CUDA_OK(cudaMemcpyAsync(drowblk, rowblk.data(), sizeof(int) * N, cudaMemcpyHostToDevice, c->stream)))
+    {
+        ell_free(E);
         return nullptr;
-    bml_matrix_ellpack_t *E = ell_alloc(prec, N, M, mode, true);
-    if (!E)
-        return nullptr;
+    }
     const int grid = max(1, min(b200_ceil_div(N, 8), c->sm_count * 16));
     const bool din = A->matrix_precision == double_real, dout = prec == double_real;
     auto launch = [&](int count) {

@@ -112,6 +112,10 @@ void *b200_scratch(size_t bytes);
 // The same without a status when the memory is not there, for forms that have
 // another to leave the call to (the arena is empty then).
 void *b200_scratch_try(size_t bytes);
+// Stream-ordered device memory that outlives the call.  Where it is short the
+// scratch arena is given back first, so pointers into it from before are void
+// then (c->scratch is null).  False, with no status set, on failure.
+bool b200_device_alloc(void **p, size_t bytes);
 // Synchronise the library stream; false (error recorded) on failure.
 bool b200_sync();
 

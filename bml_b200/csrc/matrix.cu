@@ -129,12 +129,10 @@ bml_matrix_ellpack_t *ell_alloc(bml_matrix_precision_t prec, int N, int M,
     if (ok)
     {
         const size_t elems = (size_t) N * A->ld;
-        cudaError_t e1 = cudaMallocAsync(&A->d_value, elems * sz, c->stream);
-        cudaError_t e2 = cudaMallocAsync(reinterpret_cast<void **>(&A->d_index), elems * sizeof(int), c->stream);
-        cudaError_t e3 = cudaMallocAsync(reinterpret_cast<void **>(&A->d_nnz), (size_t) N * sizeof(int), c->stream);
-        if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess)
+        if (!b200_device_alloc(&A->d_value, elems * sz) ||
+            !b200_device_alloc(reinterpret_cast<void **>(&A->d_index), elems * sizeof(int)) ||
+            !b200_device_alloc(reinterpret_cast<void **>(&A->d_nnz), (size_t) N * sizeof(int)))
         {
-            cudaGetLastError();
             b200_set_error(BML_B200_ERR_ALLOC, "device arrays for N=%d M=%d (%.1f MB)", N, M,
                            (elems * (sz + 4) + N * 4.0) / 1e6);
             ok = false;
