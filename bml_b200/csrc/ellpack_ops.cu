@@ -9,6 +9,7 @@
 #include <climits>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 using namespace b200;
 
@@ -91,215 +92,37 @@ inline int rows_grid(B200Context *c, int N, int rows_per_block)
 // Reference: ellpack/bml_add_ellpack_typed.c:50-216.  Per row: A's columns in
 // A's order (x = 0 + alpha*a), then B's (x += beta*b; new columns appended in
 // B's order); kept when |x| > threshold.  A term is skipped entirely when its
-// scalar is 0.  One team of W warps per row; A's row is staged in shared
-// memory with a hash from column to position, so the row is rewritten in
-// place only after it has been read.
-// Shared memory per team: keys[TS] pos[TS] xa[ldA](T) ka[ldA] newpos[ldB] cnt.
+// scalar is 0.
+//
+// A CTA of W warps per row.  A table of TS 16-bit entries holds the place of
+// a column in B's row (plus one).  Where the row of B spans fewer than TS
+// columns a column's entry is table[column % TS], so finding B's entry of a
+// column of A is one 2-byte read; a wider row is entered by a hash of the
+// column, with linear probing, and a find compares the column that the entry
+// stands for.  Neither row is staged in shared memory: entries wait in
+// registers (MAP_U a thread) for the block's prefix.  A's part is rewritten in
+// place: a round's entries are read before they are written, at or before
+// their own places.
+//
+// Bound by HBM on long rows, by a row's chain of loads on short ones, so rows
+// of at most ADD_NARROW entries have a warp and a small table each, and 28 of
+// them run on an SM.  us, both rows staged in shared memory and hashed | so
+// (2x - y, FP64): 40^3 rows of 925 and 1221 970 | 585, 64^3 rows of 257 and 400
+// 2970 | 1483, of 925 and 1221 10224 | 3270, 64000 scattered rows of 100 425 |
+// 103, 512 rows of 33 23 | 21.  Two warps a row: 178 for the 64000 rows, 1423
+// for the 64^3 ones.
 // ---------------------------------------------------------------------------
-constexpr int ADD_U = 8; // entries per thread in flight in the add's loads
-
-template <typename T, int W>
-__global__ void __launch_bounds__(W * 32) add_kernel(T *Av, int *Ai, int *An, int lda, int Ma,
-                                                   const T *Bv, const int *Bi, const int *Bn,
-                                                   int ldb, int N, double alpha, double beta,
-                                                   double thr, int logts, const unsigned char *todo, int *overflow)
-{
-    constexpr int NT = W * 32;
-    extern __shared__ __align__(128) unsigned char smem[];
-    const int TS = 1 << logts;
-    const unsigned mask = TS - 1;
-    T *xa = reinterpret_cast<T *>(smem);    // A's entries, then x = alpha*a (+ beta*b)
-    T *newx = xa + lda;                      // B's new entries: x = beta*b, by warp segment
-    int *ka = reinterpret_cast<int *>(newx + ldb);
-    int *keys = ka + lda;
-    int *pos = keys + TS;
-    int *newk = pos + TS;
-    int *cnt = newk + ldb; // [W]
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
-    const T thr_t = (T) thr;
-    const bool use_a = alpha > 0.0 || alpha < 0.0;
-    const bool use_b = beta > 0.0 || beta < 0.0;
-
-    for (int i = blockIdx.x; i < N; i += gridDim.x)
-    {
-        if (todo && !todo[i])
-            continue;
-        for (int s = tid; s < TS; s += NT)
-            keys[s] = B200_EMPTY_KEY;
-        __syncthreads();
-        const int na = use_a ? An[i] : 0;
-        const int nb = use_b ? Bn[i] : 0;
-        // A's row into shared memory: x = 0 + alpha*a, column -> position
-        // (ADD_U entries per thread loaded before any is stored)
-        for (int p0 = 0; p0 < na; p0 += NT * ADD_U)
-        {
-            int kk[ADD_U];
-            T aa[ADD_U];
-#pragma unroll
-            for (int u = 0; u < ADD_U; ++u)
-            {
-                const int p = p0 + u * NT + tid;
-                kk[u] = p < na ? Ai[(size_t) i * lda + p] : 0;
-                aa[u] = p < na ? Av[(size_t) i * lda + p] : T(0);
-            }
-#pragma unroll
-            for (int u = 0; u < ADD_U; ++u)
-            {
-                const int p = p0 + u * NT + tid;
-                if (p < na)
-                {
-                    ka[p] = kk[u];
-                    xa[p] = axpy_d(T(0), alpha, aa[u]);
-                    hash_put(keys, pos, mask, kk[u], p);
-                }
-            }
-        }
-        __syncthreads();
-        // B's row, one contiguous segment per warp: a column of A's row takes
-        // x + beta*b (one writer: B's columns are distinct); a new column is
-        // listed at its segment's start, in B order
-        const int seg = b200_round_up(b200_ceil_div(max(nb, 1), W), 32);
-        const int s0 = min(warp * seg, nb), s1 = min(s0 + seg, nb);
-        int local = 0;
-        for (int q0 = s0; q0 < s1; q0 += 32 * ADD_U)
-        {
-            int kk[ADD_U];
-            T bb[ADD_U];
-#pragma unroll
-            for (int u = 0; u < ADD_U; ++u)
-            {
-                const int q = q0 + u * 32 + lane;
-                kk[u] = q < s1 ? Bi[(size_t) i * ldb + q] : 0;
-                bb[u] = q < s1 ? Bv[(size_t) i * ldb + q] : T(0);
-            }
-#pragma unroll
-            for (int u = 0; u < ADD_U; ++u)
-            {
-                const int q = q0 + u * 32 + lane;
-                bool isnew = false;
-                if (q < s1)
-                {
-                    const int p = hash_get(keys, pos, mask, kk[u]);
-                    if (p >= 0)
-                        xa[p] = axpy_d(xa[p], beta, bb[u]);
-                    else
-                        isnew = true;
-                }
-                const unsigned bal = __ballot_sync(FULL, isnew);
-                if (isnew)
-                {
-                    const int at = s0 + local + __popc(bal & lanemask_lt());
-                    newk[at] = kk[u];
-                    newx[at] = axpy_d(T(0), beta, bb[u]);
-                }
-                local += __popc(bal);
-            }
-        }
-        if (lane == 0)
-            cnt[warp] = local;
-        __syncthreads();
-        int npre[W];
-        int nnew = 0;
-#pragma unroll
-        for (int w = 0; w < W; ++w)
-        {
-            npre[w] = nnew;
-            nnew += cnt[w];
-        }
-        // the sum's entries: A's, then the new ones; e -> (column, value)
-        auto entry = [&](int e, int &k, T &x) {
-            if (e < na)
-            {
-                k = ka[e];
-                x = xa[e];
-                return;
-            }
-            const int r = e - na;
-            int w = 0, base = 0;
-#pragma unroll
-            for (int v = 1; v < W; ++v)
-                if (r >= npre[v])
-                {
-                    w = v;
-                    base = npre[v];
-                }
-            const int at = w * seg + (r - base);
-            k = newk[at];
-            x = newx[at];
-        };
-        const int total = na + nnew;
-        const int seg3 = b200_round_up(b200_ceil_div(max(total, 1), W), 32);
-        const int e0 = min(warp * seg3, total), e1 = min(e0 + seg3, total);
-        int kept = 0;
-        for (int c0 = e0; c0 < e1; c0 += 32)
-        {
-            const int e = c0 + lane;
-            int k = 0;
-            T x = T(0);
-            if (e < e1)
-                entry(e, k, x);
-            kept += __popc(__ballot_sync(FULL, e < e1 && fabs(x) > thr_t));
-        }
-        __syncthreads(); // every thread has read cnt
-        if (lane == 0)
-            cnt[warp] = kept;
-        __syncthreads();
-        int ll = 0, total_kept = 0;
-#pragma unroll
-        for (int w = 0; w < W; ++w)
-        {
-            ll += w < warp ? cnt[w] : 0;
-            total_kept += cnt[w];
-        }
-        for (int c0 = e0; c0 < e1; c0 += 32)
-        {
-            const int e = c0 + lane;
-            int k = 0;
-            T x = T(0);
-            if (e < e1)
-                entry(e, k, x);
-            const bool keep = e < e1 && fabs(x) > thr_t;
-            const unsigned bal = __ballot_sync(FULL, keep);
-            const int p = ll + __popc(bal & lanemask_lt());
-            if (keep && p < Ma)
-            {
-                Av[(size_t) i * lda + p] = x;
-                Ai[(size_t) i * lda + p] = k;
-            }
-            ll += __popc(bal);
-        }
-        if (tid == 0)
-        {
-            An[i] = min(total_kept, Ma);
-            if (total_kept > Ma)
-                atomicExch(overflow, 1);
-        }
-        __syncthreads(); // before the next row reuses the shared arrays
-    }
-}
-
-// The same sum through a direct table, for rows whose columns of B span less
-// than MAP_COLS: map[col % MAP_COLS] is the place of the column in B's row
-// (plus one), so finding B's entry of a column of A is one 2-byte read instead
-// of a hash probe, and neither row is staged in shared memory: entries wait in
-// registers (MAP_U a thread) for the block's prefix.  64 KB a CTA whatever M
-// is (the hash form takes 20 M + 16 times the power of two above M bytes: at
-// M = 2048 two CTAs per SM and 1.33 ms for the update of the 40^3 iterate).
-// Rows it cannot hold are left untouched and marked in `todo` for the hash
-// form, *left set.  A's part is rewritten in place: a round's entries are
-// read before they are written, at or before their own places.
-constexpr int MAP_COLS = 32768;
 constexpr int MAP_U = 4; // entries per thread of a round
+constexpr int ADD_NARROW = 512, ADD_W = 1;
 
-template <typename T, int W>
-__global__ void __launch_bounds__(W * 32, 3) add_map_kernel(T *Av, int *Ai, int *An, int lda, int Ma, const T *Bv,
-                                                       const int *Bi, const int *Bn, int ldb, int N, double alpha,
-                                                       double beta, double thr, unsigned char *todo, int *left,
-                                                       int *overflow)
+template <typename T, int W, int TS, int MINB>
+__global__ void __launch_bounds__(W * 32, MINB) add_map_kernel(T *Av, int *Ai, int *An, int lda, int Ma, const T *Bv,
+                                                               const int *Bi, const int *Bn, int ldb, int N,
+                                                               double alpha, double beta, double thr, int *overflow)
 {
     constexpr int NT = W * 32;
     constexpr unsigned short USED = 0x8000u;
-    extern __shared__ __align__(16) unsigned char smem[];
+    extern __shared__ __align__(128) unsigned char smem[];
     unsigned short *map = reinterpret_cast<unsigned short *>(smem);
     __shared__ int cnt[2][W];
     __shared__ int lo, hi;
@@ -307,16 +130,18 @@ __global__ void __launch_bounds__(W * 32, 3) add_map_kernel(T *Av, int *Ai, int 
     const T thr_t = (T) thr;
     const bool use_a = alpha > 0.0 || alpha < 0.0;
     const bool use_b = beta > 0.0 || beta < 0.0;
-    for (int s = tid; s < MAP_COLS / 8; s += NT)
+    for (int s = tid; s < TS / 8; s += NT)
         reinterpret_cast<uint4 *>(smem)[s] = make_uint4(0u, 0u, 0u, 0u);
-    auto claim = [&](int at) { // marks the place used; true for the first to do so
+    // (the high bits: columns a multiple of TS apart, a lattice's planes, differ in those alone)
+    auto slot = [](int k) { return (unsigned) k * 2654435761u / (unsigned) ((1ull << 32) / TS); };
+    auto claim = [&](unsigned at) { // marks the place used; true for the first to do so
         const unsigned bit = (unsigned) USED << 16 * (at & 1);
         return !(atomicOr(reinterpret_cast<unsigned *>(smem) + (at >> 1), bit) & bit);
     };
     for (int i = blockIdx.x; i < N; i += gridDim.x)
     {
         const int na = use_a ? An[i] : 0;
-        const int nb = use_b ? Bn[i] : 0;
+        const int nb = use_b ? min(Bn[i], TS - 1) : 0; // M is smaller still
         if (tid == 0)
         {
             lo = INT_MAX;
@@ -337,25 +162,24 @@ __global__ void __launch_bounds__(W * 32, 3) add_map_kernel(T *Av, int *Ai, int 
             xb[u] = p < nb ? __ldg(Bv + rb + p) : T(0);
         }
         __syncthreads(); // also: the map is clear, and cnt free
-        int mn = INT_MAX, mx = -1;
+        // f(column, place) for every entry of B
+        auto each_b = [&](auto f) {
 #pragma unroll
-        for (int u = 0; u < MAP_U; ++u)
-        {
-            const int p = (warp * MAP_U + u) * 32 + lane;
-            if (p < nb)
+            for (int u = 0; u < MAP_U; ++u)
             {
-                mn = min(mn, kb[u]);
-                mx = max(mx, kb[u]);
-                map[kb[u] & (MAP_COLS - 1)] = (unsigned short) (p + 1);
+                const int p = (warp * MAP_U + u) * 32 + lane;
+                if (p < nb)
+                    f(kb[u], p);
             }
-        }
-        for (int q = NT * MAP_U + tid; q < nb; q += NT)
-        {
-            const int k = __ldg(Bi + rb + q);
+            for (int q = NT * MAP_U + tid; q < nb; q += NT)
+                f(__ldg(Bi + rb + q), q);
+        };
+        int mn = INT_MAX, mx = -1;
+        each_b([&](int k, int p) {
             mn = min(mn, k);
             mx = max(mx, k);
-            map[k & (MAP_COLS - 1)] = (unsigned short) (q + 1);
-        }
+            map[k & (TS - 1)] = (unsigned short) (p + 1);
+        });
         for (int o = 16; o; o >>= 1)
         {
             mn = min(mn, __shfl_xor_sync(FULL, mn, o));
@@ -368,102 +192,132 @@ __global__ void __launch_bounds__(W * 32, 3) add_map_kernel(T *Av, int *Ai, int 
         }
         __syncthreads();
         const int blo = lo, bhi = hi;
-        if (bhi - blo >= MAP_COLS || nb >= USED)
+        const bool wide = bhi - blo >= TS;
+        if (wide)
         {
-            for (int q = tid; q < nb; q += NT)
-                map[__ldg(Bi + rb + q) & (MAP_COLS - 1)] = 0;
-            if (tid == 0)
-            {
-                todo[i] = 1;
-                *reinterpret_cast<volatile int *>(left) = 1;
-            }
+            each_b([&](int k, int) { map[k & (TS - 1)] = 0; });
             __syncthreads();
-            continue;
+            each_b([&](int k, int p) {
+                unsigned at = slot(k);
+                while (atomicCAS(&map[at], (unsigned short) 0, (unsigned short) (p + 1)) != 0)
+                    at = (at + 1) & (TS - 1);
+            });
+            __syncthreads();
         }
         int ll = 0; // kept so far (uniform)
-        int flip = 0;
-        // A's entries, then B's new ones, in rounds of NT * MAP_U; thread t of warp w holds entries
-        // w * 32 * MAP_U + u * 32 + lane of the round
-        auto emit = [&](const int(&ek)[MAP_U], const T(&ex)[MAP_U]) {
-            int c = 0;
-#pragma unroll
-            for (int u = 0; u < MAP_U; ++u)
-                c += __popc(keep[u]);
-            if (lane == 0)
-                cnt[flip][warp] = c;
-            __syncthreads();
-            int at = ll, all = 0;
-#pragma unroll
-            for (int w = 0; w < W; ++w)
-            {
-                const int cw = cnt[flip][w];
-                at += w < warp ? cw : 0;
-                all += cw;
-            }
-#pragma unroll
-            for (int u = 0; u < MAP_U; ++u)
-            {
-                const int p = at + __popc(keep[u] & lanemask_lt());
-                if ((keep[u] >> lane & 1u) && p < Ma)
+        // A's entries and then B's; a version each for narrow and wide rows (one that asks for every entry: 640 us
+        // against 585 for the update of the 40^3 iterate)
+        auto passes = [&](auto spans) {
+            constexpr bool wide = decltype(spans)::value;
+            // entry of a column in the map and its place, or 0 (fewer than TS entries are in it, so an empty one ends
+            // every search)
+            auto find = [&](int k, unsigned &at) -> unsigned short {
+                at = k & (TS - 1);
+                if (!wide)
+                    return k >= blo && k <= bhi ? map[at] : 0;
+                for (at = slot(k);; at = (at + 1) & (TS - 1))
                 {
-                    Av[ra + p] = ex[u];
-                    Ai[ra + p] = ek[u];
+                    const unsigned short m = map[at];
+                    if (!m || __ldg(Bi + rb + (m & (USED - 1)) - 1) == k)
+                        return m;
                 }
-                at += __popc(keep[u]);
-            }
-            ll += all;
-            flip ^= 1;
-        };
-        for (int p0 = 0; p0 < na; p0 += NT * MAP_U)
-        {
-            if (p0 > 0)
+            };
+            // place of B's entry p, of column k
+            auto own = [&](int k, int p) {
+                unsigned at = wide ? slot(k) : k & (TS - 1);
+                while (wide && (map[at] & (USED - 1)) != p + 1)
+                    at = (at + 1) & (TS - 1);
+                return at;
+            };
+            int flip = 0;
+            // A's entries, then B's new ones, in rounds of NT * MAP_U; thread t of warp w holds entries
+            // w * 32 * MAP_U + u * 32 + lane of the round
+            auto emit = [&](const int(&ek)[MAP_U], const T(&ex)[MAP_U]) {
+                int c = 0;
+#pragma unroll
+                for (int u = 0; u < MAP_U; ++u)
+                    c += __popc(keep[u]);
+                if (lane == 0)
+                    cnt[flip][warp] = c;
+                __syncthreads();
+                int at = ll, all = 0;
+#pragma unroll
+                for (int w = 0; w < W; ++w)
+                {
+                    const int cw = cnt[flip][w];
+                    at += w < warp ? cw : 0;
+                    all += cw;
+                }
 #pragma unroll
                 for (int u = 0; u < MAP_U; ++u)
                 {
-                    const int p = p0 + (warp * MAP_U + u) * 32 + lane;
-                    kk[u] = p < na ? Ai[ra + p] : -1;
-                    xx[u] = p < na ? Av[ra + p] : T(0);
+                    const int p = at + __popc(keep[u] & lanemask_lt());
+                    if ((keep[u] >> lane & 1u) && p < Ma)
+                    {
+                        Av[ra + p] = ex[u];
+                        Ai[ra + p] = ek[u];
+                    }
+                    at += __popc(keep[u]);
                 }
-#pragma unroll
-            for (int u = 0; u < MAP_U; ++u)
+                ll += all;
+                flip ^= 1;
+            };
+            for (int p0 = 0; p0 < na; p0 += NT * MAP_U)
             {
-                xx[u] = axpy_d(T(0), alpha, xx[u]);
-                if (kk[u] >= blo && kk[u] <= bhi)
+                if (p0 > 0)
+#pragma unroll
+                    for (int u = 0; u < MAP_U; ++u)
+                    {
+                        const int p = p0 + (warp * MAP_U + u) * 32 + lane;
+                        kk[u] = p < na ? Ai[ra + p] : -1;
+                        xx[u] = p < na ? Av[ra + p] : T(0);
+                    }
+#pragma unroll
+                for (int u = 0; u < MAP_U; ++u)
                 {
+                    const bool have = p0 + (warp * MAP_U + u) * 32 + lane < na;
+                    xx[u] = axpy_d(T(0), alpha, xx[u]);
                     // of several entries of A in one column (set_element appends to short rows), one takes B's
-                    const unsigned short m = map[kk[u] & (MAP_COLS - 1)];
-                    if (m && !(m & USED) && claim(kk[u] & (MAP_COLS - 1)))
+                    unsigned at = 0;
+                    const unsigned short m = have ? find(kk[u], at) : 0;
+                    if (m && !(m & USED) && claim(at))
                         xx[u] = axpy_d(xx[u], beta, __ldg(Bv + rb + m - 1));
+                    keep[u] = __ballot_sync(FULL, have && fabs(xx[u]) > thr_t);
                 }
-                keep[u] = __ballot_sync(FULL, p0 + (warp * MAP_U + u) * 32 + lane < na && fabs(xx[u]) > thr_t);
+                emit(kk, xx);
             }
-            emit(kk, xx);
-        }
-        __syncthreads(); // A's marks in the map
-        for (int p0 = 0; p0 < nb; p0 += NT * MAP_U)
-        {
-            if (p0 > 0)
+            __syncthreads(); // A's marks in the map
+            for (int p0 = 0; p0 < nb; p0 += NT * MAP_U)
+            {
+                if (p0 > 0)
+#pragma unroll
+                    for (int u = 0; u < MAP_U; ++u)
+                    {
+                        const int p = p0 + (warp * MAP_U + u) * 32 + lane;
+                        kb[u] = p < nb ? __ldg(Bi + rb + p) : -1;
+                        xb[u] = p < nb ? __ldg(Bv + rb + p) : T(0);
+                    }
 #pragma unroll
                 for (int u = 0; u < MAP_U; ++u)
                 {
+                    bool fresh = false;
                     const int p = p0 + (warp * MAP_U + u) * 32 + lane;
-                    kb[u] = p < nb ? __ldg(Bi + rb + p) : -1;
-                    xb[u] = p < nb ? __ldg(Bv + rb + p) : T(0);
+                    if (p < nb)
+                    {
+                        const unsigned at = own(kb[u], p);
+                        fresh = !(map[at] & USED);
+                        map[at] = 0;
+                        xb[u] = axpy_d(T(0), beta, xb[u]);
+                    }
+                    keep[u] = __ballot_sync(FULL, fresh && fabs(xb[u]) > thr_t);
                 }
-#pragma unroll
-            for (int u = 0; u < MAP_U; ++u)
-            {
-                bool fresh = false;
-                if (p0 + (warp * MAP_U + u) * 32 + lane < nb)
-                {
-                    fresh = !(map[kb[u] & (MAP_COLS - 1)] & USED);
-                    map[kb[u] & (MAP_COLS - 1)] = 0;
-                    xb[u] = axpy_d(T(0), beta, xb[u]);
-                }
-                keep[u] = __ballot_sync(FULL, fresh && fabs(xb[u]) > thr_t);
+                emit(kb, xb);
             }
-            emit(kb, xb);
-        }
+        };
+        if (wide)
+            passes(std::true_type());
+        else
+            passes(std::false_type());
         if (tid == 0)
         {
             An[i] = min(ll, Ma);
@@ -1018,64 +872,49 @@ bool check_pair(const bml_matrix_ellpack_t *A, const bml_matrix_ellpack_t *B, co
     return true;
 }
 
-constexpr int ADD_W = 8; // warps of an add CTA
-
-// xa[lda] newx[ldb] (matrix precision) | ka[lda] keys[TS] pos[TS] newk[ldb] cnt[8]
-template <typename T> size_t add_hash_smem(const bml_matrix_ellpack_t *A, const bml_matrix_ellpack_t *B, int logts)
+// Bytes of shared memory that both rows, a hash of A's and a list take at the
+// widest: rows beyond the device's limit go through a dense image instead
+// (M above about 4200 where A and B are of one M, in FP64).
+size_t add_row_bytes(const bml_matrix_ellpack_t *A, const bml_matrix_ellpack_t *B)
 {
-    return (size_t) (A->ld + B->ld) * (sizeof(T) + 4) + ((size_t) 2 << logts) * 4 + ADD_W * 4 + 64;
+    int logts = 5;
+    while ((1 << logts) < 2 * A->M)
+        ++logts;
+    return (size_t) (A->ld + B->ld) * (prec_size(A->matrix_precision) + 4) + ((size_t) 2 << logts) * 4 + 96;
 }
 
-template <typename T>
-bool add_typed(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, double alpha, double beta, double threshold)
+template <typename T, int W, int TS, int MINB>
+bool add_launch(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, double alpha, double beta, double threshold)
 {
     B200Context *c = b200_ctx();
-    // flags: rows left to the hash form, overflow
-    int *flags = reinterpret_cast<int *>(static_cast<unsigned char *>(c->d_small) + 2048);
-    int *pin = reinterpret_cast<int *>(static_cast<unsigned char *>(c->pinned) + 2048);
-    T *av = static_cast<T *>(A->d_value);
-    const T *bv = static_cast<const T *>(B->d_value);
-    unsigned char *todo = static_cast<unsigned char *>(b200_scratch(A->N));
-    if (!todo || !CUDA_OK(cudaMemsetAsync(todo, 0, A->N, c->stream)) ||
-        !CUDA_OK(cudaMemsetAsync(flags, 0, 2 * sizeof(int), c->stream)))
+    int *ovf = zeroed_flag(c);
+    const size_t smem = TS * sizeof(unsigned short);
+    auto k = add_map_kernel<T, W, TS, MINB>;
+    if (!ovf || !CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)))
         return false;
-    const size_t smemM = MAP_COLS * sizeof(unsigned short);
-    auto km = add_map_kernel<T, ADD_W>;
-    if (!CUDA_OK(cudaFuncSetAttribute(km, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smemM)))
-        return false;
-    km<<<min(A->N, c->sm_count * 3), 32 * ADD_W, smemM, c->stream>>>(av, A->d_index, A->d_nnz, A->ld, A->M, bv,
-                                                                     B->d_index, B->d_nnz, B->ld, A->N, alpha, beta,
-                                                                     threshold, todo, flags, flags + 1);
+    k<<<min(A->N, c->sm_count * MINB), 32 * W, smem, c->stream>>>(
+        static_cast<T *>(A->d_value), A->d_index, A->d_nnz, A->ld, A->M, static_cast<const T *>(B->d_value),
+        B->d_index, B->d_nnz, B->ld, A->N, alpha, beta, threshold, ovf);
     if (!LAUNCH_OK("add_map_kernel"))
         return false;
     ell_mark_device(A);
-    if (!CUDA_OK(cudaMemcpyAsync(pin, flags, 2 * sizeof(int), cudaMemcpyDeviceToHost, c->stream)) || !b200_sync())
+    int hov = 0;
+    if (!read_flag(c, ovf, &hov))
         return false;
-    if (pin[0])
-    {
-        // the hash holds A's row at most half full
-        int logts = 5;
-        while ((1 << logts) < 2 * A->M)
-            ++logts;
-        const size_t smem = add_hash_smem<T>(A, B, logts);
-        auto k = add_kernel<T, ADD_W>;
-        if (!CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)))
-            return false;
-        int occ = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 32 * ADD_W, smem);
-        k<<<min(A->N, c->sm_count * (occ > 0 ? occ : 1)), 32 * ADD_W, smem, c->stream>>>(
-            av, A->d_index, A->d_nnz, A->ld, A->M, bv, B->d_index, B->d_nnz, B->ld, A->N, alpha, beta, threshold,
-            logts, todo, flags + 1);
-        if (!LAUNCH_OK("add_kernel") ||
-            !CUDA_OK(cudaMemcpyAsync(pin, flags, 2 * sizeof(int), cudaMemcpyDeviceToHost, c->stream)) || !b200_sync())
-            return false;
-    }
-    if (pin[1])
+    if (hov)
     {
         b200_set_error(BML_B200_ERR_ROW_OVERFLOW, "add: a row of the sum has more than M=%d entries", A->M);
         return false;
     }
     return true;
+}
+
+template <typename T>
+bool add_typed(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, double alpha, double beta, double threshold)
+{
+    if (max(A->M, B->M) <= ADD_NARROW)
+        return add_launch<T, ADD_W, 2048, 28>(A, B, alpha, beta, threshold);
+    return add_launch<T, 8, 32768, 3>(A, B, alpha, beta, threshold);
 }
 
 } // namespace
@@ -1098,14 +937,9 @@ bool ell_add(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, double alpha, dou
         ell_free(T0);
         return ok;
     }
-    int logts = 5;
-    while ((1 << logts) < 2 * A->M)
-        ++logts;
-    const size_t smem =
-        A->matrix_precision == double_real ? add_hash_smem<double>(A, B, logts) : add_hash_smem<float>(A, B, logts);
-    if (smem > c->smem_optin)
+    if (add_row_bytes(A, B) > c->smem_optin)
     {
-        // rows too wide for the hash: through a dense image of the row sums
+        // through a dense image of the row sums
         // (unordered form; rows come out in ascending column order)
         if (!ell_x2_exact() && threshold >= 0.0)
         {
@@ -1324,7 +1158,8 @@ bool ell_trace_mult(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, double *tr
             if (!CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)))
                 return false;
             kern<<<grid, 32 * warps_per_block, smem, c->stream>>>(av, A->d_index, A->d_nnz, A->ld, bv, B->d_index,
-                                                                  B->d_nnz, B->ld, A->N, logts, done, need, beyond, call, part);
+                                                                  B->d_nnz, B->ld, A->N, logts, done, need, beyond,
+                                                                  call, part);
             return LAUNCH_OK("trace_mult_kernel");
         };
         if (A->matrix_precision == double_real

@@ -2,8 +2,9 @@
 A's entries in A's order as alpha*a (+ beta*b), then B's new columns in B's
 order as beta*b, each step rounded as the reference rounds it
 (ellpack/bml_add_ellpack_typed.c:50-216), kept when |x| > threshold.  Rows at
-the edges of the table (32768 columns of B), wider ones beside them (which the
-hash form adds), rows longer than one round of a CTA (2048 entries), empty
+the edges of the tables (2048 columns of B where M is at most 512, else 32768),
+wider ones beside them (found by a hash), rows longer than one round of a CTA
+(256 and 1024 entries), columns that are multiples of a table apart, empty
 rows, zero scalars; and tr(A B^T) of matrices large enough to be sized by their
 rows."""
 import numpy as np
@@ -48,6 +49,7 @@ def _sum(a, b, alpha, beta, thr, dtype):
 @pytest.mark.parametrize("ncols,M,wide_a,wide_b,span", [
     (40, 40, (0, 1, 7, 40), (40, 0, 3), (40,)),
     (70000, 600, (300, 0, 31), (0, 290, 17, 1), (32768, 32769, 500, 70000)),
+    (70000, 512, (250, 0, 31, 257), (0, 240, 17, 255), (2048, 2049, 500, 70000)),
     (9000, 4096, (2048, 2049, 2500, 0), (1500, 0, 1590, 2100, 1), (9000, 2600)),
 ])
 def test_add_rows(ncols, M, wide_a, wide_b, span, alpha, beta, thr, dtype):
@@ -59,6 +61,9 @@ def test_add_rows(ncols, M, wide_a, wide_b, span, alpha, beta, thr, dtype):
         b[2][i] = min(b[2][i], M - a[2][i]) if ncols > M else b[2][i]
     if dtype == np.float32:
         b[0][:, ::3] = -b[0][:, ::3]
+    if ncols > 2 ** 16:  # columns that are multiples of the table apart
+        a[1][1, :8] = b[1][1, :8] = np.arange(8) * 8192
+        a[2][1], b[2][1] = 8, 8
     # half of B's columns where A has them too
     for i in range(0, N, 2):
         n = min(a[2][i], b[2][i]) // 2
