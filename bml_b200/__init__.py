@@ -129,6 +129,8 @@ _PROTOS = {
     "bml_b200_set_kernel_timing": (_i, [_i]),
     "bml_b200_set_dense_tier": (_i, [_i]),
     "bml_b200_last_x2_dense": (_i, []),
+    "bml_b200_set_tiles": (_i, [_i]),
+    "bml_b200_last_product_form": (_i, []),
     "bml_b200_last_x2_kernel_ms": (_d, []),
     "bml_getNRanks": (_i, []),
     "bml_getMyRank": (_i, []),
@@ -262,6 +264,14 @@ def multiply_x2(X, X2, threshold):
     tr = (C.c_double * 2)()
     st = lib.bml_b200_multiply_x2(X.h, X2.h, threshold, tr)
     return st, (tr[0], tr[1])
+
+
+# Values of bml_b200_last_product_form.
+PRODUCT_FORMS = ("ordered", "sparse", "sparse_symmetric", "tiles", "tiles_symmetric", "tiles_masked", "dense")
+
+
+def product_form():
+    return PRODUCT_FORMS[lib.bml_b200_last_product_form()]
 
 
 # Multiply tiers in the order of bml_b200_last_tier_counts.

@@ -40,6 +40,17 @@
 // same kernel, the second operand packed as rows of its transpose, the blocks
 // those that hold an entry of the pattern.
 //
+// Which form.  The counts of both forms' products decide (TILE_COST,
+// general_pays).  A counting kernel makes them, and a sample of entries looks
+// for mirrors, so that an X that is not symmetric is mostly known before it is
+// packed; a small X is counted while it is packed, and the symmetry check tells
+// the host at its start what was counted, so that a form that does not apply
+// costs the fill kernel and not the rest (X^2 without symmetry, us, sparse form
+// alone | with a packing and a wait before it | so: 500 rows of 21 59 | 75 |
+// 61, 2000 rows of 21 87 | 108 | 92; symmetric but scattered, which the sparse
+// form has to check once more: 500 rows of 40 86 | 130 | 110, 4096 rows of 40 259
+// | 353 | 285).
+//
 // The general product (A B, and X^2 of an X that is not symmetric) packs the
 // second operand the same way, forms the blocks (G, H) with H on both sides of
 // G, and writes rows from them alone.  The columns that a row touches, which
@@ -49,14 +60,15 @@
 // Measured against the sparse form on one B200: X^2 of the 40^3 lattice's wide
 // iterate (rows of 825) 65.0 -> 21.1 ms, first X^2 of that lattice (rows of
 // 113) 6.3 -> 2.5 ms, FP32 on 26999 rows 2.07 -> 0.82 ms, a chain of 4096 rows
-// of 340 745 -> 132 us, of 512 rows of 33 71 -> 55 us; the adjoint of 3
-// iterations on the 16^3 lattice 32 -> 21 ms with the host's share.
+// of 340 745 -> 132 us, of 512 rows of 33 71 -> 55 us; the masked products of
+// the adjoint of 3 iterations on the 16^3 lattice 24.4 -> 3.7 ms.
 // At 40^3 the MMAs that have both tiles take 9.0 ms of the product kernel's 18,
 // those in a pair with only one about 2; the rest is the handling of a common
 // column (4.4 products on average there, 7.8 at 30^3).
 #include "device_util.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <climits>
 #include <cstring>
 #include <type_traits>
@@ -85,20 +97,19 @@ constexpr size_t TL_SMALL = 40960; // place in the context's small buffers
 // 3880 to 7360 / 3840, 0.64 2050 / 2110, 1.45 (2000 rows) 167 to 185 / 134,
 // 1.88 847 / 1770, 1.94 370 / 807, 5.3 140 / 475; lattices have 8 to 70).
 constexpr double TILE_COST = 1.5;
-// A general product's ten launches and two waits take about 150 us whatever
-// its size, so matrices of fewer rows stay with the sparse form (A*B on
-// lattices, tile form against sparse form in us: 1721 rows 176 / 105, 207 /
-// 150, 202 / 151 and 250 / 274 for 5, 20, 17 and 82 M products; 4089 rows 200
-// / 200 and 287 / 488 for 11 and 90 M; 7993 rows 264 / 303 and 479 / 710).
-constexpr int GENERAL_ROWS = 4096;
 constexpr long long LAZY_BYTES = 128 << 20; // most tile places of a matrix laid out without counting them
+
+// 0 never, 1 where the rules below take it for the faster form, 2 wherever it applies.
+int g_tiles = 1;
 
 struct TileFlags
 {
-    unsigned long long products; // sum over rows of width^2 (the sparse form's products, X symmetric)
-    unsigned long long tiles2;   // sum over tile rows of tiles^2 (tile products)
+    unsigned long long products; // the sparse form's products: sum over rows of width^2 (X symmetric), or over entries
+    unsigned long long stored;   // entries of X
+    unsigned long long tiles2;   // tile products: sum over tile rows of tiles^2, or over tiles
     unsigned long long pool;     // words of the packed result taken
-    int entries;                 // (group, J) entries of X
+    int entries;                 // (group, J) entries handed out
+    int counted;                 // those the counting kernels found
     int reach, reachB;           // largest |column - row|; of the second operand
     int bad;                     // a row length or column out of range
     int odd;                     // an entry not finite, or a row whose tiles are zero: not for this form
@@ -107,7 +118,8 @@ struct TileFlags
     int next;                    // work item counter
     int full;                    // the pool ran out
     int overflow, max_width;
-    int done;                    // CTAs of the row kernel that have finished
+    int skipped;                 // a group was not packed
+    int counters, done;          // CTAs of the counting and of the row kernel that have finished
     int blocks;                  // blocks of the masked product
     double trA, trC;
 };
@@ -124,13 +136,18 @@ struct TileArgs
     unsigned *ent;               // entry << 4 | mask of the tile rows present; its tiles at 4 entry + row
     unsigned short *entJ;        // tile column of an entry
     double *tiles;               // 64 doubles per tile, four places per entry
-    int lazy;                    // no counting pass: the fill kernel counts
+    int *tileN, *tileC;          // product of two matrices: tiles of a tile row of B, of a tile column of A
+    const int *nB;               // row lengths of B
+    double cost;                 // sparse products that a tile product is taken for (0: whatever they are)
+    int4 *early;                 // pinned: {told, products, tile products, stored entries * 2 + asym} before the check
+    int sample;                  // who counts looks for the mirrors of a few entries, and packs no group that packs badly
     int *tab; int span;          // [NG][span] place of block (G, G + s) in the pool, or -1
     unsigned long long *pool; unsigned long long cap;
     void *Cv; int *Ci; int *Cn; int ldc; int Mc;
     double thr;
     double *dA, *dC;             // per-group sums of the diagonals of X and X^2
-    TileFlags *flags, *host;     // host: pinned, written by the row kernel's last CTA
+    TileFlags *flags, *host;     // host: pinned, written by the last CTA of the counting and of the row kernel,
+    int told;                    // which then set the word behind it to this
     // second operand, as rows of its transpose (the sparse X^2: the same lists)
     const unsigned *bitsB; const unsigned short *rankB; const int *eoffB; const int2 *rangeB;
     // masked product
@@ -147,31 +164,71 @@ struct TileArgs
     int reach, check_pre;
 };
 
-// The flags as they are in L2, into the host's copy (complete when the kernel
-// is); one warp.
+constexpr int TOLD = 32; // the word behind the host's copy of the flags
+constexpr size_t EARLY = 1024; // and where the early counts lie
+
+// The flags as they are in L2, into the host's copy, and then the word that
+// the host waits for (0: it waits for the kernel); one warp.
 __device__ __forceinline__ void tell_host(const TileArgs &g, int lane)
 {
-    static_assert(sizeof(TileFlags) <= 32 * sizeof(int), "a word per lane");
+    static_assert(sizeof(TileFlags) <= TOLD * sizeof(int), "a word per lane");
+    volatile int *host = reinterpret_cast<volatile int *>(g.host);
     if (lane < (int) (sizeof(TileFlags) / sizeof(int)))
-        reinterpret_cast<volatile int *>(g.host)[lane] = reinterpret_cast<const volatile int *>(g.flags)[lane];
+        host[lane] = reinterpret_cast<const volatile int *>(g.flags)[lane];
+    __threadfence_system();
+    __syncwarp();
+    if (lane == 0 && g.told)
+        host[TOLD] = g.told;
 }
 
-// The form does not apply: the kernels after the fill do nothing.
-__device__ __forceinline__ bool declined(const TileFlags *f)
+// By the counts the sparse form does better, or a sample told that X is not
+// symmetric.
+__host__ __device__ __forceinline__ bool left_to_sparse(const TileFlags &f, double cost)
 {
-    return f->bad || f->odd || f->asym || f->alone || (double) f->tiles2 * TILE_COST > (double) f->products;
+    return f.bad || f.asym || (double) f.tiles2 * cost > (double) f.products;
+}
+
+// A product of two matrices by its counts (cost 0: whatever they are): what the
+// sparse form takes longer for, in us, a row, an entry of A (each visits a row
+// of B) and a product, against a tile product and what the tile form's twelve
+// launches take whatever the sizes.  Fitted to 95 products of bands, lattices,
+// diagonals and scattered matrices of 500 to 64000 rows, on which it takes
+// neither form where the other is more than 5 % faster (tile form / sparse form,
+// us: bands of 3 and 3 of 4096 rows 114 / 83, of 8000 144 / 135, of 20000 243 /
+// 303, of 31 and 31 122 / 109, 160 / 192 and 270 / 427, of 301 and 301 of 500
+// rows 209 / 114, of 1700 231 / 351, of 4096 261 / 799; a diagonal times a 16^3
+// lattice 130 / 105, times a 28^3 one 416 / 562; lattices of radii 3 and 3.5, 14^3
+// 222 / 196, 22^3 628 / 784; 4096 scattered rows of 20 1059 / 142).
+__host__ __device__ __forceinline__ bool general_pays(double rows, double stored, double products, double tiles2,
+                                                      double cost)
+{
+    return cost == 0.0 || 6.5e-3 * rows + 1e-4 * stored + 1.4e-6 * products - 45e-6 * tiles2 > 65.0;
+}
+// The form does not apply: the kernels after the fill do nothing.  (`alone` says
+// so only when the symmetry check is through; the others are set for good.)
+__device__ __forceinline__ bool unpacked(const TileArgs &g)
+{
+    const TileFlags *f = g.flags;
+    return f->bad || f->odd || f->skipped || (!g.general && left_to_sparse(*f, g.cost));
+}
+__device__ __forceinline__ bool declined(const TileArgs &g)
+{
+    return unpacked(g) || (!g.general && g.flags->alone);
 }
 
 // The four tile rows' bitmaps of group G from the stored columns, in shared
 // memory, and which rows are strictly ascending (bit of *order; zero before);
 // false (uniform) when a row or column is out of range.
-__device__ __forceinline__ bool group_bitmaps(const TileArgs &g, int G, unsigned *bm, int *reach, unsigned *order)
+template <bool CROSS>
+__device__ __forceinline__ bool group_bitmaps(const TileArgs &g, int G, unsigned *bm, int *reach, unsigned *order,
+                                              unsigned long long *products)
 {
     for (int w = threadIdx.x; w < 4 * g.nw; w += FT)
         bm[w] = 0u;
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int bad = 0, far = 0;
+    unsigned long long prod = 0;
     for (int r = warp; r < GR; r += FT / 32)
     {
         const int i = G * GR + r;
@@ -208,6 +265,8 @@ __device__ __forceinline__ bool group_bitmaps(const TileArgs &g, int G, unsigned
                     continue;
                 }
                 far = max(far, abs(k - i));
+                if (CROSS)
+                    prod += max(0, __ldg(g.nB + k));
                 const unsigned bit = 1u << ((k >> 3) & 31);
                 if (!(*(volatile unsigned *) &row[k >> 8] & bit))
                     atomicOr(&row[k >> 8], bit);
@@ -217,12 +276,18 @@ __device__ __forceinline__ bool group_bitmaps(const TileArgs &g, int G, unsigned
             atomicOr(order, 1u << r);
     }
     *reach = far;
+    if (CROSS)
+        *products = prod;
     return __syncthreads_or(bad) == 0;
 }
 
 // Tiles of each tile row and entries of group G (tot[0..4], zero before), and
-// its share of both forms' products and of the reach.
-__device__ __forceinline__ void group_counts(const TileArgs &g, int G, const unsigned *bm, int far, int *tot)
+// its share of both forms' products and of the reach; sums[0..2] (zero
+// before): products, tile products, stored entries.  CROSS: of a product of two
+// matrices (products: this thread's; the tiles go to their columns).
+template <bool CROSS>
+__device__ __forceinline__ void group_counts(const TileArgs &g, int G, const unsigned *bm, int far,
+                                             unsigned long long products, int *tot, unsigned long long *sums)
 {
     int c[5] = {0, 0, 0, 0, 0};
     for (int w = threadIdx.x; w < g.nw; w += FT)
@@ -236,18 +301,26 @@ __device__ __forceinline__ void group_counts(const TileArgs &g, int G, const uns
             any |= b;
         }
         c[4] += __popc(any);
+        if (CROSS)
+            for (unsigned m = any; m; m &= m - 1)
+            {
+                const int q = __ffs(m) - 1;
+                int n = 0;
+#pragma unroll
+                for (int a = 0; a < 4; ++a)
+                    n += bm[a * g.nw + w] >> q & 1u;
+                atomicAdd(&g.tileC[w * 32 + q], n);
+            }
     }
-    unsigned long long n2 = 0;
-    if (threadIdx.x < GR && G * GR + threadIdx.x < g.N)
-    {
-        const unsigned long long n = (unsigned long long) g.Xn[G * GR + threadIdx.x];
-        n2 = n * n;
-    }
+    const int n1 = threadIdx.x < GR && G * GR + threadIdx.x < g.N ? g.Xn[G * GR + threadIdx.x] : 0;
+    int n = n1;
+    unsigned long long n2 = CROSS ? products : (unsigned long long) n1 * n1;
     for (int o = 16; o; o >>= 1)
     {
 #pragma unroll
         for (int a = 0; a < 5; ++a)
             c[a] += __shfl_xor_sync(FULL, c[a], o);
+        n += __shfl_xor_sync(FULL, n, o);
         n2 += __shfl_xor_sync(FULL, n2, o);
         far = max(far, __shfl_xor_sync(FULL, far, o));
     }
@@ -258,7 +331,9 @@ __device__ __forceinline__ void group_counts(const TileArgs &g, int G, const uns
             if (c[a])
                 atomicAdd(&tot[a], c[a]);
         if (n2)
-            atomicAdd(&g.flags->products, n2);
+            atomicAdd(&sums[0], n2);
+        if (n)
+            atomicAdd(&sums[2], (unsigned long long) n);
         if (far > *(volatile int *) &g.flags->reach)
             atomicMax(&g.flags->reach, far);
     }
@@ -266,35 +341,177 @@ __device__ __forceinline__ void group_counts(const TileArgs &g, int G, const uns
     if (threadIdx.x == 0)
     {
         unsigned long long t2 = 0;
-        for (int a = 0; a < 4; ++a)
+        for (int a = 0; a < 4 && !CROSS; ++a)
             t2 += (unsigned long long) tot[a] * tot[a];
-        atomicAdd(&g.flags->tiles2, t2);
+        sums[1] = t2;
+        atomicAdd(&g.flags->products, sums[0]);
+        atomicAdd(&g.flags->stored, sums[2]);
+        if (!CROSS)
+            atomicAdd(&g.flags->tiles2, t2);
+        atomicAdd(&g.flags->counted, tot[4]);
     }
 }
 
+// A look for the mirror of one entry of a row, in two parts, so that the loads
+// of the first are under way while the caller counts: find() tells of a row
+// without it.  One warp.
+template <typename T, int U> struct MirrorSample
+{
+    int i, k, kk[U];
+    T x, v[U];
+
+    __device__ __forceinline__ void choose(const TileArgs &g, int row)
+    {
+        i = row;
+        k = -1;
+        const int n = i < g.N ? g.Xn[i] : 0;
+        if (n < 1 || n > g.ld)
+            return;
+        const size_t at = (size_t) i * g.ld + ((unsigned) i * 2654435761u >> 8) % (unsigned) n;
+        k = __ldg(g.Xi + at);
+        x = __ldg(static_cast<const T *>(g.Xv) + at);
+    }
+    __device__ __forceinline__ void load(const TileArgs &g, int p0, int lane)
+    {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+        {
+            const int p = p0 + 32 * u + lane;
+            const size_t at = (size_t) k * g.ld + p;
+            kk[u] = k >= 0 && k < g.N && p < g.ld ? __ldg(g.Xi + at) : -1;
+            v[u] = k >= 0 && k < g.N && p < g.ld ? __ldg(static_cast<const T *>(g.Xv) + at) : T(0);
+        }
+    }
+    __device__ __forceinline__ bool missing(const TileArgs &g, int lane)
+    {
+        if (k < 0 || k >= g.N)
+            return false;
+        const int m = min(g.Xn[k], g.ld);
+        bool twin = false;
+        for (int p0 = 0;;)
+        {
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                twin |= p0 + 32 * u + lane < m && kk[u] == i && v[u] == x;
+            p0 += 32 * U;
+            if (__any_sync(FULL, twin) || p0 >= m)
+                break;
+            load(g, p0, lane);
+        }
+        return !__any_sync(FULL, twin);
+    }
+};
+
+// The last CTA of a launch to come here (uniform), with what all have counted.
+__device__ __forceinline__ bool last_cta(const TileArgs &g, int *fin)
+{
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        __threadfence(); // this CTA's counts come before its own
+        *fin = atomicAdd(&g.flags->counters, 1) == (int) gridDim.x - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    return *fin;
+}
+
 // Counts: tiles, entries and the products of both forms.
-__global__ void __launch_bounds__(FT) tile_count_kernel(TileArgs g)
+// Two CTAs per SM, and so 32 registers a thread: one took 45 us instead of 27
+// for 26999 rows.
+template <typename T> __global__ void __launch_bounds__(FT, 2) tile_count_kernel(TileArgs g)
 {
     extern __shared__ unsigned bm[];
     __shared__ int tot[5];
+    __shared__ unsigned long long sums[3];
+    __shared__ int fin;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int G = blockIdx.x; G < g.NG; G += gridDim.x)
     {
         if (threadIdx.x < 5)
             tot[threadIdx.x] = 0;
+        if (threadIdx.x < 3)
+            sums[threadIdx.x] = 0;
+        // one row in eight of one group in eight
+        MirrorSample<T, 1> look;
+        const bool looks = g.sample && !(G & 7) && !(warp & 7);
+        if (looks)
+            look.choose(g, G * GR + warp);
         int far = 0;
-        if (!group_bitmaps(g, G, bm, &far, nullptr))
+        if (!group_bitmaps<false>(g, G, bm, &far, nullptr, nullptr))
         {
             if (threadIdx.x == 0)
                 atomicExch(&g.flags->bad, 1);
-            return;
+            break;
         }
-        group_counts(g, G, bm, far, tot);
-        if (threadIdx.x == 0)
+        if (looks)
+            look.load(g, 0, lane);
+        group_counts<false>(g, G, bm, far, 0, tot, sums);
+        if (looks && look.missing(g, lane) && lane == 0)
+            atomicExch(&g.flags->asym, 1);
+        __syncthreads();
+    }
+    if (g.told && last_cta(g, &fin) && warp == 0)
+        tell_host(g, lane);
+}
+
+// The same for a product of two matrices: a's counts, the products of its
+// entries with b's rows, and, once all groups of both have been through, the
+// tile products: tiles of a's tile column J times tiles of b's tile row J.
+__global__ void __launch_bounds__(FT, 2) tile_cross_kernel(TileArgs a, TileArgs b)
+{
+    extern __shared__ unsigned bm[];
+    __shared__ int tot[5];
+    __shared__ unsigned long long sums[3];
+    __shared__ int fin;
+    const int lane = threadIdx.x & 31;
+    bool ok = true;
+    for (int q = blockIdx.x; ok && q < 2 * a.NG; q += gridDim.x)
+    {
+        if (threadIdx.x < 5)
+            tot[threadIdx.x] = 0;
+        if (threadIdx.x < 3)
+            sums[threadIdx.x] = 0;
+        int far = 0;
+        unsigned long long products = 0;
+        if (q < a.NG)
         {
-            atomicAdd(&g.flags->entries, tot[4]);
+            ok = group_bitmaps<true>(a, q, bm, &far, nullptr, &products);
+            if (ok)
+                group_counts<true>(a, q, bm, far, products, tot, sums);
+        }
+        else
+        {
+            ok = group_bitmaps<false>(b, q - a.NG, bm, &far, nullptr, nullptr);
+            // a warp per tile row
+            if (ok && threadIdx.x < 128)
+            {
+                int n = 0;
+                for (int w = lane; w < b.nw; w += 32)
+                    n += __popc(bm[(threadIdx.x >> 5) * b.nw + w]);
+                for (int o = 16; o; o >>= 1)
+                    n += __shfl_xor_sync(FULL, n, o);
+                if (lane == 0)
+                    a.tileN[4 * (q - a.NG) + (threadIdx.x >> 5)] = n;
+            }
         }
         __syncthreads();
     }
+    if (!ok && threadIdx.x == 0)
+        atomicExch(&a.flags->bad, 1);
+    if (!last_cta(a, &fin))
+        return;
+    unsigned long long t2 = 0;
+    for (int J = threadIdx.x; J < 4 * a.NG; J += FT)
+        t2 += (unsigned long long) __ldcg(a.tileC + J) * __ldcg(a.tileN + J);
+    for (int o = 16; o; o >>= 1)
+        t2 += __shfl_xor_sync(FULL, t2, o);
+    if (lane == 0)
+        atomicAdd(&a.flags->tiles2, t2);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x < 32)
+        tell_host(a, lane);
 }
 
 __device__ __forceinline__ int tile_at(int r, int c) { return 2 * (4 * r + (c & 3)) + (c >> 2); }
@@ -302,7 +519,8 @@ __device__ __forceinline__ int tile_at(int r, int c) { return 2 * (4 * r + (c & 
 // Lists, zero-filled tiles and the scatter of group G's entries.  Rows in
 // ascending order have distinct columns and are stored; other rows are added
 // (duplicate columns add up, as they do in the sparse form).
-template <typename T> __global__ void __launch_bounds__(FT) tile_fill_kernel(TileArgs g)
+// LAZY: there was no counting pass, and no more groups than SMs.
+template <typename T, bool LAZY> __global__ void __launch_bounds__(FT, LAZY ? 1 : 2) tile_fill_kernel(TileArgs g)
 {
     extern __shared__ unsigned bm[]; // [4][nw] bitmaps | [nw] entries before the word
     int *before = reinterpret_cast<int *>(bm + 4 * g.nw);
@@ -312,6 +530,7 @@ template <typename T> __global__ void __launch_bounds__(FT) tile_fill_kernel(Til
     __shared__ int2 used;
     __shared__ double diag[GR];
     __shared__ int tot[5];
+    __shared__ unsigned long long sums[3];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     for (int G = blockIdx.x; G < g.NG; G += gridDim.x)
     {
@@ -323,6 +542,12 @@ template <typename T> __global__ void __launch_bounds__(FT) tile_fill_kernel(Til
         }
         if (tid < 5)
             tot[tid] = 0;
+        if (tid < 3)
+            sums[tid] = 0;
+        MirrorSample<T, 4> look;
+        const bool looks = LAZY && g.sample && !(warp & 7);
+        if (looks)
+            look.choose(g, G * GR + warp);
         int far = 0;
         if (g.gb)
         {
@@ -330,14 +555,27 @@ template <typename T> __global__ void __launch_bounds__(FT) tile_fill_kernel(Til
                 bm[w] = g.gb[(size_t) G * 4 * g.nw + w];
             __syncthreads();
         }
-        else if (!group_bitmaps(g, G, bm, &far, &order))
+        else if (!group_bitmaps<false>(g, G, bm, &far, &order, nullptr))
         {
             if (tid == 0)
                 atomicExch(&g.flags->bad, 1);
             return;
         }
-        if (g.lazy)
-            group_counts(g, G, bm, far, tot);
+        if (LAZY)
+        {
+            if (looks)
+                look.load(g, 0, lane);
+            group_counts<false>(g, G, bm, far, 0, tot, sums);
+            const bool alone = looks && look.missing(g, lane);
+            if (alone && lane == 0)
+                atomicExch(&g.flags->asym, 1);
+            // a group that packs badly is not packed until the counts of all say that the others make up for it
+            const bool badly = g.sample && (double) sums[1] * g.cost > 2.0 * (double) sums[0];
+            if (badly && tid == 0)
+                g.flags->skipped = 1;
+            if (__syncthreads_or(alone || badly))
+                continue;
+        }
         for (int s = tid; s < g.span; s += FT)
             g.tab[(size_t) G * g.span + s] = -1;
         if (tid == 0 && !g.masked)
@@ -489,7 +727,13 @@ __global__ void __launch_bounds__(PT) tile_sym_kernel(TileArgs g)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     __shared__ int lastH, alone;
-    if (g.flags->bad)
+    if (g.early && blockIdx.x == 0 && threadIdx.x == 0)
+        // one store of 16 bytes: the host sees all of it or nothing
+        asm volatile("st.volatile.global.v4.s32 [%0], {%1, %2, %3, %4};" ::"l"(g.early), "r"(g.told),
+                     "r"(__float_as_int((float) g.flags->products)), "r"(__float_as_int((float) g.flags->tiles2)),
+                     "r"((int) g.flags->stored * 2 + (g.flags->asym || g.flags->bad))
+                     : "memory");
+    if (__syncthreads_or(unpacked(g))) // other CTAs may find an entry without its mirror meanwhile
         return;
     for (int G = blockIdx.x; G < g.NG; G += gridDim.x)
     {
@@ -655,7 +899,7 @@ template <typename T, int MODE> __global__ void __launch_bounds__(TW * 32, TMIN)
     constexpr bool MASKED = MODE == TILE_MASKED, GENERAL = MODE == TILE_GENERAL;
     extern __shared__ __align__(16) unsigned char tsm[]; // per warp: stages[TS][8 tiles] | queue[QCAP]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (MASKED ? g.flags->odd : declined(g.flags))
+    if (__any_sync(FULL, MASKED ? g.flags->odd : declined(g))) // other warps may set odd meanwhile
         return;
     uint2 *qu = reinterpret_cast<uint2 *>(tsm + warp * WARP_SMEM + TS * 4096);
     const unsigned stage0 = (unsigned) __cvta_generic_to_shared(tsm + warp * WARP_SMEM) + lane * 16;
@@ -917,7 +1161,7 @@ template <typename T> __global__ void __launch_bounds__(RT, sizeof(T) == 8 ? 1 :
     __shared__ int wtot[W];
     __shared__ int nblk;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (declined(g.flags) || g.flags->full)
+    if (declined(g) || g.flags->full)
     {
         if (blockIdx.x == 0 && warp == 0)
             tell_host(g, lane);
@@ -1126,7 +1370,7 @@ __global__ void __launch_bounds__(PT) tile_tbits_kernel(TileArgs g)
                 atomicExch(&g.flags->bad, 1);
             continue;
         }
-        if (lane == 0 && n)
+        if (lane == 0 && n && !g.general)
             atomicAdd(&g.flags->products, (unsigned long long) n * n);
         const unsigned bit = 1u << ((j >> 3) & 31);
         int far = 0;
@@ -1154,6 +1398,7 @@ __global__ void __launch_bounds__(PT) tile_tbits_kernel(TileArgs g)
 __global__ void __launch_bounds__(PT) tile_tcount_kernel(TileArgs g)
 {
     __shared__ int tot[5];
+    __shared__ int fin;
     for (int G = blockIdx.x; G < g.NG; G += gridDim.x)
     {
         if (threadIdx.x < 5)
@@ -1182,11 +1427,14 @@ __global__ void __launch_bounds__(PT) tile_tcount_kernel(TileArgs g)
             unsigned long long t2 = 0;
             for (int a = 0; a < 4; ++a)
                 t2 += (unsigned long long) tot[a] * tot[a];
-            atomicAdd(&g.flags->tiles2, t2);
-            atomicAdd(&g.flags->entries, tot[4]);
+            if (!g.general)
+                atomicAdd(&g.flags->tiles2, t2);
+            atomicAdd(&g.flags->counted, tot[4]);
         }
         __syncthreads();
     }
+    if (g.told && last_cta(g, &fin) && threadIdx.x < 32)
+        tell_host(g, threadIdx.x);
 }
 
 // B's entries into the transpose's tiles; one warp per row of B.
@@ -1317,6 +1565,60 @@ template <typename T> __global__ void __launch_bounds__(PT) tile_gather_kernel(T
     }
 }
 
+void pause()
+{
+#ifdef __x86_64__
+    __builtin_ia32_pause();
+#endif
+}
+
+// The host's copy of the flags, once a kernel has told (tell_host) the given
+// number.  The word in pinned memory is read for a while before the stream is
+// waited for: it is there some microseconds before cudaStreamSynchronize
+// returns, and no copy has to be queued.
+bool flags_told(B200Context *c, const TileFlags *hf, int told)
+{
+    const volatile int *word = reinterpret_cast<const volatile int *>(hf) + TOLD;
+    for (int spin = 0; spin < 20000 && *word != told; ++spin)
+        pause();
+    std::atomic_thread_fence(std::memory_order_acquire);
+    if (*word == told)
+        return true;
+    if (!b200_sync())
+        return false;
+    std::atomic_thread_fence(std::memory_order_acquire);
+    if (*word == told)
+        return true;
+    b200_set_error(BML_B200_ERR_CUDA, "multiply: the tile kernels did not report");
+    return false;
+}
+
+// What the symmetry check has told of the counts at its start, if it does
+// within the wait.
+bool early_told(const TileArgs &g, TileOutcome *out)
+{
+    const volatile int4 *e = g.early;
+    for (int spin = 0; spin < 20000 && e->x != g.told; ++spin)
+        pause();
+    std::atomic_thread_fence(std::memory_order_acquire);
+    if (e->x != g.told)
+        return false;
+    const int p = e->y, t = e->z, w = e->w;
+    float products, tiles2;
+    memcpy(&products, &p, 4);
+    memcpy(&tiles2, &t, 4);
+    out->asym = w & 1;
+    out->counted = true;
+    out->counts = {(unsigned long long) products, (unsigned long long) (w >> 1), (unsigned long long) tiles2, 0, 0};
+    return true;
+}
+
+int next_told()
+{
+    static std::atomic<unsigned> n{0};
+    return (int) (++n & 0x7fffffffu) | 1 << 30; // never 0
+}
+
 template <typename T> bool tile_masked_typed(TileArgs a, TileArgs b, bool *taken)
 {
     B200Context *c = b200_ctx();
@@ -1364,7 +1666,7 @@ template <typename T> bool tile_masked_typed(TileArgs a, TileArgs b, bool *taken
         tile_tcount_kernel<<<per, PT, 0, c->stream>>>(b);
         if (!LAUNCH_OK("tile_tcount_kernel"))
             return false;
-        tile_count_kernel<<<per, FT, smemC, c->stream>>>(a);
+        tile_count_kernel<T><<<per, FT, smemC, c->stream>>>(a);
         if (!LAUNCH_OK("tile_count_kernel"))
             return false;
         a.count_only = 1;
@@ -1372,12 +1674,12 @@ template <typename T> bool tile_masked_typed(TileArgs a, TileArgs b, bool *taken
         if (!LAUNCH_OK("tile_pattern_kernel") ||
             !CUDA_OK(cudaMemcpyAsync(hf, small, sizeof(TileFlags), cudaMemcpyDeviceToHost, c->stream)) || !b200_sync())
             return false;
-        if (hf->bad || hf->entries >= (1 << 28) || (double) hf->tiles2 * TILE_COST > (double) hf->products)
+        if (hf->counted >= (1 << 28) || left_to_sparse(*hf, a.cost))
             return true;
         take(0);
-        const size_t o_ent = take((size_t) hf->entries * sizeof(unsigned));
-        const size_t o_entJ = take((size_t) hf->entries * sizeof(unsigned short));
-        const size_t o_tiles = take((size_t) hf->entries * 2048);
+        const size_t o_ent = take((size_t) hf->counted * sizeof(unsigned));
+        const size_t o_entJ = take((size_t) hf->counted * sizeof(unsigned short));
+        const size_t o_tiles = take((size_t) hf->counted * 2048);
         const size_t o_blk = take((size_t) hf->blocks * sizeof(int2));
         const size_t o_out = take((size_t) hf->blocks * 8192);
         if (at > ((size_t) 64 << 30))
@@ -1410,10 +1712,10 @@ template <typename T> bool tile_masked_typed(TileArgs a, TileArgs b, bool *taken
     a.count_only = 0;
     if (!CUDA_OK(cudaMemsetAsync(small, 0, sizeof(TileFlags), c->stream)))
         return false;
-    tile_fill_kernel<T><<<per, FT, smemF, c->stream>>>(a);
+    tile_fill_kernel<T, false><<<per, FT, smemF, c->stream>>>(a);
     if (!LAUNCH_OK("tile_fill_kernel"))
         return false;
-    tile_fill_kernel<T><<<per, FT, smemF, c->stream>>>(b);
+    tile_fill_kernel<T, false><<<per, FT, smemF, c->stream>>>(b);
     if (!LAUNCH_OK("tile_fill_kernel"))
         return false;
     tile_scatter_kernel<T><<<std::min(b200_ceil_div(b.N, PT / 32), c->sm_count * 8), PT, 0, c->stream>>>(b);
@@ -1507,8 +1809,16 @@ __global__ void __launch_bounds__(PT) tile_touch_kernel(TileArgs g)
     }
 }
 
+// Whether the counts can say so at all, by the room of the rows.
+bool general_may_pay(const bml_matrix_ellpack_t *A, const bml_matrix_ellpack_t *B, double cost)
+{
+    const double stored = (double) A->N * A->ld;
+    return general_pays(A->N, stored, stored * B->ld, 0.0, cost);
+}
+
 template <typename T>
-bool tile_general_typed(TileArgs a, TileArgs b, double *trace, int *required_M, bool *taken, cudaEvent_t *timer)
+bool tile_general_typed(TileArgs a, TileArgs b, const TileCounts *known, double *trace, int *required_M, bool *taken,
+                        cudaEvent_t *timer)
 {
     B200Context *c = b200_ctx();
     if (!c)
@@ -1516,7 +1826,7 @@ bool tile_general_typed(TileArgs a, TileArgs b, double *trace, int *required_M, 
     unsigned char *small = static_cast<unsigned char *>(c->d_small) + TL_SMALL;
     TileFlags *hf = reinterpret_cast<TileFlags *>(static_cast<unsigned char *>(c->pinned) + TL_SMALL);
     a.flags = b.flags = reinterpret_cast<TileFlags *>(small);
-    a.host = hf;
+    a.host = b.host = hf;
     const int NG = a.NG, nw = a.nw;
     const int per = std::min(NG, c->sm_count * 8);
     const int rows = std::min(b200_ceil_div(a.N, PT / 32), c->sm_count * 8);
@@ -1534,41 +1844,75 @@ bool tile_general_typed(TileArgs a, TileArgs b, double *trace, int *required_M, 
     const size_t o_rank = take((size_t) 2 * NG * nw * sizeof(unsigned short));
     const size_t o_eoff = take((size_t) 2 * NG * sizeof(int)), o_range = take((size_t) 2 * NG * sizeof(int2));
     const size_t o_touched = take((size_t) a.N * sizeof(int)), o_diag = take((size_t) 2 * NG * sizeof(double));
+    const size_t o_tileN = take((size_t) 8 * NG * sizeof(int));
     const size_t fixed = at;
     size_t o_ent = 0, o_entJ = 0, o_tiles = 0, o_tab = 0, o_pool = 0;
-    unsigned char *scr = nullptr;
+    unsigned char *scr = static_cast<unsigned char *>(b200_scratch_try(fixed));
+    if (!scr)
+        return true; // the sparse form takes less
+    // the products of both forms, unless X^2's symmetric attempt has counted them
+    TileCounts n{};
+    if (known)
+        n = *known;
+    else
+    {
+        a.told = next_told();
+        if (!CUDA_OK(cudaMemsetAsync(small, 0, sizeof(TileFlags), c->stream)))
+            return false;
+        if (a.Xi == b.Xi)
+            tile_count_kernel<T><<<per, FT, smemC, c->stream>>>(a);
+        else
+        {
+            TileArgs rows_b = b;
+            a.nB = b.Xn;
+            a.tileN = reinterpret_cast<int *>(scr + o_tileN);
+            a.tileC = a.tileN + 4 * NG;
+            if (!CUDA_OK(cudaMemsetAsync(a.tileC, 0, (size_t) 4 * NG * sizeof(int), c->stream)))
+                return false;
+            tile_cross_kernel<<<std::min(2 * NG, c->sm_count * 8), FT, smemC, c->stream>>>(a, rows_b);
+        }
+        if (!LAUNCH_OK("tile counts") || !flags_told(c, hf, a.told))
+            return false;
+        a.told = 0;
+        if (hf->bad)
+            return true;
+        n = {hf->products, hf->stored, hf->tiles2, hf->counted, hf->reach};
+    }
+    if (n.entries <= 0 || !general_pays(a.N, (double) n.stored, (double) n.products, (double) n.tiles2, a.cost))
+        return true;
     int reach = 0;
-    // the counts, then the layout; a larger arena loses B's bitmaps, which are then made again
+    // the second operand's entries, then the layout; a larger arena loses B's bitmaps, which are then made again
     for (int attempt = 0; attempt < 2; ++attempt)
     {
         if (attempt && at <= c->scratch_bytes)
+        {
+            if (!CUDA_OK(cudaMemsetAsync(b.rowbits, 0, n_rb, c->stream)))
+                return false;
             break;
+        }
         scr = static_cast<unsigned char *>(b200_scratch_try(attempt ? at : fixed));
         if (!scr)
             return true; // the sparse form takes less
         b.gb = reinterpret_cast<unsigned *>(scr + o_gb);
         b.rowbits = reinterpret_cast<unsigned *>(scr + o_rb);
-        if (!CUDA_OK(cudaMemsetAsync(b.gb, 0, n_gb, c->stream)) ||
-            !CUDA_OK(cudaMemsetAsync(b.rowbits, 0, n_rb, c->stream)) ||
-            !CUDA_OK(cudaMemsetAsync(small, 0, sizeof(TileFlags), c->stream)))
+        if (!CUDA_OK(cudaMemsetAsync(small, 0, sizeof(TileFlags), c->stream)) ||
+            !CUDA_OK(cudaMemsetAsync(b.gb, 0, n_gb, c->stream)) ||
+            (attempt && !CUDA_OK(cudaMemsetAsync(b.rowbits, 0, n_rb, c->stream))))
             return false;
         tile_tbits_kernel<<<rows, PT, 0, c->stream>>>(b);
         if (!LAUNCH_OK("tile_tbits_kernel"))
             return false;
         if (attempt)
             break;
+        b.told = next_told();
         tile_tcount_kernel<<<per, PT, 0, c->stream>>>(b);
-        if (!LAUNCH_OK("tile_tcount_kernel"))
+        if (!LAUNCH_OK("tile_tcount_kernel") || !flags_told(c, hf, b.told))
             return false;
-        tile_count_kernel<<<per, FT, smemC, c->stream>>>(a);
-        if (!LAUNCH_OK("tile_count_kernel") ||
-            !CUDA_OK(cudaMemcpyAsync(hf, small, sizeof(TileFlags), cudaMemcpyDeviceToHost, c->stream)) || !b200_sync())
-            return false;
-        if (hf->bad || hf->entries <= 0 || hf->entries >= (1 << 28) ||
-            (double) hf->tiles2 * TILE_COST > (double) hf->products)
+        b.told = 0;
+        const long long entries = (long long) n.entries + hf->counted;
+        if (hf->bad || hf->counted <= 0 || entries >= (1 << 28))
             return true;
-        const long long entries = hf->entries;
-        reach = std::min(a.N, hf->reach + hf->reachB);
+        reach = std::min(a.N, n.reach + hf->reachB);
         a.back = std::min(NG - 1, reach / GR + 1);
         a.span = 2 * a.back + 1;
         const size_t words = (size_t) a.N * a.Mc * sizeof(T) / 8 + 1 + (size_t) 17 * NG * a.span;
@@ -1610,10 +1954,10 @@ bool tile_general_typed(TileArgs a, TileArgs b, double *trace, int *required_M, 
     tile_touch_kernel<<<rows, PT, 0, c->stream>>>(a);
     if (!LAUNCH_OK("tile_touch_kernel"))
         return false;
-    tile_fill_kernel<T><<<per, FT, smemF, c->stream>>>(a);
+    tile_fill_kernel<T, false><<<per, FT, smemF, c->stream>>>(a);
     if (!LAUNCH_OK("tile_fill_kernel"))
         return false;
-    tile_fill_kernel<T><<<per, FT, smemF, c->stream>>>(b);
+    tile_fill_kernel<T, false><<<per, FT, smemF, c->stream>>>(b);
     if (!LAUNCH_OK("tile_fill_kernel"))
         return false;
     tile_scatter_kernel<T><<<rows, PT, 0, c->stream>>>(b);
@@ -1632,8 +1976,9 @@ bool tile_general_typed(TileArgs a, TileArgs b, double *trace, int *required_M, 
         return false;
     if (timer && !CUDA_OK(cudaEventRecord(timer[1], c->stream)))
         return false;
+    a.told = next_told();
     tile_rows_kernel<T><<<NG, RT, smemR, c->stream>>>(a);
-    if (!LAUNCH_OK("tile_rows_kernel") || !b200_sync())
+    if (!LAUNCH_OK("tile_rows_kernel") || !flags_told(c, hf, a.told))
         return false;
     if (hf->bad || hf->odd || hf->full)
         return true;
@@ -1655,14 +2000,14 @@ bool tile_general_typed(TileArgs a, TileArgs b, double *trace, int *required_M, 
 }
 
 template <typename T>
-bool tile_x2_typed(TileArgs g, double *trace, int *required_M, bool *taken, bool *asym, cudaEvent_t *timer)
+bool tile_x2_typed(TileArgs g, double *trace, int *required_M, TileOutcome *out, cudaEvent_t *timer,
+                   bool pack_all = false)
 {
     B200Context *c = b200_ctx();
     if (!c)
         return false;
     unsigned char *small = static_cast<unsigned char *>(c->d_small) + TL_SMALL;
-    unsigned char *pin = static_cast<unsigned char *>(c->pinned) + TL_SMALL;
-    TileFlags *hf = reinterpret_cast<TileFlags *>(pin);
+    TileFlags *hf = reinterpret_cast<TileFlags *>(static_cast<unsigned char *>(c->pinned) + TL_SMALL);
     g.flags = reinterpret_cast<TileFlags *>(small);
     g.host = hf;
     const int per = (int) std::min<long long>(g.NG, (long long) c->sm_count * 8);
@@ -1670,27 +2015,31 @@ bool tile_x2_typed(TileArgs g, double *trace, int *required_M, bool *taken, bool
     const size_t smemF = (size_t) 5 * g.nw * sizeof(unsigned); // at most 40 KB
     if (!CUDA_OK(cudaMemsetAsync(small, 0, sizeof(TileFlags), c->stream)))
         return false;
-    // Small matrices are laid out for the most tiles they can have, which saves the counting pass and its
-    // round trip; the fill kernel then counts, and the later kernels find the form declined.
+    // Small matrices are laid out for the most tiles they can have, which saves the counting pass and its round trip;
+    // the fill kernel then counts, and the later kernels find the form declined.  (LAZY_BYTES admits 4096 rows: X^2 of
+    // rows of 33 and of 341 takes 71 and 138 us there, 76 and 151 at 4097, with the counting pass.)
     const long long nbk = b200_ceil_div(g.N, 8);
     long long entries = std::min((long long) g.NG * nbk, (long long) g.N * g.ld);
     int span = g.NG;
-    g.lazy = entries * 2048 <= LAZY_BYTES;
-    if (!g.lazy)
+    const bool lazy = entries * 2048 <= LAZY_BYTES;
+    auto note = [&]() {
+        out->asym = hf->asym || hf->alone;
+        out->counted = out->complete = !hf->bad;
+        out->counts = {hf->products, hf->stored, hf->tiles2, hf->counted, hf->reach};
+    };
+    g.sample = pack_all ? 0 : 1;
+    if (!lazy)
     {
-        tile_count_kernel<<<per, FT, smemC, c->stream>>>(g);
-        if (!LAUNCH_OK("tile_count_kernel") ||
-            !CUDA_OK(cudaMemcpyAsync(pin, small, sizeof(TileFlags), cudaMemcpyDeviceToHost, c->stream)) ||
-            !b200_sync())
+        g.told = next_told();
+        tile_count_kernel<T><<<per, FT, smemC, c->stream>>>(g);
+        if (!LAUNCH_OK("tile_count_kernel") || !flags_told(c, hf, g.told))
             return false;
-        if (hf->bad || hf->entries <= 0 || hf->entries >= (1 << 28) ||
-            (double) hf->tiles2 * TILE_COST > (double) hf->products)
+        g.told = 0;
+        note();
+        if (hf->counted <= 0 || hf->counted >= (1 << 28) || left_to_sparse(*hf, g.cost))
             return true;
-        entries = hf->entries;
+        entries = hf->counted;
         span = std::min(g.NG, 2 * (hf->reach / GR + 1) + 1);
-        // the counters start again at zero: the fill kernel hands out places with them
-        if (!CUDA_OK(cudaMemsetAsync(small, 0, sizeof(TileFlags), c->stream)))
-            return false;
     }
     const size_t smemR = (size_t) 2 * span * sizeof(int2);
     if (smemR > c->smem_optin - 8192)
@@ -1741,18 +2090,28 @@ bool tile_x2_typed(TileArgs g, double *trace, int *required_M, bool *taken, bool
     g.rankB = g.rank;
     g.eoffB = g.eoff;
     g.rangeB = g.range;
-    tile_fill_kernel<T><<<per, FT, smemF, c->stream>>>(g);
+    const long long items =
+        (long long) ((g.NG + SG - 1) / SG * SG) * ((span + SC - 1) / SC * SC); // counted in an int by the kernel
+    if (items >= 1 << 30)
+        return true;
+    if (!lazy)
+        tile_fill_kernel<T, false><<<per, FT, smemF, c->stream>>>(g);
+    else
+    {
+        g.told = next_told();
+        g.early = reinterpret_cast<int4 *>(reinterpret_cast<unsigned char *>(hf) + EARLY);
+        tile_fill_kernel<T, true><<<per, FT, smemF, c->stream>>>(g);
+    }
     if (!LAUNCH_OK("tile_fill_kernel"))
         return false;
     tile_sym_kernel<<<per, PT, 0, c->stream>>>(g);
     if (!LAUNCH_OK("tile_sym_kernel"))
         return false;
+    // what follows is queued while the check runs, or left out; if the word does not come, the flags will tell
+    if (lazy && early_told(g, out) && (out->asym || (double) out->counts.tiles2 * g.cost > (double) out->counts.products))
+        return true;
     if (timer && !CUDA_OK(cudaEventRecord(timer[0], c->stream)))
         return false;
-    const long long items =
-        (long long) ((g.NG + SG - 1) / SG * SG) * ((span + SC - 1) / SC * SC); // counted in an int by the kernel
-    if (items >= 1 << 30)
-        return true;
     const size_t smemQ = (size_t) TW * WARP_SMEM;
     if (!CUDA_OK(cudaFuncSetAttribute(tile_x2_kernel<T, TILE_SQUARE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smemQ)))
         return false;
@@ -1765,15 +2124,16 @@ bool tile_x2_typed(TileArgs g, double *trace, int *required_M, bool *taken, bool
     if (smemR > 32768 && !CUDA_OK(cudaFuncSetAttribute(
                              tile_rows_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smemR)))
         return false;
+    g.told = next_told();
     tile_rows_kernel<T><<<g.NG, RT, smemR, c->stream>>>(g);
-    if (!LAUNCH_OK("tile_rows_kernel") || !b200_sync())
+    if (!LAUNCH_OK("tile_rows_kernel") || !flags_told(c, hf, g.told))
         return false;
-    if (hf->bad || hf->odd || hf->asym || hf->alone || hf->full || (double) hf->tiles2 * TILE_COST > (double) hf->products)
-    {
-        *asym = hf->asym || hf->alone;
+    note();
+    if (hf->skipped && !hf->odd && !out->asym && !left_to_sparse(*hf, g.cost))
+        return tile_x2_typed<T>(g, trace, required_M, out, timer, true);
+    if (hf->bad || hf->odd || hf->skipped || out->asym || hf->full || left_to_sparse(*hf, g.cost))
         return true;
-    }
-    *taken = true;
+    out->taken = true;
     if (required_M)
         *required_M = hf->max_width;
     if (trace)
@@ -1793,14 +2153,15 @@ bool tile_x2_typed(TileArgs g, double *trace, int *required_M, bool *taken, bool
 } // namespace
 
 bool ell_x2_tiles(bml_matrix_ellpack_t *X, bml_matrix_ellpack_t *C, double threshold, double *trace, int *required_M,
-                  bool *taken, bool *asym, cudaEvent_t *timer)
+                  TileOutcome *out, cudaEvent_t *timer)
 {
-    *taken = *asym = false;
+    *out = TileOutcome{};
     // a place in a group's list is kept in 16 bits
     const int nbk = b200_ceil_div(X->N, 8);
-    if (!(threshold >= 0.0) || X->N != C->N || X->N < 1 || nbk > 65535)
+    if (!g_tiles || !(threshold >= 0.0) || X->N != C->N || X->N < 1 || nbk > 65535)
         return true;
     TileArgs g{};
+    g.cost = g_tiles == 1 ? TILE_COST : 0.0;
     g.Xv = X->d_value;
     g.Xi = X->d_index;
     g.Xn = X->d_nnz;
@@ -1815,8 +2176,8 @@ bool ell_x2_tiles(bml_matrix_ellpack_t *X, bml_matrix_ellpack_t *C, double thres
     g.ldc = C->ld;
     g.Mc = C->M;
     g.thr = threshold;
-    return X->matrix_precision == double_real ? tile_x2_typed<double>(g, trace, required_M, taken, asym, timer)
-                                              : tile_x2_typed<float>(g, trace, required_M, taken, asym, timer);
+    return X->matrix_precision == double_real ? tile_x2_typed<double>(g, trace, required_M, out, timer)
+                                              : tile_x2_typed<float>(g, trace, required_M, out, timer);
 }
 
 bool ell_masked_tiles(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bml_matrix_ellpack_t *P,
@@ -1824,9 +2185,10 @@ bool ell_masked_tiles(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bml_matr
 {
     *taken = false;
     const int nbk = b200_ceil_div(A->N, 8);
-    if (A->N != B->N || A->N != C->N || nbk > 65535)
+    if (!g_tiles || A->N != B->N || A->N != C->N || nbk > 65535)
         return true;
     TileArgs a{};
+    a.cost = g_tiles == 1 ? TILE_COST : 0.0;
     a.N = a.ncols = A->N;
     a.NG = b200_ceil_div(A->N, GR);
     a.nw = b200_ceil_div(nbk, 32);
@@ -1854,13 +2216,20 @@ bool ell_masked_tiles(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bml_matr
 }
 
 bool ell_general_tiles(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bml_matrix_ellpack_t *C, double threshold,
-                       double *trace, int *required_M, bool check_pre, bool *taken, cudaEvent_t *timer)
+                       const TileOutcome *known, double *trace, int *required_M, bool check_pre, bool *taken,
+                       cudaEvent_t *timer)
 {
     *taken = false;
     const int nbk = b200_ceil_div(A->N, 8);
-    if (!(threshold >= 0.0) || A->N < GENERAL_ROWS || A->N != B->N || A->N != C->N || nbk > 65535)
+    if (!g_tiles || !(threshold >= 0.0) || A->N != B->N || A->N != C->N || nbk > 65535)
         return true;
     TileArgs a{};
+    a.cost = g_tiles == 1 ? TILE_COST : 0.0;
+    if (known ? !general_pays(A->N, (double) known->counts.stored, (double) known->counts.products,
+                              (double) known->counts.tiles2, a.cost)
+              : !general_may_pay(A, B, a.cost))
+        return true;
+    const TileCounts *counts = known && known->complete ? &known->counts : nullptr;
     a.N = a.ncols = A->N;
     a.NG = b200_ceil_div(A->N, GR);
     a.nw = b200_ceil_div(nbk, 32);
@@ -1885,6 +2254,13 @@ bool ell_general_tiles(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bml_mat
     a.ldc = C->ld;
     a.Mc = C->M;
     a.check_pre = check_pre ? 1 : 0;
-    return A->matrix_precision == double_real ? tile_general_typed<double>(a, b, trace, required_M, taken, timer)
-                                              : tile_general_typed<float>(a, b, trace, required_M, taken, timer);
+    return A->matrix_precision == double_real ? tile_general_typed<double>(a, b, counts, trace, required_M, taken, timer)
+                                              : tile_general_typed<float>(a, b, counts, trace, required_M, taken, timer);
+}
+
+extern "C" BML_B200_API int bml_b200_set_tiles(int mode)
+{
+    const int old = g_tiles;
+    g_tiles = mode < 0 ? 0 : mode > 2 ? 2 : mode;
+    return old;
 }

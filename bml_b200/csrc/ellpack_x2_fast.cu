@@ -797,6 +797,7 @@ bool g_x2_exact = false;
 bool g_x2_symmetric = true;
 bool g_last_symmetric = false;
 bool g_last_dense = false;
+int g_last_form = BML_B200_PRODUCT_ORDERED;
 // CUDA events around the product kernel (when timing is on), on the library
 // stream; the last duration in ms, or -1.
 bool g_time_kernel = false;
@@ -971,6 +972,7 @@ bool fast_multiply_typed(FastArgs g, double *trace, int *required_M, bool touch)
     const FastFlags *hf = reinterpret_cast<const FastFlags *>(pin);
     const double *ht = reinterpret_cast<const double *>(pin + 64);
     g_last_symmetric = g.sym_try && !hf->asym && !hf->bad_input;
+    g_last_form = g_last_symmetric ? BML_B200_PRODUCT_SPARSE_SYMMETRIC : BML_B200_PRODUCT_SPARSE;
     g_last_kernel_ms = -1.0f;
     if (timed && !CUDA_OK(cudaEventElapsedTime(&g_last_kernel_ms, g_kev[0], g_kev[1])))
         return false;
@@ -997,6 +999,11 @@ bool fast_multiply_typed(FastArgs g, double *trace, int *required_M, bool touch)
 
 } // namespace
 
+void ell_product_ordered()
+{
+    g_last_form = BML_B200_PRODUCT_ORDERED;
+}
+
 bool ell_x2_exact()
 {
     return g_x2_exact;
@@ -1014,6 +1021,7 @@ bool ell_multiply_dense_tier(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, b
     *taken = true;
     g_last_symmetric = false;
     g_last_dense = true;
+    g_last_form = BML_B200_PRODUCT_DENSE;
     return ell_multiply_dense(A, B, C, threshold, trace, required_M);
 }
 
@@ -1045,20 +1053,22 @@ bool ell_multiply_unordered(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bm
     const bool touch = check_pre || !(threshold >= 0.0);
     // on tiles: the symmetric square, or the general product where there is no symmetry to use
     const bool timed = kernel_timer();
-    bool taken = false, ok = true;
+    TileOutcome square{};
+    bool ok = true;
     if (g.sym_try && !touch)
     {
-        bool asym = false;
-        ok = ell_x2_tiles(A, C, threshold, trace, required_M, &taken, &asym, timed ? g_kev : nullptr);
-        if (asym)
+        ok = ell_x2_tiles(A, C, threshold, trace, required_M, &square, timed ? g_kev : nullptr);
+        if (square.asym)
             g.sym_try = 0;
     }
-    const bool square = taken;
+    bool taken = square.taken;
     if (ok && !taken && !g.sym_try)
-        ok = ell_general_tiles(A, B, C, threshold, trace, required_M, check_pre, &taken, timed ? g_kev : nullptr);
+        ok = ell_general_tiles(A, B, C, threshold, square.counted ? &square : nullptr, trace, required_M,
+                               check_pre, &taken, timed ? g_kev : nullptr);
     if (taken || !ok)
     {
-        g_last_symmetric = square;
+        g_last_symmetric = square.taken;
+        g_last_form = square.taken ? BML_B200_PRODUCT_TILES_SYMMETRIC : BML_B200_PRODUCT_TILES;
         g_last_kernel_ms = -1.0f;
         return !(timed && taken && !CUDA_OK(cudaEventElapsedTime(&g_last_kernel_ms, g_kev[0], g_kev[1]))) && ok;
     }
@@ -1092,6 +1102,7 @@ bool ell_multiply_masked(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bml_m
         if (tiles)
         {
             g_last_symmetric = false;
+            g_last_form = BML_B200_PRODUCT_TILES_MASKED;
             g_last_kernel_ms = -1.0f;
             ell_mark_device(C);
         }
@@ -1134,6 +1145,12 @@ extern "C" BML_B200_API int bml_b200_set_kernel_timing(int on)
 extern "C" BML_B200_API double bml_b200_last_x2_kernel_ms(void)
 {
     return (double) g_last_kernel_ms;
+}
+
+// Form of the last ELLPACK product (BML_B200_PRODUCT_*).
+extern "C" BML_B200_API int bml_b200_last_product_form(void)
+{
+    return g_last_form;
 }
 
 // 1 when the last unordered product ran on the dense tier.

@@ -155,19 +155,36 @@ bool ell_multiply_AB(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B,
 // ell_multiply_AB uses it unless the ordered (bit-identical) form is selected
 // (bml_b200_set_x2_exact) or the row width exceeds what it holds.
 bool ell_x2_exact();
+// Notes that the product at hand takes the ordered tiers.
+void ell_product_ordered();
 bool ell_unordered_fits(const bml_matrix_ellpack_t *A);
 bool ell_multiply_unordered(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bml_matrix_ellpack_t *C,
                             double threshold, double *trace, int *required_M, bool check_pre);
+// Counts that decide between the tile form and the sparse form.
+struct TileCounts
+{
+    unsigned long long products, stored, tiles2; // of stored entries; those of the first operand; of tiles
+    int entries, reach;                  // tile columns of the first operand's groups; its largest |column - row|
+};
+// How the symmetric attempt ended: whether it formed the product, found X not
+// to be symmetric, counted products and tiles, and entries and reach as well.
+struct TileOutcome
+{
+    bool taken, asym, counted, complete;
+    TileCounts counts;
+};
 // The tile form of the unordered X^2 (ellpack_tiles.cu): symmetric X whose rows
-// pack well into 8 x 8 tiles, threshold >= 0.  Leaves *taken false, with no
-// status set, where it does not apply (*asym: X was found not to be
-// symmetric); timer (nullable): events recorded around the product kernel.
+// pack well into 8 x 8 tiles, threshold >= 0.  Not taken, with no status set,
+// where it does not apply; timer (nullable): events recorded around the
+// product kernel.
 bool ell_x2_tiles(bml_matrix_ellpack_t *X, bml_matrix_ellpack_t *C, double threshold, double *trace, int *required_M,
-                  bool *taken, bool *asym, cudaEvent_t *timer);
+                  TileOutcome *out, cudaEvent_t *timer);
 // The tile form of the unordered A*B (and X^2 whatever its symmetry) of square
-// matrices of one N, threshold >= 0; check_pre as for ell_multiply_unordered.
+// matrices of one N, threshold >= 0; check_pre as for ell_multiply_unordered;
+// known (nullable): what an attempt at the symmetric square has counted.
 bool ell_general_tiles(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bml_matrix_ellpack_t *C, double threshold,
-                       double *trace, int *required_M, bool check_pre, bool *taken, cudaEvent_t *timer);
+                       const TileOutcome *known, double *trace, int *required_M, bool check_pre, bool *taken,
+                       cudaEvent_t *timer);
 // The tile form of the masked product below; *taken false, with no status
 // set, where it does not apply.
 bool ell_masked_tiles(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bml_matrix_ellpack_t *P,

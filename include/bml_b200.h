@@ -343,6 +343,24 @@ BML_B200_API int bml_b200_last_x2_symmetric(void);
  * No reference counterpart. */
 BML_B200_API int bml_b200_set_dense_tier(int allow);
 BML_B200_API int bml_b200_last_x2_dense(void);
+/* The tile form of the unordered products (8 x 8 tiles on the FP64 tensor
+ * instructions): set_tiles(0) forbids it, 1 (the default) takes it where the
+ * counts of both forms' products say that it is the faster one, 2 wherever it
+ * applies; returns the previous setting.  last_product_form() tells the form
+ * of the last ELLPACK product (a masked one: the adjoint's, at a given
+ * pattern).  No reference counterpart. */
+enum
+{
+    BML_B200_PRODUCT_ORDERED = 0,
+    BML_B200_PRODUCT_SPARSE = 1,
+    BML_B200_PRODUCT_SPARSE_SYMMETRIC = 2,
+    BML_B200_PRODUCT_TILES = 3,
+    BML_B200_PRODUCT_TILES_SYMMETRIC = 4,
+    BML_B200_PRODUCT_TILES_MASKED = 5,
+    BML_B200_PRODUCT_DENSE = 6
+};
+BML_B200_API int bml_b200_set_tiles(int mode);
+BML_B200_API int bml_b200_last_product_form(void);
 BML_B200_API int bml_b200_set_kernel_timing(int on);
 BML_B200_API double bml_b200_last_x2_kernel_ms(void);
 

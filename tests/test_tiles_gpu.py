@@ -14,6 +14,14 @@ pytestmark = [pytest.mark.gpu, pytest.mark.unordered]
 SINGLE, DOUBLE = 1, 2
 
 
+@pytest.fixture
+def tiles():
+    """The tile form wherever it applies, whatever the counts say."""
+    old = B.lib.bml_b200_set_tiles(2)
+    yield
+    B.lib.bml_b200_set_tiles(old)
+
+
 def _banded(N, band, density, seed, empty=(), dtype=np.float64):
     """Symmetric matrix of a band, each pair present with the given
     probability, rows and columns in `empty` without entries."""
@@ -87,17 +95,20 @@ CASES = [(1, 0, 1.0, ()), (7, 3, 0.6, ()), (8, 8, 0.9, ()), (9, 2, 1.0, ()), (31
 @pytest.mark.parametrize("prec", [DOUBLE, SINGLE], ids=["fp64", "fp32"])
 @pytest.mark.parametrize("shuffle", [False, True], ids=["ascending", "any_order"])
 @pytest.mark.parametrize("N,band,density,empty", CASES)
-def test_tiles_against_restatement(N, band, density, empty, shuffle, prec):
+def test_tiles_against_restatement(tiles, N, band, density, empty, shuffle, prec):
     from oracle import oracle as O
     D = _banded(N, band, density, N + band, empty, np.float64 if prec == DOUBLE else np.float32)
     for thr in (0.0, 1e-2):
         _check(O, D, shuffle, thr, prec)
+        assert B.product_form() == "tiles_symmetric"
     assert B.lib.bml_b200_last_x2_symmetric() == 1
 
 
-def test_tiles_long_lists():
-    """More common tile columns than a warp lists at a time (1024: 8192 columns)."""
-    N, M = 8400, 8400
+@pytest.mark.parametrize("N", [8 * 127, 8 * 128, 8 * 129, 8400])
+def test_tiles_long_lists(N):
+    """As many common tile columns as a warp lists at a time (128), one more
+    and less, and many more."""
+    M = N
     rng = np.random.default_rng(0)
     D = np.zeros((N, N))
     D[:8, :] = rng.standard_normal((8, N))
@@ -106,6 +117,7 @@ def test_tiles_long_lists():
     arrs = _rows(D, M, False, 0)
     st, tr, got = _x2(arrs, N, M, N, 1e-9, DOUBLE)
     assert st == B.OK
+    assert B.product_form() == "tiles_symmetric"
     Dt = torch.from_numpy(D).cuda()  # the FP64 dense product as the oracle
     want, S = Dt @ Dt, Dt.abs() @ Dt.abs()
     G = torch.from_numpy(_dense(got, N, N)).cuda()
@@ -131,6 +143,7 @@ def test_matrices_the_tile_form_leaves_to_the_sparse_one():
     asym[9 * M] += 1.0
     for vals in (inf, zero, asym):
         st, tr, got = _x2((vals, ix, nz), N, M, N, 1e-5, DOUBLE)
+        assert B.product_form() == ("sparse" if vals is asym else "sparse_symmetric")
         old = B.lib.bml_b200_set_x2_symmetric(0)
         st0, tr0, want = _x2((vals, ix, nz), N, M, N, 1e-5, DOUBLE)
         B.lib.bml_b200_set_x2_symmetric(old)
@@ -150,6 +163,7 @@ def test_entries_of_a_row_that_cancel():
     st, tr, got = _x2((v, ix, nz), N, M, N, 1e-9, DOUBLE)
     assert st == B.OK
     assert got[2][50] == 0
+    assert B.product_form() == "sparse"
     assert tr[1] == pytest.approx(np.trace(D @ D), rel=1e-12)
 
 
@@ -168,6 +182,7 @@ def test_an_entry_without_its_mirror(i, j):
     assert (np.abs(_dense(got, N, N) - D @ D) <= 1e-12 * S).all()
     assert tr[1] == pytest.approx(np.trace(D @ D), rel=1e-12)
     assert B.lib.bml_b200_last_x2_symmetric() == 0
+    assert B.product_form() == "sparse"
 
 
 @pytest.mark.parametrize("M2", [40, 76], ids=["pool_runs_out", "rows_too_wide"])
@@ -195,10 +210,11 @@ def test_tiles_row_overflow(M2):
         np.testing.assert_allclose(got[0][i * M2:i * M2 + n], X2[i, k], rtol=0, atol=1e-11)
     if M2 == 76:
         assert B.lib.bml_b200_last_required_M() == 81
+    assert B.product_form() == ("tiles_symmetric" if M2 == 76 else "sparse_symmetric")
 
 
 @pytest.mark.parametrize("L,radius", [(6, 2), (7, 3)])
-def test_masked_tiles_unsymmetric_weights(L, radius):
+def test_masked_tiles_unsymmetric_weights(tiles, L, radius):
     """The adjoint's masked products on tiles (the second operand through its
     transpose): weights that are not symmetric, so neither are the gradients
     that the products take; against the ordered form's gradient (whole
@@ -218,6 +234,7 @@ def test_masked_tiles_unsymmetric_weights(L, radius):
         dH = B.Ellpack(N, M)
         loss = C.c_double()
         B.check(B.lib.bml_b200_sp2_adjoint(H.h, V.h, 1e-5, N / 2.0, 6, 2, M, dH.h, C.byref(loss)))
+        assert B.product_form() == ("ordered" if exact else "tiles_masked")
         grads.append((loss.value, dH.download()))
         B.lib.bml_b200_set_x2_exact(old)
     (l0, (g0, i0, n0)), (l1, (g1, i1, n1)) = grads
@@ -240,10 +257,9 @@ def _random_band(N, band, density, seed, empty, dtype):
 @pytest.mark.parametrize("N,ba,bb,density,empty", [
     (1, 0, 0, 1.0, ()), (9, 2, 8, 0.9, (3,)), (32, 31, 5, 0.8, ()), (33, 4, 33, 0.7, (0, 32)),
     (257, 30, 60, 0.6, tuple(range(32, 64))), (400, 399, 20, 0.5, ()), (900, 12, 80, 0.9, ()),
-    # matrices of fewer than 4096 rows take the sparse form
     (4095, 4, 33, 0.7, ()), (4096, 12, 80, 0.9, ()), (4097, 399, 20, 0.5, (0, 4096)),
     (4129, 30, 60, 0.6, tuple(range(32, 64)))])
-def test_general_tiles(N, ba, bb, density, empty, square, dtype):
+def test_general_tiles(tiles, N, ba, bb, density, empty, square, dtype):
     """A*B and X^2 of matrices that are not symmetric, rows in any order: the
     kept entries and the diagonal where some product touches it, against the
     dense FP64 product; and the refusal of a row that touches more than M
@@ -281,6 +297,8 @@ def test_general_tiles(N, ba, bb, density, empty, square, dtype):
         B.clear_error()
         B.lib.bml_b200_set_verbose(1)
         assert st == status
+        # (a single row is symmetric)
+        assert B.product_form() == ("tiles_symmetric" if square and N == 1 else "tiles")
         if status != B.OK:
             continue
         got = Cm.download()
@@ -293,3 +311,79 @@ def test_general_tiles(N, ba, bb, density, empty, square, dtype):
         sure |= np.eye(N, dtype=bool)
         assert np.array_equal(K[sure], keep[sure])
         assert (abs(G - want)[K] <= (tol + 1e-300)[K] + (abs(want)[K] * 2.0 ** -24 if dtype == np.float32 else 0)).all()
+
+
+def _random_rows(N, w, seed, symmetric):
+    """ELLPACK arrays of w random columns a row."""
+    rng = np.random.default_rng(seed)
+    D = np.zeros((N, N))
+    for i in range(N):
+        D[i, rng.choice(N, w, replace=False)] = rng.standard_normal(w)
+    if symmetric:
+        D = D + D.T
+    M = int((D != 0).sum(1).max())
+    return D, _rows(D, M, False, 0), M
+
+
+def _check_dense(got, D, E, thr):
+    N = D.shape[0]
+    want, S = D @ E, abs(D) @ abs(E)
+    G = _dense(got, N, len(got[0]) // N)
+    assert (abs(G - want) <= 1e-12 * S + np.where(G == 0, thr, 0.0)).all()
+
+
+@pytest.mark.parametrize("kind,N,w,form", [
+    # few products per tile product: the sparse form, counted while packed and (4200 rows) before
+    ("random", 700, 6, "sparse_symmetric"), ("random", 4200, 3, "sparse_symmetric"),
+    # the same without symmetry: found by the sample of entries
+    ("random_asym", 700, 6, "sparse"), ("random_asym", 4200, 3, "sparse"),
+    # a band without symmetry, too little work for the tile form's launches, and enough of it
+    ("band_asym", 700, 31, "sparse"), ("band_asym", 3000, 201, "tiles"), ("band_asym", 4200, 201, "tiles"),
+    # symmetric but for one entry: found by the check of all
+    ("band_one", 700, 31, "sparse"), ("band_one", 4200, 201, "tiles"),
+    ("band", 700, 31, "tiles_symmetric"), ("band", 4200, 31, "tiles_symmetric"),
+    # a few groups that pack badly among many that do not
+    ("mixed", 2000, 61, "tiles_symmetric")])
+def test_which_form(kind, N, w, form):
+    if kind.startswith("random"):
+        D, arrs, M = _random_rows(N, w, 1, kind == "random")
+    else:
+        D = _random_band(N, w // 2, 1.0, 1, (), np.float64)
+        if kind != "band_asym":
+            D = np.triu(D) + np.triu(D, 1).T
+        if kind == "band_one":
+            D[5, 6] += 1.0
+        if kind == "mixed":
+            far = np.random.default_rng(2).choice(np.arange(64, N), 40, replace=False)
+            D[np.arange(40) % 32, far] = D[far, np.arange(40) % 32] = 0.25
+        M = int((D != 0).sum(1).max())
+        arrs = _rows(D, M, False, 0)
+    st, tr, got = _x2(arrs, N, M, min(N, 1024), 1e-9, DOUBLE)
+    assert st == B.OK
+    assert B.product_form() == form
+    _check_dense(got, D, D, 1e-9)
+
+
+@pytest.mark.parametrize("wa,wb,N,form", [(3, 3, 600, "sparse"), (201, 201, 600, "sparse"), (201, 201, 3000, "tiles"),
+                                          (1, 41, 2000, "sparse"), (41, 1, 3000, "sparse"), (201, 3, 4200, "tiles")])
+def test_which_form_of_a_product(wa, wb, N, form):
+    Da, Db = (_random_band(N, w // 2, 1.0, w, (), np.float64) for w in (wa, wb))
+    A, Bm = (B.Ellpack.from_arrays(*_rows(D, 512, False, 0), N, 512) for D in (Da, Db))
+    Cm = B.Ellpack(N, min(N, 512))
+    B.lib.bml_multiply_AB(A.h, Bm.h, Cm.h, 1e-9)
+    B.check()
+    assert B.product_form() == form
+    _check_dense(Cm.download(), Da, Db, 1e-9)
+
+
+def test_set_tiles():
+    D = _banded(300, 20, 1.0, 2)
+    arrs = _rows(D, 41, False, 0)
+    forms = []
+    for mode in (0, 1, 2, 1):
+        old = B.lib.bml_b200_set_tiles(mode)
+        st, tr, got = _x2(arrs, 300, 41, 128, 0.0, DOUBLE)
+        B.lib.bml_b200_set_tiles(old)
+        assert st == B.OK and old == 1
+        forms.append(B.product_form())
+    assert forms == ["sparse_symmetric", "tiles_symmetric", "tiles_symmetric", "tiles_symmetric"]
