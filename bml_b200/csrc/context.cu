@@ -1,6 +1,7 @@
 // Library context, error state and logging.
 #include "internal.h"
 
+#include <atomic>
 #include <cstdarg>
 #include <cstdlib>
 #include <cstring>
@@ -188,6 +189,37 @@ bool b200_sync()
     if (!c)
         return false;
     return CUDA_OK(cudaStreamSynchronize(c->stream));
+}
+
+int b200_next_told()
+{
+    static std::atomic<unsigned> n{0};
+    return (int) (++n & 0x3fffffffu) | 1 << 30;
+}
+
+bool b200_spin(const volatile int *word, int told)
+{
+    for (int spin = 0; spin < 20000 && *word != told; ++spin)
+    {
+#ifdef __x86_64__
+        __builtin_ia32_pause();
+#endif
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
+    return *word == told;
+}
+
+bool b200_told(const volatile int *word, int told)
+{
+    if (b200_spin(word, told))
+        return true;
+    if (!b200_sync())
+        return false;
+    std::atomic_thread_fence(std::memory_order_acquire);
+    if (*word == told)
+        return true;
+    b200_set_error(BML_B200_ERR_CUDA, "the kernels did not report");
+    return false;
 }
 
 // ---------------------------------------------------------------------------

@@ -59,6 +59,8 @@ struct F64Flags
     int max_touched;
     int next;
     int overflow, max_kept;
+    int done;                 // CTAs of the closing kernel that have finished
+    double trA, trC;
 };
 
 struct F64Args
@@ -78,9 +80,18 @@ struct F64Args
     unsigned long long *spill_at; // first spill block of a row
     unsigned char *keep;          // [ib][q]
     double *spill;
-    double *dA, *dC;              // per-row traces (nullable)
-    F64Flags *flags;
+    double *dA, *dC;              // per-row traces
+    F64Flags *flags, *host;       // host: pinned, written by the closing kernel's last CTA, then
+    int told;                     // this to the word behind it
 };
+
+// Rows of up to SHORT_NB blocks into a C with room for all of them: nothing can
+// spill, so the product is queued without the host learning the lists' lengths
+// first, a numeric kernel for either outcome of the symmetry check among it.
+// (8 block rows of 4 blocks: 80 us with that wait, four memsets and a copy at
+// the end, 57 in the accumulating form, 55 so; 27 rows of up to 7 85, 92 and 62.)
+constexpr int SHORT_NB = 128;
+constexpr int TOLD = 32;
 
 __global__ void __launch_bounds__(PT) f64_table_kernel(F64Args g)
 {
@@ -193,11 +204,11 @@ __global__ void __launch_bounds__(PT) f64_symbolic_kernel(F64Args g)
         if (tid == 0)
         {
             g.count[ib] = lb;
+            g.dA[ib] = tr;
+            g.dC[ib] = 0.0;
             if (lb > g.MC)
                 g.spill_at[ib] = atomicAdd(&g.flags->spill, (unsigned long long) (lb - g.MC));
             atomicMax(&g.flags->max_touched, lb);
-            if (g.dA)
-                g.dA[ib] = tr;
         }
         __syncthreads();
     }
@@ -210,8 +221,11 @@ __device__ __forceinline__ double *place_of(const F64Args &g, int ib, int q)
 }
 
 // SYM: X^2 of a symmetric X, both operands read along their rows.
-template <bool SYM> __global__ void __launch_bounds__(FW * 32, FMIN) f64_numeric_kernel(F64Args g, int chunks)
+// only: return unless the symmetry check came out for this form.
+template <bool SYM> __global__ void __launch_bounds__(FW * 32, FMIN) f64_numeric_kernel(F64Args g, int chunks, int only)
 {
+    if (only && SYM == (g.flags->asym != 0))
+        return;
     __shared__ unsigned queue[FW][PAIRS];
     __shared__ int item, nextq;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -394,7 +408,7 @@ template <bool SYM> __global__ void __launch_bounds__(FW * 32, FMIN) f64_numeric
                 if (SYM && !diag)
                     g.keep[(size_t) kb * g.NB + qm] = kept;
             }
-            if (diag && g.dC)
+            if (diag)
             {
                 for (int o = 16; o; o >>= 1)
                     tr += __shfl_xor_sync(FULL, tr, o);
@@ -479,6 +493,52 @@ __global__ void __launch_bounds__(PT) f64_close_kernel(F64Args g)
                 atomicExch(&g.flags->overflow, 1);
         }
     }
+    // the traces, summed over rows in a fixed order by the CTA that finishes last, and the flags for the host
+    __shared__ double part[2][W];
+    __shared__ int fin;
+    __syncthreads();
+    if (tid == 0)
+    {
+        __threadfence(); // this CTA's rows come before its count
+        fin = atomicAdd(&g.flags->done, 1) == (int) gridDim.x - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!fin)
+        return;
+    double a = 0.0, d = 0.0;
+    for (int ib = tid; ib < g.NB; ib += PT)
+    {
+        a += __ldcg(g.dA + ib);
+        d += __ldcg(g.dC + ib);
+    }
+    for (int o = 16; o; o >>= 1)
+    {
+        a += __shfl_xor_sync(FULL, a, o);
+        d += __shfl_xor_sync(FULL, d, o);
+    }
+    if (lane == 0)
+    {
+        part[0][warp] = a;
+        part[1][warp] = d;
+    }
+    __syncthreads();
+    if (tid != 0)
+        return;
+    for (int w = 1; w < W; ++w)
+    {
+        a += part[0][w];
+        d += part[1][w];
+    }
+    volatile F64Flags *h = g.host;
+    const volatile F64Flags *f = g.flags;
+    h->asym = f->asym;
+    h->overflow = f->overflow;
+    h->max_kept = f->max_kept;
+    h->trA = a;
+    h->trC = d;
+    __threadfence_system();
+    reinterpret_cast<volatile int *>(g.host)[TOLD] = g.told;
 }
 
 } // namespace
@@ -517,7 +577,8 @@ bool eb_multiply_f64(bml_matrix_ellblock_t *A, bml_matrix_ellblock_t *B, bml_mat
     unsigned char *pin = static_cast<unsigned char *>(c->pinned) + F64_SMALL;
     F64Flags *hf = reinterpret_cast<F64Flags *>(pin);
     g.flags = reinterpret_cast<F64Flags *>(small);
-    double *dtrace = reinterpret_cast<double *>(small + 128);
+    g.host = hf;
+    const bool brief = NB <= SHORT_NB && C->MB >= NB;
     const int rows = std::min(NB, c->sm_count * 8);
     const size_t smemS = (size_t) NB * sizeof(unsigned short);
     size_t spill = 0;
@@ -533,13 +594,12 @@ bool eb_multiply_f64(bml_matrix_ellblock_t *A, bml_matrix_ellblock_t *B, bml_mat
         g.keep = scr + o_keep;
         g.count = reinterpret_cast<int *>(scr + o_count);
         g.spill_at = reinterpret_cast<unsigned long long *>(scr + o_sat);
-        g.dA = trace ? reinterpret_cast<double *>(scr + o_diag) : nullptr;
-        g.dC = trace ? g.dA + NB : nullptr;
+        g.dA = reinterpret_cast<double *>(scr + o_diag);
+        g.dC = g.dA + NB;
         g.spill = reinterpret_cast<double *>(scr + fixed);
-        if (!CUDA_OK(cudaMemsetAsync(small, 0, 256, c->stream)) ||
-            !CUDA_OK(cudaMemsetAsync(g.colT, 0xff, nn * 2, c->stream)) ||
-            (g.square && !CUDA_OK(cudaMemsetAsync(g.rowT, 0xff, nn * 2, c->stream))) ||
-            (trace && !CUDA_OK(cudaMemsetAsync(g.dA, 0, (size_t) 2 * NB * sizeof(double), c->stream))))
+        // (both tables: they lie side by side)
+        if (!CUDA_OK(cudaMemsetAsync(small, 0, sizeof(F64Flags), c->stream)) ||
+            !CUDA_OK(cudaMemsetAsync(scr + o_row, 0xff, o_list - o_row, c->stream)))
             return false;
         f64_table_kernel<<<rows, PT, 0, c->stream>>>(g);
         if (!LAUNCH_OK("f64_table_kernel"))
@@ -551,8 +611,11 @@ bool eb_multiply_f64(bml_matrix_ellblock_t *A, bml_matrix_ellblock_t *B, bml_mat
                 return false;
         }
         f64_symbolic_kernel<<<rows, PT, smemS, c->stream>>>(g);
-        if (!LAUNCH_OK("f64_symbolic_kernel") ||
-            !CUDA_OK(cudaMemcpyAsync(pin, small, sizeof(F64Flags), cudaMemcpyDeviceToHost, c->stream)) || !b200_sync())
+        if (!LAUNCH_OK("f64_symbolic_kernel"))
+            return false;
+        if (brief)
+            break;
+        if (!CUDA_OK(cudaMemcpyAsync(pin, small, sizeof(F64Flags), cudaMemcpyDeviceToHost, c->stream)) || !b200_sync())
             return false;
         if (hf->spill * 8192 > budget)
             return true;
@@ -561,29 +624,30 @@ bool eb_multiply_f64(bml_matrix_ellblock_t *A, bml_matrix_ellblock_t *B, bml_mat
         // room for the blocks past MB: the lists are made again in the larger arena
         spill = (size_t) hf->spill;
     }
-    const bool sym = g.square && !hf->asym;
-    const int chunks = (std::max(hf->max_touched, 1) + CHUNK - 1) / CHUNK;
+    const int chunks = ((brief ? NB : std::max(hf->max_touched, 1)) + CHUNK - 1) / CHUNK;
     const int grid = (int) std::min<long long>((long long) NB * chunks, (long long) c->sm_count * FMIN);
-    if (sym)
-        f64_numeric_kernel<true><<<grid, FW * 32, 0, c->stream>>>(g, chunks);
-    else
-        f64_numeric_kernel<false><<<grid, FW * 32, 0, c->stream>>>(g, chunks);
-    if (!LAUNCH_OK("f64_numeric_kernel"))
-        return false;
-    f64_close_kernel<<<rows, PT, 0, c->stream>>>(g);
-    if (!LAUNCH_OK("f64_close_kernel"))
-        return false;
-    if (trace)
+    if (g.square && (brief || !hf->asym))
     {
-        b200_sum_rows_kernel<<<1, 1024, 0, c->stream>>>(g.dA, g.dC, NB, dtrace);
-        if (!LAUNCH_OK("b200_sum_rows_kernel"))
+        f64_numeric_kernel<true><<<grid, FW * 32, 0, c->stream>>>(g, chunks, brief);
+        if (!LAUNCH_OK("f64_numeric_kernel"))
             return false;
     }
-    if (!CUDA_OK(cudaMemcpyAsync(pin, small, 256, cudaMemcpyDeviceToHost, c->stream)) || !b200_sync())
+    if (!g.square || brief || hf->asym)
+    {
+        f64_numeric_kernel<false><<<grid, FW * 32, 0, c->stream>>>(g, chunks, g.square && brief);
+        if (!LAUNCH_OK("f64_numeric_kernel"))
+            return false;
+    }
+    g.told = b200_next_told();
+    f64_close_kernel<<<rows, PT, 0, c->stream>>>(g);
+    if (!LAUNCH_OK("f64_close_kernel") || !b200_told(reinterpret_cast<const int *>(hf) + TOLD, g.told))
         return false;
     *taken = true;
     if (trace)
-        memcpy(trace, pin + 128, 2 * sizeof(double));
+    {
+        trace[0] = hf->trA;
+        trace[1] = hf->trC;
+    }
     if (hf->overflow)
     {
         b200_set_error(BML_B200_ERR_ROW_OVERFLOW,

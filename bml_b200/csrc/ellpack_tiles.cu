@@ -68,7 +68,6 @@
 #include "device_util.cuh"
 
 #include <algorithm>
-#include <atomic>
 #include <climits>
 #include <cstring>
 #include <type_traits>
@@ -1565,43 +1564,12 @@ template <typename T> __global__ void __launch_bounds__(PT) tile_gather_kernel(T
     }
 }
 
-void pause()
-{
-#ifdef __x86_64__
-    __builtin_ia32_pause();
-#endif
-}
-
-// The host's copy of the flags, once a kernel has told (tell_host) the given
-// number.  The word in pinned memory is read for a while before the stream is
-// waited for: it is there some microseconds before cudaStreamSynchronize
-// returns, and no copy has to be queued.
-bool flags_told(B200Context *c, const TileFlags *hf, int told)
-{
-    const volatile int *word = reinterpret_cast<const volatile int *>(hf) + TOLD;
-    for (int spin = 0; spin < 20000 && *word != told; ++spin)
-        pause();
-    std::atomic_thread_fence(std::memory_order_acquire);
-    if (*word == told)
-        return true;
-    if (!b200_sync())
-        return false;
-    std::atomic_thread_fence(std::memory_order_acquire);
-    if (*word == told)
-        return true;
-    b200_set_error(BML_B200_ERR_CUDA, "multiply: the tile kernels did not report");
-    return false;
-}
-
 // What the symmetry check has told of the counts at its start, if it does
 // within the wait.
 bool early_told(const TileArgs &g, TileOutcome *out)
 {
     const volatile int4 *e = g.early;
-    for (int spin = 0; spin < 20000 && e->x != g.told; ++spin)
-        pause();
-    std::atomic_thread_fence(std::memory_order_acquire);
-    if (e->x != g.told)
+    if (!b200_spin(&e->x, g.told))
         return false;
     const int p = e->y, t = e->z, w = e->w;
     float products, tiles2;
@@ -1611,12 +1579,6 @@ bool early_told(const TileArgs &g, TileOutcome *out)
     out->counted = true;
     out->counts = {(unsigned long long) products, (unsigned long long) (w >> 1), (unsigned long long) tiles2, 0, 0};
     return true;
-}
-
-int next_told()
-{
-    static std::atomic<unsigned> n{0};
-    return (int) (++n & 0x7fffffffu) | 1 << 30; // never 0
 }
 
 template <typename T> bool tile_masked_typed(TileArgs a, TileArgs b, bool *taken)
@@ -1856,7 +1818,7 @@ bool tile_general_typed(TileArgs a, TileArgs b, const TileCounts *known, double 
         n = *known;
     else
     {
-        a.told = next_told();
+        a.told = b200_next_told();
         if (!CUDA_OK(cudaMemsetAsync(small, 0, sizeof(TileFlags), c->stream)))
             return false;
         if (a.Xi == b.Xi)
@@ -1871,7 +1833,7 @@ bool tile_general_typed(TileArgs a, TileArgs b, const TileCounts *known, double 
                 return false;
             tile_cross_kernel<<<std::min(2 * NG, c->sm_count * 8), FT, smemC, c->stream>>>(a, rows_b);
         }
-        if (!LAUNCH_OK("tile counts") || !flags_told(c, hf, a.told))
+        if (!LAUNCH_OK("tile counts") || !b200_told(reinterpret_cast<const int *>(hf) + TOLD, a.told))
             return false;
         a.told = 0;
         if (hf->bad)
@@ -1904,9 +1866,9 @@ bool tile_general_typed(TileArgs a, TileArgs b, const TileCounts *known, double 
             return false;
         if (attempt)
             break;
-        b.told = next_told();
+        b.told = b200_next_told();
         tile_tcount_kernel<<<per, PT, 0, c->stream>>>(b);
-        if (!LAUNCH_OK("tile_tcount_kernel") || !flags_told(c, hf, b.told))
+        if (!LAUNCH_OK("tile_tcount_kernel") || !b200_told(reinterpret_cast<const int *>(hf) + TOLD, b.told))
             return false;
         b.told = 0;
         const long long entries = (long long) n.entries + hf->counted;
@@ -1976,9 +1938,9 @@ bool tile_general_typed(TileArgs a, TileArgs b, const TileCounts *known, double 
         return false;
     if (timer && !CUDA_OK(cudaEventRecord(timer[1], c->stream)))
         return false;
-    a.told = next_told();
+    a.told = b200_next_told();
     tile_rows_kernel<T><<<NG, RT, smemR, c->stream>>>(a);
-    if (!LAUNCH_OK("tile_rows_kernel") || !flags_told(c, hf, a.told))
+    if (!LAUNCH_OK("tile_rows_kernel") || !b200_told(reinterpret_cast<const int *>(hf) + TOLD, a.told))
         return false;
     if (hf->bad || hf->odd || hf->full)
         return true;
@@ -2030,9 +1992,9 @@ bool tile_x2_typed(TileArgs g, double *trace, int *required_M, TileOutcome *out,
     g.sample = pack_all ? 0 : 1;
     if (!lazy)
     {
-        g.told = next_told();
+        g.told = b200_next_told();
         tile_count_kernel<T><<<per, FT, smemC, c->stream>>>(g);
-        if (!LAUNCH_OK("tile_count_kernel") || !flags_told(c, hf, g.told))
+        if (!LAUNCH_OK("tile_count_kernel") || !b200_told(reinterpret_cast<const int *>(hf) + TOLD, g.told))
             return false;
         g.told = 0;
         note();
@@ -2098,7 +2060,7 @@ bool tile_x2_typed(TileArgs g, double *trace, int *required_M, TileOutcome *out,
         tile_fill_kernel<T, false><<<per, FT, smemF, c->stream>>>(g);
     else
     {
-        g.told = next_told();
+        g.told = b200_next_told();
         g.early = reinterpret_cast<int4 *>(reinterpret_cast<unsigned char *>(hf) + EARLY);
         tile_fill_kernel<T, true><<<per, FT, smemF, c->stream>>>(g);
     }
@@ -2124,9 +2086,9 @@ bool tile_x2_typed(TileArgs g, double *trace, int *required_M, TileOutcome *out,
     if (smemR > 32768 && !CUDA_OK(cudaFuncSetAttribute(
                              tile_rows_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smemR)))
         return false;
-    g.told = next_told();
+    g.told = b200_next_told();
     tile_rows_kernel<T><<<g.NG, RT, smemR, c->stream>>>(g);
-    if (!LAUNCH_OK("tile_rows_kernel") || !flags_told(c, hf, g.told))
+    if (!LAUNCH_OK("tile_rows_kernel") || !b200_told(reinterpret_cast<const int *>(hf) + TOLD, g.told))
         return false;
     note();
     if (hf->skipped && !hf->odd && !out->asym && !left_to_sparse(*hf, g.cost))

@@ -118,6 +118,13 @@ void *b200_scratch_try(size_t bytes);
 bool b200_device_alloc(void **p, size_t bytes);
 // Synchronise the library stream; false (error recorded) on failure.
 bool b200_sync();
+// Kernels that report through pinned memory: a number for the word that they
+// write last, never 0; a bounded wait for it (b200_spin), and the same followed
+// by b200_sync (b200_told).  The word is there some microseconds before
+// cudaStreamSynchronize returns, and no copy has to be queued.
+int b200_next_told();
+bool b200_spin(const volatile int *word, int told);
+bool b200_told(const volatile int *word, int told);
 
 // ---------------------------------------------------------------------------
 // Matrix helpers (matrix.cu)

@@ -92,7 +92,9 @@ def test_x2_symmetric_lattice(L, radius):
 
 
 @pytest.mark.parametrize("symmetric", [True, False])
-@pytest.mark.parametrize("nb,per_row,thr", [(5, 2, 0.0), (17, 3, 1e-5), (40, 3, 20.0), (40, 4, 1e-3), (64, 40, 1e-5)])
+@pytest.mark.parametrize("nb,per_row,thr", [(5, 2, 0.0), (17, 3, 1e-5), (40, 3, 20.0), (40, 4, 1e-3), (64, 40, 1e-5),
+                                            # queued without the lists' lengths up to 128 block rows
+                                            (128, 3, 1e-5), (129, 3, 1e-5)])
 def test_x2_random_blocks(nb, per_row, thr, symmetric):
     X = _random_blocks(nb, per_row, nb, symmetric, small=0.4)
     _compare(X, None, nb, nb, thr)
