@@ -1145,9 +1145,12 @@ bool ell_trace_mult(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, double *tr
     int *beyond = reinterpret_cast<int *>(static_cast<unsigned char *>(c->d_small) + 3072) + 16;
     const int *need = nullptr;
     int done = -1;
+    // (few rows: the last size alone, whose warps go round them four times or less; 4096 rows with M = 1024 31 us, 33
+    // with two launches more)
+    const bool few = (size_t) A->N * (2 * sizeof(int) << full) <= 4 * (size_t) c->sm_count * c->smem_optin;
     for (int logts : {TRACE_NARROW, TRACE_WIDE, full})
     {
-        if (logts > full)
+        if (logts > full || (few && logts != full))
             continue;
         int warps_per_block = 4;
         while ((size_t) warps_per_block * 2 * sizeof(int) << logts > c->smem_optin)
