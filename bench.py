@@ -467,10 +467,10 @@ def formed_fraction(X, n, sample=400, seed=0):
 
 
 # ncu capture of one X^2 call on the 30^3 lattice's SP2 iterate (bench.py
-# --profile, 18.57 G reference product terms; profiles/x2_tiles_lattice30.md):
-# the product kernel's dram__bytes_read.sum + dram__bytes_write.sum
+# --profile, 18.57 G reference product terms): the product kernel's
+# dram__bytes_read.sum + dram__bytes_write.sum
 NCU_X2_PRODUCTS = 18570945128
-NCU_X2_KERNEL_DRAM = 2796406784 + 115515136
+NCU_X2_KERNEL_DRAM = 2766112768 + 115035904
 
 
 def x2_roofline(B, H, info):

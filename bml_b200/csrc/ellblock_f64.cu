@@ -11,7 +11,9 @@
 // warp takes 16 columns of the block at a time, so that the registers hold the
 // sum and, apart from it, the product of the current pair: a sum of pair
 // products, as in eb_mul32_kernel, rounds less than one chain over all pairs
-// (1.7e-16 against 8.3e-16 of the result's norm on the 11^3 block lattice).
+// (against 80-bit sums, block lattices of 3^3 to 5^3: 1.8e-16 of the result's
+// norm, as eb_mul32_kernel; on the 11^3 lattice a chain is four times as far
+// from an FP64 product as this).
 //
 // Steps.  A table T[kb][j] gives the slot of block (j, kb) of B (X^2 of a
 // symmetric X: of block (kb, j), which is its transpose, so both operands are
@@ -70,7 +72,6 @@ struct F64Args
     double *Cp; int *Ci; int *Cn; int MC;
     int NB;
     int square;                   // A == B
-    int fast_norm;                // keep test on the double norm (X^2) or after rounding (the same in FP64)
     double thr;
     unsigned short *rowT;         // [ib][jb]: slot of block (ib, jb) of A (square only)
     unsigned short *colT;         // [kb][j]: slot of block (j, kb) of B

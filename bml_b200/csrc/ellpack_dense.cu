@@ -14,12 +14,12 @@
 // dropped by the rule, as the sparse kernels drop it, so only the diagonal
 // needs the structure: it is touched when some j has A[i,j] and B[j,i]
 // stored, found through a byte image of B's pattern (in a symmetric square
-// through the values).  The traces are those of the sparse kernels: tr A from A's diagonal entries, tr C from the
-// pre-threshold diagonal where touched.
+// through the image itself).  The traces are those of the sparse kernels: tr A
+// from A's diagonal entries, tr C from the pre-threshold diagonal where touched.
 //
 // Symmetric squares (the image equal to its transpose) form the tiles on and
-// above the diagonal only.  X^2 of 5001 full rows in FP64: 13.93 ms with the
-// FMA kernel below for both types and both triangles, 5.08 ms now.
+// above the diagonal only.  X^2 of 5001 full rows in FP64: 13.93 ms on the FMA
+// pipe, as the FP32 GEMM below, with both triangles, 5.01 ms so.
 //
 // The FP32 GEMM: 128 x 128 tiles of C per CTA of 256 threads, each thread 8 x 8
 // outputs (rows ty + 16 m, columns tx + 16 n) in registers; K in steps of 16

@@ -14,8 +14,9 @@
 // lies), filled matrices on the dense tier (ellpack_dense.cu).
 //
 // Every product a*b is a separately rounded multiply followed by one
-// rounded add, so |C - C_ref| <= (n-1) u sum_j |A_ij B_jk| for a column summed
-// from n products: 1e-12 of that sum for any n below 4500 in FP64.
+// rounded add, as in the reference but in another order, so |C - C_ref| <= 2 n u
+// sum_j |A_ij B_jk| to first order for a column summed from n products: 1e-12 of
+// that sum for any n below 4500 in FP64.
 //
 // B200 design.  One CTA per output row at a time (persistent CTAs claim rows
 // from a counter, so rows in flight are neighbours and share the rows of B

@@ -308,11 +308,12 @@ BML_B200_API int bml_b200_set_x2_tiers(int mask);
 /* Chooses how later ELLPACK products (bml_multiply_x2, bml_multiply,
  * bml_multiply_AB and the SP2 drivers) sum.  exact = 0 (the default): the
  * unordered kernels, which form the same products and apply the same keep
- * rule but add the products of one entry in another order, so an entry differs
- * from the reference's by at most (n-1) u sum|a_ij b_jk| for n products (the
- * sparse form rounds every multiply and every add; the tile form, taken where
- * the matrix packs into 8 x 8 tiles, and the dense tier add the products with
- * fused multiply-adds, which round once less), and write a row's kept entries
+ * rule but add the products of one entry in another order (the sparse form
+ * rounds every multiply and every add; the tile form, taken where the matrix
+ * packs into 8 x 8 tiles, and the dense tier add the products with fused
+ * multiply-adds), so that each of the two sums lies within n u sum|a_ij b_jk|
+ * of the exact one for n products, to first order in u, and an entry differs
+ * from the reference's by at most twice that; they write a row's kept entries
  * in ascending column order.  exact = 1: the ordered tiers
  * above, bit-identical to the reference, rows in its first-touch order.
  * Rows wider than the unordered kernel holds (M above about 8000) always use
@@ -337,8 +338,8 @@ BML_B200_API int bml_b200_last_x2_symmetric(void);
 /* The dense tier of the unordered product: when both operands' rows fill at
  * least 40 % of their columns on average (and the dense images fit 64 GiB),
  * A and B are scattered into dense images, multiplied by a GEMM (FP64 on the
- * tensor cores, FP32 register-tiled) and compacted with the same keep rule, rows in ascending column
- * order.  set_dense_tier(0) forbids it (default 1; returns the previous
+ * tensor cores, FP32 register-tiled) and compacted with the same keep rule,
+ * rows in ascending column order.  set_dense_tier(0) forbids it (default 1; returns the previous
  * setting); last_x2_dense() is 1 when the last unordered product ran on it.
  * No reference counterpart. */
 BML_B200_API int bml_b200_set_dense_tier(int allow);
