@@ -4,7 +4,7 @@ order as beta*b, each step rounded as the reference rounds it
 (ellpack/bml_add_ellpack_typed.c:50-216), kept when |x| > threshold.  Rows at
 the edges of the tables (2048 columns of B where M is at most 512, else 32768),
 wider ones beside them (found by a hash), rows longer than one round of a CTA
-(256 and 1024 entries), columns that are multiples of a table apart, empty
+(128 and 1024 entries), columns that are multiples of a table apart, empty
 rows, zero scalars; and tr(A B^T) of matrices large enough to be sized by their
 rows."""
 import numpy as np
