@@ -47,8 +47,8 @@
 // the host at its start what was counted, so that a form that does not apply
 // costs the fill kernel and not the rest (X^2 without symmetry, us, sparse form
 // alone | with a packing and a wait before it | so: 500 rows of 21 59 | 75 |
-// 61, 2000 rows of 21 87 | 108 | 92; symmetric but scattered, which the sparse
-// form has to check once more: 500 rows of 40 86 | 130 | 110, 4096 rows of 40 259
+// 61, 2000 rows of 21 87 | 108 | 88; symmetric but scattered, which the sparse
+// form has to check once more: 500 rows of 40 86 | 130 | 108, 4096 rows of 40 259
 // | 353 | 285).
 //
 // The general product (A B, and X^2 of an X that is not symmetric) packs the
@@ -190,18 +190,19 @@ __host__ __device__ __forceinline__ bool left_to_sparse(const TileFlags &f, doub
 // A product of two matrices by its counts (cost 0: whatever they are): what the
 // sparse form takes longer for, in us, a row, an entry of A (each visits a row
 // of B) and a product, against a tile product and what the tile form's twelve
-// launches take whatever the sizes.  Fitted to 95 products of bands, lattices,
+// launches take whatever the sizes.  Fitted to 143 products of bands, lattices,
 // diagonals and scattered matrices of 500 to 64000 rows, on which it takes
-// neither form where the other is more than 5 % faster (tile form / sparse form,
+// neither form where the other is more than 3 % faster (tile form / sparse form,
 // us: bands of 3 and 3 of 4096 rows 114 / 83, of 8000 144 / 135, of 20000 243 /
 // 303, of 31 and 31 122 / 109, 160 / 192 and 270 / 427, of 301 and 301 of 500
 // rows 209 / 114, of 1700 231 / 351, of 4096 261 / 799; a diagonal times a 16^3
 // lattice 130 / 105, times a 28^3 one 416 / 562; lattices of radii 3 and 3.5, 14^3
-// 222 / 196, 22^3 628 / 784; 4096 scattered rows of 20 1059 / 142).
+// 222 / 196, 22^3 628 / 784, of 2 and 4.5, 18^3 345 / 333, 23^3 711 / 734; 4096
+// scattered rows of 20 1059 / 142).
 __host__ __device__ __forceinline__ bool general_pays(double rows, double stored, double products, double tiles2,
                                                       double cost)
 {
-    return cost == 0.0 || 6.5e-3 * rows + 1e-4 * stored + 1.4e-6 * products - 45e-6 * tiles2 > 65.0;
+    return cost == 0.0 || 10e-3 * rows + 1.4e-4 * stored + 1e-6 * products - 30e-6 * tiles2 > 90.0;
 }
 // The form does not apply: the kernels after the fill do nothing.  (`alone` says
 // so only when the symmetry check is through; the others are set for good.)
@@ -351,9 +352,10 @@ __device__ __forceinline__ void group_counts(const TileArgs &g, int G, const uns
     }
 }
 
-// A look for the mirror of one entry of a row, in two parts, so that the loads
-// of the first are under way while the caller counts: find() tells of a row
-// without it.  One warp.
+// A look for the mirror of a row's last entry, in two parts, so that the loads
+// of the first are under way while the caller counts; missing() tells of a row
+// without it.  (Of ascending rows the mirror is the first in its own: any entry
+// of rows of 700 took 8 us longer to find.)  One warp.
 template <typename T, int U> struct MirrorSample
 {
     int i, k, kk[U];
@@ -366,7 +368,7 @@ template <typename T, int U> struct MirrorSample
         const int n = i < g.N ? g.Xn[i] : 0;
         if (n < 1 || n > g.ld)
             return;
-        const size_t at = (size_t) i * g.ld + ((unsigned) i * 2654435761u >> 8) % (unsigned) n;
+        const size_t at = (size_t) i * g.ld + n - 1;
         k = __ldg(g.Xi + at);
         x = __ldg(static_cast<const T *>(g.Xv) + at);
     }
@@ -518,11 +520,11 @@ __device__ __forceinline__ int tile_at(int r, int c) { return 2 * (4 * r + (c & 
 // Lists, zero-filled tiles and the scatter of group G's entries.  Rows in
 // ascending order have distinct columns and are stored; other rows are added
 // (duplicate columns add up, as they do in the sparse form).
-// LAZY: there was no counting pass, and no more groups than SMs.  (In FP64 one
-// CTA per SM, with the registers for its loads: 600 us against 652 with two for
-// 64000 rows of 925; in FP32 two: 49 us against 65 for 26999 rows of 113.)
-template <typename T, bool LAZY>
-__global__ void __launch_bounds__(FT, LAZY || sizeof(T) == 8 ? 1 : 2) tile_fill_kernel(TileArgs g)
+// LAZY: there was no counting pass, and no more groups than SMs.
+// CTAS per SM: two for narrow rows, one, with the registers for its loads, for
+// wide ones (FP64, of the whole call: 20000 rows of 101 193 us with two and 201
+// with one, 8000 of 257 397 and 398; the kernel on 64000 of 925 652 and 600).
+template <typename T, bool LAZY, int CTAS> __global__ void __launch_bounds__(FT, CTAS) tile_fill_kernel(TileArgs g)
 {
     extern __shared__ unsigned bm[]; // [4][nw] bitmaps | [nw] entries before the word
     int *before = reinterpret_cast<int *>(bm + 4 * g.nw);
@@ -1584,6 +1586,16 @@ bool early_told(const TileArgs &g, TileOutcome *out)
     return true;
 }
 
+// The fill kernel after a counting pass.
+constexpr int FILL_WIDE = 300; // entries a row
+template <typename T> void tile_fill(const TileArgs &g, int grid, size_t smem, cudaStream_t stream, double stored)
+{
+    if (sizeof(T) == 8 && stored >= (double) FILL_WIDE * g.N)
+        tile_fill_kernel<T, false, 1><<<grid, FT, smem, stream>>>(g);
+    else
+        tile_fill_kernel<T, false, 2><<<grid, FT, smem, stream>>>(g);
+}
+
 template <typename T> bool tile_masked_typed(TileArgs a, TileArgs b, bool *taken)
 {
     B200Context *c = b200_ctx();
@@ -1610,6 +1622,7 @@ template <typename T> bool tile_masked_typed(TileArgs a, TileArgs b, bool *taken
     const size_t o_pb = take((size_t) NG * a.hw * sizeof(unsigned)), o_pr = take((size_t) NG * a.hw * sizeof(int));
     const size_t fixed = at;
     unsigned char *scr = nullptr;
+    double stored = 0.0;
     // the counts, then the layout; a larger arena loses the transpose's bitmaps, which are then made again
     for (int attempt = 0; attempt < 2; ++attempt)
     {
@@ -1641,6 +1654,7 @@ template <typename T> bool tile_masked_typed(TileArgs a, TileArgs b, bool *taken
             return false;
         if (hf->counted >= (1 << 28) || left_to_sparse(*hf, a.cost))
             return true;
+        stored = (double) hf->stored;
         take(0);
         const size_t o_ent = take((size_t) hf->counted * sizeof(unsigned));
         const size_t o_entJ = take((size_t) hf->counted * sizeof(unsigned short));
@@ -1677,10 +1691,10 @@ template <typename T> bool tile_masked_typed(TileArgs a, TileArgs b, bool *taken
     a.count_only = 0;
     if (!CUDA_OK(cudaMemsetAsync(small, 0, sizeof(TileFlags), c->stream)))
         return false;
-    tile_fill_kernel<T, false><<<per, FT, smemF, c->stream>>>(a);
+    tile_fill<T>(a, per, smemF, c->stream, stored);
     if (!LAUNCH_OK("tile_fill_kernel"))
         return false;
-    tile_fill_kernel<T, false><<<per, FT, smemF, c->stream>>>(b);
+    tile_fill<T>(b, per, smemF, c->stream, 0.0);
     if (!LAUNCH_OK("tile_fill_kernel"))
         return false;
     tile_scatter_kernel<T><<<std::min(b200_ceil_div(b.N, PT / 32), c->sm_count * 8), PT, 0, c->stream>>>(b);
@@ -1919,10 +1933,10 @@ bool tile_general_typed(TileArgs a, TileArgs b, const TileCounts *known, double 
     tile_touch_kernel<<<rows, PT, 0, c->stream>>>(a);
     if (!LAUNCH_OK("tile_touch_kernel"))
         return false;
-    tile_fill_kernel<T, false><<<per, FT, smemF, c->stream>>>(a);
+    tile_fill<T>(a, per, smemF, c->stream, (double) n.stored);
     if (!LAUNCH_OK("tile_fill_kernel"))
         return false;
-    tile_fill_kernel<T, false><<<per, FT, smemF, c->stream>>>(b);
+    tile_fill<T>(b, per, smemF, c->stream, 0.0);
     if (!LAUNCH_OK("tile_fill_kernel"))
         return false;
     tile_scatter_kernel<T><<<rows, PT, 0, c->stream>>>(b);
@@ -2066,12 +2080,12 @@ bool tile_x2_typed(TileArgs g, double *trace, int *required_M, TileOutcome *out,
                                                         (int) smemR))))
         return false;
     if (!lazy)
-        tile_fill_kernel<T, false><<<per, FT, smemF, c->stream>>>(g);
+        tile_fill<T>(g, per, smemF, c->stream, (double) out->counts.stored);
     else
     {
         g.told = b200_next_told();
         g.early = reinterpret_cast<int4 *>(reinterpret_cast<unsigned char *>(hf) + EARLY);
-        tile_fill_kernel<T, true><<<per, FT, smemF, c->stream>>>(g);
+        tile_fill_kernel<T, true, 1><<<per, FT, smemF, c->stream>>>(g);
     }
     if (!LAUNCH_OK("tile_fill_kernel"))
         return false;
