@@ -131,6 +131,58 @@ __device__ __forceinline__ bool hash_add(int *keys, int *pay, unsigned mask, int
     return false;
 }
 
+// Whether a product of two matrices is the tile form's (ellpack_tiles.cu), by its
+// counts (cost 0: whatever they are): what the
+// sparse form takes longer for, in us, a row, an entry of A (each visits a row
+// of B) and a product, against a tile product and what the tile form's twelve
+// launches take whatever the sizes.  Fitted to 143 products of bands, lattices,
+// diagonals and scattered matrices of 500 to 64000 rows, on which it takes
+// neither form where the other is more than 3 % faster (tile form / sparse form,
+// us: bands of 3 and 3 of 4096 rows 114 / 83, of 8000 144 / 135, of 20000 243 /
+// 303, of 31 and 31 122 / 109, 160 / 192 and 270 / 427, of 301 and 301 of 500
+// rows 209 / 114, of 1700 231 / 351, of 4096 261 / 799; a diagonal times a 16^3
+// lattice 130 / 105, times a 28^3 one 416 / 562; lattices of radii 3 and 3.5, 14^3
+// 222 / 196, 22^3 628 / 784, of 2 and 4.5, 18^3 345 / 333, 23^3 711 / 734; 4096
+// scattered rows of 20 1059 / 142).
+__host__ __device__ __forceinline__ bool general_pays(double rows, double stored, double products, double tiles2,
+                                                      double cost)
+{
+    return cost == 0.0 || 10e-3 * rows + 1.4e-4 * stored + 1e-6 * products - 30e-6 * tiles2 > 90.0;
+}
+
+// Whether the row lengths of A and B speak for tiles, with 40 products per tile
+// product (lattices have 20 to 60, bands hundreds).  One CTA of 1024 threads;
+// the answer is thread 0's.
+__device__ __forceinline__ bool rows_for_tiles(const int *An, int lda, const int *Bn, int ldb, int n)
+{
+    __shared__ double part[2][32];
+    double a = 0.0, b = 0.0;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n; i += 1024)
+    {
+        a += min(max(An[i], 0), lda);
+        b += min(max(Bn[i], 0), ldb);
+    }
+    for (int o = 16; o; o >>= 1)
+    {
+        a += __shfl_xor_sync(FULL, a, o);
+        b += __shfl_xor_sync(FULL, b, o);
+    }
+    if ((threadIdx.x & 31) == 0)
+    {
+        part[0][threadIdx.x >> 5] = a;
+        part[1][threadIdx.x >> 5] = b;
+    }
+    __syncthreads();
+    for (int w = 1; threadIdx.x == 0 && w < 32; ++w)
+    {
+        a += part[0][w];
+        b += part[1][w];
+    }
+    const double products = a * b / n;
+    return general_pays(n, a, products, products / 40.0, 1.0);
+}
+
 } // namespace b200
 
 // Sum of one or two per-row arrays in FP64 with a fixed order (each thread a

@@ -187,23 +187,6 @@ __host__ __device__ __forceinline__ bool left_to_sparse(const TileFlags &f, doub
     return f.bad || f.asym || (double) f.tiles2 * cost > (double) f.products;
 }
 
-// A product of two matrices by its counts (cost 0: whatever they are): what the
-// sparse form takes longer for, in us, a row, an entry of A (each visits a row
-// of B) and a product, against a tile product and what the tile form's twelve
-// launches take whatever the sizes.  Fitted to 143 products of bands, lattices,
-// diagonals and scattered matrices of 500 to 64000 rows, on which it takes
-// neither form where the other is more than 3 % faster (tile form / sparse form,
-// us: bands of 3 and 3 of 4096 rows 114 / 83, of 8000 144 / 135, of 20000 243 /
-// 303, of 31 and 31 122 / 109, 160 / 192 and 270 / 427, of 301 and 301 of 500
-// rows 209 / 114, of 1700 231 / 351, of 4096 261 / 799; a diagonal times a 16^3
-// lattice 130 / 105, times a 28^3 one 416 / 562; lattices of radii 3 and 3.5, 14^3
-// 222 / 196, 22^3 628 / 784, of 2 and 4.5, 18^3 345 / 333, 23^3 711 / 734; 4096
-// scattered rows of 20 1059 / 142).
-__host__ __device__ __forceinline__ bool general_pays(double rows, double stored, double products, double tiles2,
-                                                      double cost)
-{
-    return cost == 0.0 || 10e-3 * rows + 1.4e-4 * stored + 1e-6 * products - 30e-6 * tiles2 > 90.0;
-}
 // The form does not apply: the kernels after the fill do nothing.  (`alone` says
 // so only when the symmetry check is through; the others are set for good.)
 __device__ __forceinline__ bool unpacked(const TileArgs &g)
@@ -456,6 +439,18 @@ template <typename T> __global__ void __launch_bounds__(FT, 2) tile_count_kernel
         tell_host(g, lane);
 }
 
+// Before the counts of a product of two matrices: whether the row lengths speak
+// for tiles at all.  The counts are left out if not, and the host, told by one
+// store of 8 bytes, begins the sparse form.  One CTA.
+__global__ void __launch_bounds__(1024) tile_lengths_kernel(TileArgs a, TileArgs b, int told)
+{
+    const int go = rows_for_tiles(a.Xn, a.ld, b.Xn, b.ld, a.N);
+    if (threadIdx.x)
+        return;
+    a.flags->skipped = !go;
+    asm volatile("st.volatile.global.v2.s32 [%0], {%1, %2};" ::"l"(a.early), "r"(told), "r"(go) : "memory");
+}
+
 // The same for a product of two matrices: a's counts, the products of its
 // entries with b's rows, and, once all groups of both have been through, the
 // tile products: tiles of a's tile column J times tiles of b's tile row J.
@@ -466,6 +461,8 @@ __global__ void __launch_bounds__(FT, 2) tile_cross_kernel(TileArgs a, TileArgs 
     __shared__ unsigned long long sums[3];
     __shared__ int fin;
     const int lane = threadIdx.x & 31;
+    if (a.flags->skipped)
+        return;
     bool ok = true;
     for (int q = blockIdx.x; ok && q < 2 * a.NG; q += gridDim.x)
     {
@@ -1788,6 +1785,14 @@ __global__ void __launch_bounds__(PT) tile_touch_kernel(TileArgs g)
     }
 }
 
+// Rows below which the row lengths are asked in the sparse form's flight, from
+// there to 9000 ahead of the counts.  Most products of fewer rows stay on the
+// sparse form, which then pays 3 us; most of more rows take tiles, which would
+// pay 10 to 17 us for the flight stopped and pay 3 so (18^3 lattices of radii 3
+// and 2.5 316 and 306; of 2 and 2.5, which stay, 220 and 227, 240 with the counts
+// alone, 217 with nothing asked).
+constexpr int FEW_ROWS = 4096;
+
 // Whether the counts can say so at all, by the room of the rows.
 bool general_may_pay(const bml_matrix_ellpack_t *A, const bml_matrix_ellpack_t *B, double cost)
 {
@@ -1848,7 +1853,26 @@ bool tile_general_typed(TileArgs a, TileArgs b, const TileCounts *known, double 
             a.tileC = a.tileN + 4 * NG;
             if (!CUDA_OK(cudaMemsetAsync(a.tileC, 0, (size_t) 4 * NG * sizeof(int), c->stream)))
                 return false;
+            const int told = b200_next_told();
+            // (of fewer rows they were asked before the call came here)
+            const bool lengths = a.N >= FEW_ROWS && !general_pays(a.N, 0.0, 0.0, 0.0, a.cost);
+            if (lengths)
+            {
+                a.early = reinterpret_cast<int4 *>(reinterpret_cast<unsigned char *>(hf) + EARLY);
+                tile_lengths_kernel<<<1, 1024, 0, c->stream>>>(a, b, told);
+                if (!LAUNCH_OK("tile_lengths_kernel"))
+                    return false;
+            }
             tile_cross_kernel<<<std::min(2 * NG, c->sm_count * 8), FT, smemC, c->stream>>>(a, rows_b);
+            if (lengths)
+            {
+                const volatile int4 *e = a.early;
+                if (!LAUNCH_OK("tile_cross_kernel") || !b200_told(&e->x, told))
+                    return false;
+                if (!e->y)
+                    return true;
+                a.early = nullptr;
+            }
         }
         if (!LAUNCH_OK("tile counts") || !b200_told(reinterpret_cast<const int *>(hf) + TOLD, a.told))
             return false;
@@ -2192,6 +2216,13 @@ bool ell_masked_tiles(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bml_matr
     a.Mc = C->M;
     return A->matrix_precision == double_real ? tile_masked_typed<double>(a, b, taken)
                                               : tile_masked_typed<float>(a, b, taken);
+}
+
+bool ell_general_tiles_by_rows(const bml_matrix_ellpack_t *A, const bml_matrix_ellpack_t *B,
+                               const bml_matrix_ellpack_t *C, double threshold)
+{
+    return g_tiles == 1 && threshold >= 0.0 && A->N < FEW_ROWS && A->N == B->N && A->N == C->N &&
+           general_may_pay(A, B, TILE_COST);
 }
 
 bool ell_general_tiles(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bml_matrix_ellpack_t *C, double threshold,

@@ -192,6 +192,10 @@ bool ell_x2_tiles(bml_matrix_ellpack_t *X, bml_matrix_ellpack_t *C, double thres
 bool ell_general_tiles(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bml_matrix_ellpack_t *C, double threshold,
                        const TileOutcome *known, double *trace, int *required_M, bool check_pre, bool *taken,
                        cudaEvent_t *timer);
+// Whether the row lengths alone should be asked first, on the device, if that
+// form can pay: few rows, with room for enough.
+bool ell_general_tiles_by_rows(const bml_matrix_ellpack_t *A, const bml_matrix_ellpack_t *B,
+                               const bml_matrix_ellpack_t *C, double threshold);
 // The tile form of the masked product below; *taken false, with no status
 // set, where it does not apply.
 bool ell_masked_tiles(bml_matrix_ellpack_t *A, bml_matrix_ellpack_t *B, bml_matrix_ellpack_t *P,

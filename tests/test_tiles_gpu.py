@@ -364,8 +364,10 @@ def test_which_form(kind, N, w, form):
     _check_dense(got, D, D, 1e-9)
 
 
+# rooms of 512: up to 4095 rows the lengths are asked first, and the counts where those speak for tiles
 @pytest.mark.parametrize("wa,wb,N,form", [(3, 3, 600, "sparse"), (201, 201, 600, "sparse"), (201, 201, 3000, "tiles"),
-                                          (1, 41, 2000, "sparse"), (41, 1, 3000, "sparse"), (201, 3, 4200, "tiles")])
+                                          (1, 41, 2000, "sparse"), (41, 1, 3000, "sparse"), (201, 3, 4200, "tiles"),
+                                          (201, 201, 4095, "tiles"), (3, 3, 4095, "sparse"), (3, 3, 4096, "sparse")])
 def test_which_form_of_a_product(wa, wb, N, form):
     Da, Db = (_random_band(N, w // 2, 1.0, w, (), np.float64) for w in (wa, wb))
     A, Bm = (B.Ellpack.from_arrays(*_rows(D, 512, False, 0), N, 512) for D in (Da, Db))
@@ -374,6 +376,18 @@ def test_which_form_of_a_product(wa, wb, N, form):
     B.check()
     assert B.product_form() == form
     _check_dense(Cm.download(), Da, Db, 1e-9)
+
+
+def test_lengths_for_tiles_and_counts_against():
+    """Wide rows of scattered columns: the row lengths speak for tiles, the
+    tile products against; the sparse form is begun twice."""
+    N, w = 2500, 250
+    (D, arrs, M), (E, brrs, _) = (_random_rows(N, w, s, False) for s in (1, 2))
+    A, Bm, Cm = B.Ellpack.from_arrays(*arrs, N, M), B.Ellpack.from_arrays(*brrs, N, M), B.Ellpack(N, N)
+    B.lib.bml_multiply_AB(A.h, Bm.h, Cm.h, 1e-9)
+    B.check()
+    assert B.product_form() == "sparse"
+    _check_dense(Cm.download(), D, E, 1e-9)
 
 
 def test_set_tiles():
